@@ -328,7 +328,7 @@ __device__ void adjoint_tile_mixed(const AdjSmem<double>& a, const AdjSmem<float
 // each reverse stage is followed by the boundary's transpose, and the first
 // reverse stage of a boundary tile also covers the ghost cells (their
 // cotangents reach the interior through the Neumann mirrors).
-template <class T, int EQ, int REC>
+template <class T, int EQ, int REC, int FLUX>
 __device__ void adjoint_tile(const AdjSmem<T>& a, Win<T> gout, int te, T dtdx, const OpParams<T>& p,
                              const BcView& bc = BcView(), int64_t g0 = 0, int64_t n = 0,
                              const StageOut<const stage_t<T, REC>>& st =
@@ -382,6 +382,32 @@ __device__ void adjoint_tile(const AdjSmem<T>& a, Win<T> gout, int te, T dtdx, c
         }
     }
     if (!stored) {
+    if constexpr (FLUX == kFluxRusanovFx) {
+        // the stages of step_tile_fx on this window (T1: the listed faces)
+        Smem<T> f = a.fwd(a.K1);
+        f.fx = win_cast<int>(a.T1);
+        if (tid < kFxCounters) f.fx[tid] = 0;
+        __syncthreads();
+        const T c = dtdx * (1.0 / 288.0);
+        {
+            const int lo = HU - 15, hi = HU + te + 15;
+            fx_fluxes(a.U, lo - 1, hi, f, p, 0, StoreFaces<Win<T>>{a.CLu, a.CRu, HU - 6, HU + te + 6, 0});
+            for (int i = lo + tid; i < hi; i += nt) a.K1[i] = fma(c, a.D[i - 1] - a.D[i], a.U[i]);
+            __syncthreads();
+            if (np) apply_bc(a.K1, g0, n, lo, hi, bc, 1);
+        }
+        {
+            const int lo = HU - 12, hi = HU + te + 12;
+            fx_fluxes(a.K1, lo - 1, hi, f, p, 1, StoreFaces<Win<T>>{a.CL1, a.CR1, HU - 6, HU + te + 6, 0});
+            for (int i = lo + tid; i < hi; i += nt) {
+                const T k = fma(c, a.D[i - 1] - a.D[i], a.K1[i]);
+                a.K2[i] = fma(1.0 / 4.0, k, (3.0 / 4.0) * a.U[i]);
+            }
+            __syncthreads();
+            if (np) apply_bc(a.K2, g0, n, lo, hi, bc, 2);
+        }
+        fx_fluxes(a.K2, HU - 10, HU + te + 9, f, p, 2, StoreFaces<Win<T>>{a.UL, a.UR, HU - 9, HU + te + 9, 0});
+    } else {
     {
         const int lo = HU - 15, hi = HU + te + 15;
         // WENO-JS5: the face values of u stay in CLu/CRu for reverse stage 1
@@ -420,6 +446,7 @@ __device__ void adjoint_tile(const AdjSmem<T>& a, Win<T> gout, int te, T dtdx, c
         // forms them (as the stored ones; the fluxes it also leaves in D are
         // not used)
         face_fluxes<T, EQ, REC, SHK_FLUX_RUSANOV>(a.K2, HU - 8, HU + te + 8, a.fwd(a.K2, a.UL, a.UR), p);
+    }
     }
     }
     // reverse stage 3: k2b = 2/3 (p + dt J(k2)^T p) on [HU-6, HU+te+6)
@@ -493,8 +520,8 @@ __device__ __forceinline__ bool adjoint_load(const AdjSmem<T>& a, const T* um, c
     return load_window<T>(a.PB + (HU - HP), pn, n, s0 - HP, te + 2 * HP, bar, phase);
 }
 
-template <class T, int EQ, int REC>
-__global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 2 : 1) batched_adjoint_kernel(PlanDev P, const T* __restrict__ um,
+template <class T, int EQ, int REC, int FLUX>
+__global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED || FLUX == kFluxRusanovFx ? 2 : 1) batched_adjoint_kernel(PlanDev P, const T* __restrict__ um,
                                                                    const T* __restrict__ pnext,
                                                                    T* __restrict__ pout,
                                                                    const double* __restrict__ dt_row,
@@ -540,7 +567,7 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 2 : 1) batc
         const StageOut<const stage_t<T, REC>> st =
             as_const(stage_out<T, REC>(const_cast<void*>(stages), total, off));
         if constexpr (kMixed) adjoint_tile_mixed<EQ>(a, af, gpout + (off + s0), te, dtdx, p, bc, g0, n, st);
-        else adjoint_tile<T, EQ, REC>(a, gpout + (off + s0), te, dtdx, p, bc, g0, n, st);
+        else adjoint_tile<T, EQ, REC, FLUX>(a, gpout + (off + s0), te, dtdx, p, bc, g0, n, st);
         __syncthreads();
     }
     finish_items(P, 2);
@@ -551,8 +578,8 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 2 : 1) batc
 // stages (optional): the step's stage storage, kStageArrays<T, REC> arrays of
 // P's cells in the stage precision (stage_arrays), for a reverse step that
 // skips its forward recompute; uout may then be null.
-template <class T, int EQ, int REC>
-__global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : 1) replay_step_kernel(PlanDev P, const T* __restrict__ uin,
+template <class T, int EQ, int REC, int FLUX>
+__global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : (FLUX == kFluxRusanovFx ? 2 : 1)) replay_step_kernel(PlanDev P, const T* __restrict__ uin,
                                                                T* __restrict__ uout,
                                                                const double* __restrict__ dt_row,
                                                                OpParams<T> p, void* stages,
@@ -561,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : 1) repl
     __shared__ __align__(8) uint64_t bar;
     constexpr int HL = step_halo<T>();
     Smem<T> sm;
-    carve_step<T, REC>(sm, smem_raw, P.tile + 2 * HL);
+    carve_step<T, REC, FLUX>(sm, smem_raw, P.tile + 2 * HL);
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_mbar_init();
@@ -590,7 +617,7 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : 1) repl
             break;
         }
         const T dtdx = static_cast<T>(dt * P.inv_dx[b]);
-        step_tile<T, EQ, REC, SHK_FLUX_RUSANOV>(sm, uout ? guout + (off + s0) : Win<T>(), te, dtdx, p,
+        step_tile<T, EQ, REC, FLUX>(sm, uout ? guout + (off + s0) : Win<T>(), te, dtdx, p,
                                                 plan_bc(P, b, step), s0 - HL, n,
                                                 stage_out<T, REC>(stages, total, off + s0));
         __syncthreads();
@@ -599,7 +626,7 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : 1) repl
 }
 
 // single instance on the reference's ghosted layout (drop-in adjoint_step)
-template <class T, int EQ>
+template <class T, int EQ, int FLUX>
 __global__ void __launch_bounds__(kThreads) single_vjp_kernel(const T* __restrict__ u, const T* __restrict__ pn,
                                                               T* __restrict__ pout, int64_t n, int g,
                                                               int tile, T dtdx, OpParams<T> p,
@@ -629,7 +656,7 @@ __global__ void __launch_bounds__(kThreads) single_vjp_kernel(const T* __restric
     bc.neu_ss = 2;
     bc.dx = dx;
     const Win<T> gpout = make_win(pout, n + 2 * g);
-    adjoint_tile<T, EQ, SHK_REC_WENOJS53>(a, gpout + (g + s0), te, dtdx, p, bc, s0 - adj_uhalo<T>(), n);
+    adjoint_tile<T, EQ, SHK_REC_WENOJS53, FLUX>(a, gpout + (g + s0), te, dtdx, p, bc, s0 - adj_uhalo<T>(), n);
     // ghost cotangents are zero (interior-only adjoint)
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < g; i += blockDim.x) {
@@ -676,6 +703,8 @@ OpParams<T> adj_params(const shk_scheme* s) {
     p.lim_param = static_cast<T>(s->delta);
     p.atol = static_cast<T>(s->eps);
     p.dx = T(1);
+    p.e4h = static_cast<float>(4.0 * s->eps);
+    p.e4l = static_cast<float>(4.0 * s->eps - static_cast<double>(p.e4h));
     return p;
 }
 
@@ -707,13 +736,20 @@ int by_equation(int eq, F&& f) {
     return by_equation_rec<T, SHK_REC_WENOJS53>(eq, f);
 }
 
+// instances with a kFluxRusanovFx form (used for the schemes of fixed_flux_scheme)
+template <class T, int EQ, int REC>
+constexpr bool kHasFixed = sizeof(T) == 8 && EQ == SHK_EQ_BURGERS && REC == SHK_REC_WENOJS53;
+
 template <class TS>
 struct AdjLaunch {
     PlanDev D; const void* um; const void* pn; void* po; const double* dt_row; OpParams<TS> p;
     size_t smem; int grid; cudaStream_t st; const void* stages = nullptr; int64_t total = 0;
     int64_t step = 0;  // index of the forward step (its boundary data)
+    bool fixed = false;
     template <class T, int EQ, int REC> int operator()() {
-        auto k = batched_adjoint_kernel<T, EQ, REC>;
+        auto k = batched_adjoint_kernel<T, EQ, REC, SHK_FLUX_RUSANOV>;
+        if constexpr (kHasFixed<T, EQ, REC>)
+            if (fixed) k = batched_adjoint_kernel<T, EQ, REC, kFluxRusanovFx>;
         ADJ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k<<<grid, kThreads, smem, st>>>(D, static_cast<const T*>(um), static_cast<const T*>(pn),
                                          static_cast<T*>(po), dt_row, p, stages, total, step);
@@ -726,8 +762,11 @@ struct ReplayLaunch {
     PlanDev D; const void* uin; void* uout; const double* dt_row; OpParams<TS> p;
     size_t smem; int grid; cudaStream_t st; void* stages = nullptr; int64_t total = 0;
     int64_t step = 0;  // index of the replayed step (its boundary data)
+    bool fixed = false;
     template <class T, int EQ, int REC> int operator()() {
-        auto k = replay_step_kernel<T, EQ, REC>;
+        auto k = replay_step_kernel<T, EQ, REC, SHK_FLUX_RUSANOV>;
+        if constexpr (kHasFixed<T, EQ, REC>)
+            if (fixed) k = replay_step_kernel<T, EQ, REC, kFluxRusanovFx>;
         ADJ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k<<<grid, kThreads, smem, st>>>(D, static_cast<const T*>(uin), static_cast<T*>(uout), dt_row, p,
                                          stages, total, step);
@@ -738,8 +777,11 @@ struct ReplayLaunch {
 struct SingleVjpLaunch {
     const double* u; const double* pn; double* po; int64_t n; int g; int tile; double dtdx;
     OpParams<double> p; size_t smem; int blocks; cudaStream_t st; shk_boundary bc; double dx;
+    bool fixed = false;
     template <class T, int EQ, int REC> int operator()() {
-        auto k = single_vjp_kernel<T, EQ>;
+        auto k = single_vjp_kernel<T, EQ, SHK_FLUX_RUSANOV>;
+        if constexpr (kHasFixed<T, EQ, REC>)
+            if (fixed) k = single_vjp_kernel<T, EQ, kFluxRusanovFx>;
         ADJ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k<<<blocks, kThreads, smem, st>>>(u, pn, po, n, g, tile, dtdx, p, nullptr, bc, dx);
         return acuda(cudaGetLastError());
@@ -768,7 +810,7 @@ int shk_ssprk33_vjp_bc_f64(const shk_scheme* scheme, const shk_boundary* bc, con
     const size_t smem = AdjSmem<double>::host_bytes(W);
     const int blocks = static_cast<int>((n + tile - 1) / tile);
     SingleVjpLaunch f{u, p_next, p_out, n, nghosts, tile, dt / dx, adj_params<double>(scheme),
-                      smem, blocks, st, b, dx};
+                      smem, blocks, st, b, dx, fixed_flux_scheme(scheme)};
     return by_equation<double>(scheme->equation, f);
 }
 
@@ -861,7 +903,7 @@ int shk_plan_adjoint_staged(shk_plan* plan, const void* ckpt, int32_t stride, in
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev0);
         if (asmem > static_cast<size_t>(optin)) return SHK_EUNSUPPORTED;
     }
-    const size_t fsmem = dtype == SHK_F64 ? Smem<double>::step_bytes(D.tile + 2 * step_halo<double>(), sch.rec)
+    const size_t fsmem = dtype == SHK_F64 ? Smem<double>::step_bytes(D.tile + 2 * step_halo<double>(), sch.rec, fixed_flux_scheme(&sch))
                                           : Smem<float>::step_bytes(D.tile + 2 * step_halo<float>(), sch.rec);
     // adjoint grid: resident CTAs for its larger shared-memory footprint
     int dev = 0, sms = 1;
@@ -889,7 +931,7 @@ int shk_plan_adjoint_staged(shk_plan* plan, const void* ckpt, int32_t stride, in
             void* out = j < cnt ? seg_at(j) : nullptr;
             if (dtype == SHK_F64) {
                 ReplayLaunch<double> f{D, seg_at(j - 1), out, row, adj_params<double>(&sch), fsmem, grid, st,
-                                       stage_at(j - 1), total, base + j - 1};
+                                       stage_at(j - 1), total, base + j - 1, fixed_flux_scheme(&sch)};
                 r = by_scheme<double>(sch, f);
             } else {
                 ReplayLaunch<float> f{D, seg_at(j - 1), out, row, adj_params<float>(&sch), fsmem, grid, st,
@@ -902,7 +944,7 @@ int shk_plan_adjoint_staged(shk_plan* plan, const void* ckpt, int32_t stride, in
             const double* row = D.dt_hist + size_t(base + j) * D.B;
             if (dtype == SHK_F64) {
                 AdjLaunch<double> f{D, seg_at(j), cur, nxt, row, adj_params<double>(&sch), asmem, agrid, st,
-                                    stage_at(j), total, base + j};
+                                    stage_at(j), total, base + j, fixed_flux_scheme(&sch)};
                 r = by_scheme<double>(sch, f);
             } else {
                 AdjLaunch<float> f{D, seg_at(j), cur, nxt, row, adj_params<float>(&sch), asmem, agrid, st,

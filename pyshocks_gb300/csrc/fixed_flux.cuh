@@ -1,0 +1,355 @@
+// Face fluxes of a double state without the FP64 pipe (Burgers, WENO-JS5,
+// Rusanov with nu = 1).
+//
+// GB300's FP64 pipe takes 16 clocks per warp instruction and SM, 64 times an
+// FP32 or integer instruction's share, so the flux is formed from 64-bit
+// integers and pairs of floats. With E_k = v_{k+1} - 2 v_k + v_{k-1} and
+// T_k = E_{k+1} - E_k, the two face values of WENO-JS5 (R = ur_j, L = ul_{j+1})
+// on the middle sub-stencil's value plus weighted third differences give
+//   Z = 6 (R + L) = 6 (v_j + v_{j+1}) - (E_j + E_{j+1}) + pR_j + pL_{j+1}
+//   D = 6 (R - L) = T_j + pR_j - pL_{j+1}
+//   288 F = Z^2 + D (D + 24 a),  a = max(|v_j|, |v_{j+1}|)
+//   pR = -(2 r0 T_{c-1} + 3 r2 T_c) / (r0 + 6 + 3 r2)
+//   pL =  (2 r2 T_c + 3 r0 T_{c-1}) / (r2 + 6 + 3 r0)
+// with r0 = (e1/e0)^2, r2 = (e1/e2)^2, e_k = 4 (eps + beta_k). Only pR and pL
+// are nonlinear, and they carry the factor T, the third difference:
+//   * v, E, T, Z and D are 64-bit integers in units of 2^-57 of the largest of
+//     a lane's cells (a power of two per lane), finer than a double near that
+//     size; sums and differences of them are exact;
+//   * pR and pL are unevaluated sums of two floats (about 45 bits). A face is
+//     accepted while |T| <= 2^-7 of the lane's scale: their error then stays
+//     below 2^-54 of it, under the rounding of a double evaluation. Other faces
+//     (shocks, noise, non-finite values, scales outside 2^+-60) are left to
+//     the FP64 formula.
+// The two cells of a lane run in the two halves of the packed float
+// instructions (add/mul/fma.f32x2).
+#pragma once
+
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define SHK_FX __device__ __forceinline__
+#else
+#include <cmath>
+#include <cstring>
+#define SHK_FX static inline
+#endif
+
+namespace shk {
+namespace fx {
+
+// ---- pairs of floats in one register pair ------------------------------------
+#ifdef __CUDACC__
+struct P2 {
+    unsigned long long b;
+};
+SHK_FX P2 p2(float x, float y) {
+    P2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.b) : "f"(x), "f"(y));
+    return r;
+}
+SHK_FX float p2x(P2 a) {
+    return __uint_as_float(static_cast<unsigned>(a.b));
+}
+SHK_FX float p2y(P2 a) {
+    return __uint_as_float(static_cast<unsigned>(a.b >> 32));
+}
+SHK_FX P2 operator+(P2 a, P2 b) {
+    P2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
+    return r;
+}
+SHK_FX P2 operator*(P2 a, P2 b) {
+    P2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
+    return r;
+}
+SHK_FX P2 fma2(P2 a, P2 b, P2 c) {
+    P2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.b) : "l"(a.b), "l"(b.b), "l"(c.b));
+    return r;
+}
+SHK_FX float rcp1(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+SHK_FX uint32_t fbits(float x) { return __float_as_uint(x); }
+SHK_FX float bitsf(uint32_t x) { return __uint_as_float(x); }
+SHK_FX int32_t f2i(float x) { return __float2int_rn(x); }
+SHK_FX uint32_t umulhi(uint32_t a, uint32_t b) { return __umulhi(a, b); }
+SHK_FX int dhi(double x) { return __double2hiint(x); }
+SHK_FX uint32_t dlo(double x) { return static_cast<uint32_t>(__double2loint(x)); }
+SHK_FX double hilo(int hi, uint32_t lo) { return __hiloint2double(hi, static_cast<int>(lo)); }
+SHK_FX uint64_t shr64(uint64_t x, uint32_t s) {  // 0 for s >= 64
+    uint64_t r;
+    asm("shr.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+    return r;
+}
+#else
+struct P2 {
+    float x, y;
+};
+SHK_FX P2 p2(float x, float y) { return P2{x, y}; }
+SHK_FX float p2x(P2 a) { return a.x; }
+SHK_FX float p2y(P2 a) { return a.y; }
+SHK_FX P2 operator+(P2 a, P2 b) { return P2{a.x + b.x, a.y + b.y}; }
+SHK_FX P2 operator*(P2 a, P2 b) { return P2{a.x * b.x, a.y * b.y}; }
+SHK_FX P2 fma2(P2 a, P2 b, P2 c) { return P2{std::fmaf(a.x, b.x, c.x), std::fmaf(a.y, b.y, c.y)}; }
+SHK_FX float rcp1(float x) { return 1.0f / x; }
+SHK_FX uint32_t fbits(float x) { uint32_t r; std::memcpy(&r, &x, 4); return r; }
+SHK_FX float bitsf(uint32_t x) { float r; std::memcpy(&r, &x, 4); return r; }
+SHK_FX int32_t f2i(float x) { return x == x ? static_cast<int32_t>(std::nearbyintf(x)) : 0; }
+SHK_FX uint32_t umulhi(uint32_t a, uint32_t b) { return static_cast<uint32_t>((uint64_t(a) * b) >> 32); }
+SHK_FX int dhi(double x) { int64_t r; std::memcpy(&r, &x, 8); return static_cast<int>(r >> 32); }
+SHK_FX uint32_t dlo(double x) { uint64_t r; std::memcpy(&r, &x, 8); return static_cast<uint32_t>(r); }
+SHK_FX double hilo(int hi, uint32_t lo) {
+    const uint64_t r = (uint64_t(uint32_t(hi)) << 32) | lo;
+    double d;
+    std::memcpy(&d, &r, 8);
+    return d;
+}
+SHK_FX uint64_t shr64(uint64_t x, uint32_t s) { return s >= 64 ? 0 : x >> s; }
+#endif
+SHK_FX P2 dup(float x) { return p2(x, x); }
+SHK_FX P2 neg(P2 a) { return a * dup(-1.0f); }
+SHK_FX P2 sub(P2 a, P2 b) { return fma2(b, dup(-1.0f), a); }  // exactly rounded a - b
+
+// ---- unevaluated sums h + l of two floats (error-free transformations of
+// Dekker and Knuth) -------------------------------------------------------------
+struct FF {
+    P2 h, l;
+};
+SHK_FX FF add(FF a, FF b) {
+    const P2 s = a.h + b.h;
+    const P2 bb = sub(s, a.h);
+    const P2 e = sub(a.h, sub(s, bb)) + sub(b.h, bb);
+    return FF{s, e + (a.l + b.l)};
+}
+SHK_FX FF mul(FF a, FF b) {
+    const P2 p = a.h * b.h;
+    P2 e = fma2(a.h, b.h, neg(p));
+    e = fma2(a.h, b.l, e);
+    e = fma2(a.l, b.h, e);
+    return FF{p, e};
+}
+SHK_FX FF sqr(FF a) {
+    const P2 p = a.h * a.h;
+    P2 e = fma2(a.h, a.h, neg(p));
+    e = fma2(a.h + a.h, a.l, e);
+    return FF{p, e};
+}
+SHK_FX FF twice(FF a) { return FF{a.h + a.h, a.l + a.l}; }
+SHK_FX FF scale(FF a, P2 s) { return FF{a.h * s, a.l * s}; }  // s a power of two
+// n / d, sign s = +1 or -1 of the result
+SHK_FX FF quot(FF n, FF d, float s) {
+    const P2 y = p2(rcp1(p2x(d.h)), rcp1(p2y(d.h)));
+    const P2 q = n.h * y;
+    const P2 nq = neg(q);
+    P2 r = fma2(nq, d.h, n.h);
+    r = fma2(nq, d.l, r + n.l);
+    const P2 q1 = r * y;
+    return s > 0.0f ? FF{q, q1} : FF{nq, neg(q1)};
+}
+
+// ---- 64-bit integers -----------------------------------------------------------
+// magnitude and exponent of a double: m 2^(e - 1080) with m < 2^58
+struct Mag {
+    uint64_t m;
+    uint32_t e;
+    int32_t s;  // 0 or -1
+};
+SHK_FX Mag mag(double v) {
+    const uint32_t hi = static_cast<uint32_t>(dhi(v)) & 0x7fffffffu;
+    return Mag{((uint64_t((hi & 0xfffffu) | 0x100000u) << 32) | dlo(v)) << 5, hi >> 20, dhi(v) >> 31};
+}
+// |v| truncated to units of 2^(exm - 1079) (exponents up to exm + 1 fit; 0
+// stays 0, since the scale is far above the subnormals), and with its sign
+SHK_FX uint64_t fix_abs(const Mag& v, uint32_t exm) { return shr64(v.m, exm + 1u - v.e); }
+SHK_FX int64_t with_sign(uint64_t m, const Mag& v) {
+    const int64_t s = v.s;
+    return (static_cast<int64_t>(m) ^ s) - s;
+}
+// X u as two floats from pieces above bit 36, 24 bits and 12 bits (|X| < 2^60)
+SHK_FX FF to_ff(int64_t X, int64_t Y, P2 u36, P2 u12, P2 u0) {
+    const P2 h = p2(static_cast<float>(static_cast<int32_t>(X >> 36)),
+                    static_cast<float>(static_cast<int32_t>(Y >> 36))) * u36;
+    const P2 m = p2(static_cast<float>(static_cast<uint32_t>(X >> 12) & 0xffffffu),
+                    static_cast<float>(static_cast<uint32_t>(Y >> 12) & 0xffffffu));
+    const P2 l = p2(static_cast<float>(static_cast<uint32_t>(X) & 0xfffu),
+                    static_cast<float>(static_cast<uint32_t>(Y) & 0xfffu));
+    const P2 s = fma2(m, u12, h);           // |h| >= |m u12| or h = 0
+    const P2 e = fma2(m, u12, sub(h, s));   // exact
+    return FF{s, fma2(l, u0, e)};
+}
+// (third differences, |X| < 2^50: two pieces)
+SHK_FX FF to_ff50(int64_t X, int64_t Y, P2 u26, P2 u0) {
+    const P2 h = p2(static_cast<float>(static_cast<int32_t>(X >> 26)),
+                    static_cast<float>(static_cast<int32_t>(Y >> 26))) * u26;
+    const P2 l = p2(static_cast<float>(static_cast<uint32_t>(X) & 0x3ffffffu),
+                    static_cast<float>(static_cast<uint32_t>(Y) & 0x3ffffffu)) * u0;
+    const P2 s = h + l;
+    return FF{s, l + sub(h, s)};
+}
+
+// one cell c of a lane: integers in units of 2^(exm - 1079), the scale taken
+// from cells c - 1 .. c + 1
+struct Cell {
+    int64_t VV;   // v_c + v_{c+1}
+    int64_t EE;   // E_c + E_{c+1}
+    int64_t T;    // E_{c+1} - E_c
+    int64_t S, E; // v_{c+1} - v_{c-1}, E_c
+    uint64_t A;   // max(|v_c|, |v_{c+1}|)
+    float u0;     // 2^(exm - 1079)
+    float iu;     // 1 / u0
+    int kz, k;    // binary exponents of the units and of the flux units
+    bool in;      // the scale is in range
+    bool ok;      // and v_{c+2} fits it, and |T| < 2^50
+};
+SHK_FX Cell cell_begin(const Mag& vm, const Mag& v0, const Mag& v1, const Mag& v2) {
+    Cell c;
+    uint32_t exm = v0.e > v1.e ? v0.e : v1.e;
+    exm = exm > vm.e ? exm : vm.e;
+    // scales 2^-60 .. 2^60; a zero state takes the smallest
+    c.in = exm - (1023u - 60u) <= 120u || exm == 0u;
+    exm = exm == 0u || !c.in ? 1023u - 60u : exm;
+    c.u0 = bitsf((exm - 952u) << 23);
+    c.iu = bitsf((1206u - exm) << 23);
+    c.kz = static_cast<int>(exm) - 1079;
+    c.k = 2 * static_cast<int>(exm) - 2094;
+    const uint64_t A0 = fix_abs(v0, exm), A1 = fix_abs(v1, exm);
+    c.A = A0 > A1 ? A0 : A1;
+    const int64_t Vm = with_sign(fix_abs(vm, exm), vm), V0 = with_sign(A0, v0);
+    const int64_t V1 = with_sign(A1, v1), V2 = with_sign(fix_abs(v2, exm), v2);
+    const int64_t dm = V0 - Vm, d0 = V1 - V0, d1 = V2 - V1;
+    const int64_t E1 = d1 - d0;
+    c.E = d0 - dm;
+    c.S = d0 + dm;
+    c.T = E1 - c.E;
+    c.EE = c.E + E1;
+    c.VV = V0 + V1;
+    c.ok = c.in && v2.e <= exm + 1u && static_cast<uint32_t>((c.T >> 32) + 0x40000) < 0x80000u;
+    return c;
+}
+
+// the two cells c0, c0 + 1 of a lane between the exchanges with its neighbours
+struct Lane {
+    Cell x, y;
+    FF T;        // (T_{c0}, T_{c0+1}); NaN where out of range
+    FF a, b, g;  // e0 of cell k+1, e1 of cell k, e2 of cell k-1 for k = c0, c0+1
+};
+
+// part 1: from v_{c0-1} .. v_{c0+3}. Every quantity of cell c depends on its
+// own cells c-1 .. c+2 alone (not on the lane that holds it), so a flux is a
+// function of its face's six-cell stencil.
+SHK_FX Lane lane_begin(double vm, double v0, double v1, double v2, double v3, FF eps4) {
+    Lane s;
+    {
+        const Mag a = mag(vm), b = mag(v0), c = mag(v1), d = mag(v2), e = mag(v3);
+        s.x = cell_begin(a, b, c, d);
+        s.y = cell_begin(b, c, d, e);
+    }
+    const P2 u0 = p2(s.x.u0, s.y.u0);
+    const P2 u12 = u0 * dup(0x1p12f), u36 = u0 * dup(0x1p36f);
+    const FF Sf = to_ff(s.x.S, s.y.S, u36, u12, u0);
+    const FF Ef = to_ff(s.x.E, s.y.E, u36, u12, u0);
+    const float nan = bitsf(0x7fffffffu);
+    s.T = to_ff50(s.x.T, s.y.T, u0 * dup(0x1p26f), u0);
+    s.T.h = p2(s.x.ok ? p2x(s.T.h) : nan, s.y.ok ? p2y(s.T.h) : nan);
+    // b = S^2 + 13/3 E^2 + 4 eps, a / g = b + 4 E^2 +- 4 S E
+    const FF Q = sqr(Sf), W = sqr(Ef), C = mul(Sf, Ef);
+    const FF c133{dup(4.33333349f), dup(-1.58945718e-07f)};  // 13/3
+    s.b = add(add(Q, mul(W, c133)), eps4);
+    const FF base = add(s.b, scale(W, dup(4.0f)));
+    s.a = add(base, scale(C, dup(4.0f)));
+    s.g = add(base, scale(C, dup(-4.0f)));
+    s.g.h = p2(s.x.in ? p2x(s.g.h) : nan, s.y.in ? p2y(s.g.h) : nan);
+    return s;
+}
+
+// part 2: pR and pL of cells c0, c0+1 from the neighbours' am = a of cell c0-1,
+// gp = g of cell c0+2, Tm = T_{c0-1} (each as two floats)
+SHK_FX void lane_cells(const Lane& s, float amh, float aml, float gph, float gpl, float Tmh, float Tml,
+                       FF& pR, FF& pL) {
+    const FF e0{p2(amh, p2x(s.a.h)), p2(aml, p2x(s.a.l))};
+    const FF e2{p2(p2y(s.g.h), gph), p2(p2y(s.g.l), gpl)};
+    const FF Tm{p2(Tmh, p2x(s.T.h)), p2(Tml, p2x(s.T.l))};
+    const FF r0 = sqr(quot(s.b, e0, 1.0f)), r2 = sqr(quot(s.b, e2, 1.0f));
+    const FF A = mul(r0, Tm), B = mul(r2, s.T);
+    const FF X2 = twice(add(A, B));
+    const FF Y6 = add(add(r0, r2), FF{dup(6.0f), dup(0.0f)});
+    pR = quot(add(X2, B), add(Y6, twice(r2)), -1.0f);
+    pL = quot(add(X2, A), add(Y6, twice(r0)), 1.0f);
+}
+
+// p (1.0 = iu units) to units; |p| < 2^52 units
+SHK_FX int64_t p_units(float h, float l, float iu) {
+    const float x = h * iu;
+    const float magic = 0x1.8p53f;  // rounds to multiples of 2^30
+    const float t = x + magic;
+    const int32_t n = static_cast<int32_t>(fbits(t) - fbits(magic));
+    const float r = (x - (t - magic)) + l * iu;
+    return int64_t(n) * (int64_t(1) << 30) + f2i(r);
+}
+
+// Z = 6 (R + L) and D = 6 (R - L) of face c + 1/2 from its two cells'
+// corrections; false where the face is left to the FP64 formula
+SHK_FX bool face_sums(const Cell& c, float Rh, float Rl, float Lh, float Ll, int64_t& Z, int64_t& D) {
+    const float lim = 0x1p52f * c.u0;
+    const int64_t pr = p_units(Rh, Rl, c.iu), pl = p_units(Lh, Ll, c.iu);
+    Z = 6 * c.VV - c.EE + pr + pl;
+    D = c.T + pr - pl;
+#ifdef __CUDACC__
+    const bool fin = fabsf(Rh) <= lim && fabsf(Lh) <= lim;
+#else
+    const bool fin = std::fabs(Rh) <= lim && std::fabs(Lh) <= lim;
+#endif
+    return fin && D + static_cast<int64_t>(24u * c.A) >= 0;
+}
+
+// a 64-bit integer X in units of 2^k as a double (two roundings at most)
+SHK_FX double to_double(int64_t X, int k) {
+    // (2^84 + 2^63 + hi 2^32) - (2^84 + 2^63 + 2^52) + (2^52 + lo), times 2^k
+    const int ke = k * (1 << 20);
+    const double y = hilo(0x45300000 + ke, static_cast<uint32_t>(X >> 32) ^ 0x80000000u);
+    const double x = hilo(0x43300000 + ke, static_cast<uint32_t>(X));
+    const double c = hilo(0x45300000 + ke, 0x80100000u);
+    return (y - c) + x;
+}
+
+// 288 F = Z^2 + D (D + 24 a), a = A units, in units of 2^k; needs |Z| < 2^63
+// and D + 24 A >= 0. The products keep their upper 64 of 128 bits.
+SHK_FX double face_flux(uint64_t A, int k, int64_t Z, int64_t D) {
+    const uint64_t z = Z < 0 ? -static_cast<uint64_t>(Z) : static_cast<uint64_t>(Z);
+    const uint32_t zh = static_cast<uint32_t>(z >> 32), zl = static_cast<uint32_t>(z);
+    const uint64_t zz = uint64_t(zh) * zh + ((uint64_t(zh) * zl) >> 31);
+    const int64_t s = D >> 63;
+    const uint64_t dm = static_cast<uint64_t>((D ^ s) - s);
+    const uint64_t q = static_cast<uint64_t>(D) + 24u * A;
+    const uint32_t dh = static_cast<uint32_t>(dm >> 32), dl = static_cast<uint32_t>(dm);
+    const uint32_t qh = static_cast<uint32_t>(q >> 32), ql = static_cast<uint32_t>(q);
+    const uint64_t t = uint64_t(dh) * qh + umulhi(dl, qh) + umulhi(dh, ql);
+    return to_double(static_cast<int64_t>(zz) + ((static_cast<int64_t>(t) ^ s) - s), k);
+}
+
+// 288 F from face values R, L formed in double (v0, v1: the face's cells), with
+// the integer arithmetic of the other faces: next to a constant state, where R
+// = L = v, the flux equals theirs and the difference vanishes exactly. False
+// where the integers do not hold it.
+SHK_FX bool listed_flux(double R, double L, double v0, double v1, double& G) {
+    const Mag r = mag(R), l = mag(L), a = mag(v0), b = mag(v1);
+    uint32_t exm = r.e > l.e ? r.e : l.e;
+    exm = exm > a.e ? exm : a.e;
+    exm = exm > b.e ? exm : b.e;
+    if (exm == 0u) exm = 1023u - 60u;
+    if (exm - (1023u - 60u) > 120u) return false;
+    const int64_t x = with_sign(fix_abs(r, exm), r), y = with_sign(fix_abs(l, exm), l);
+    const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm), A = A0 > A1 ? A0 : A1;
+    const int64_t D = 6 * (x - y);
+    if (D + static_cast<int64_t>(24u * A) < 0) return false;
+    G = face_flux(A, 2 * static_cast<int>(exm) - 2094, 6 * (x + y), D);
+    return true;
+}
+
+}  // namespace fx
+}  // namespace shk

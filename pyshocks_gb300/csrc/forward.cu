@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : (REC ==
     using B = typename Bits<T>::type;
 
     Smem<T> sm;
-    carve_step<T, REC>(sm, smem_raw, P.tile + 2 * HL);
+    carve_step<T, REC, FLUX>(sm, smem_raw, P.tile + 2 * HL);
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_mbar_init();
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kThreads) single_step_kernel(const T* __restri
     __shared__ __align__(8) uint64_t bar;
     constexpr int HL = step_halo<T>();
     Smem<T> sm;
-    carve_step<T, REC>(sm, smem_raw, tile + 2 * HL);
+    carve_step<T, REC, FLUX>(sm, smem_raw, tile + 2 * HL);
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_mbar_init();
@@ -585,6 +585,8 @@ OpParams<T> make_params(const shk_scheme* s) {
     // FP64 Burgers-Rusanov with nu = 1 stores 4 F (see face_fluxes)
     p.fscale = (sizeof(T) == 8 && s->flux == SHK_FLUX_RUSANOV && s->rec == SHK_REC_WENOJS53 &&
                 s->equation == SHK_EQ_BURGERS && s->nu == 1.0) ? T(0.25) : T(1);
+    p.e4h = static_cast<float>(4.0 * s->eps);
+    p.e4l = static_cast<float>(4.0 * s->eps - static_cast<double>(p.e4h));
     return p;
 }
 
@@ -628,6 +630,10 @@ int dispatch_scheme(const shk_scheme* s, F&& f) {
             if (s->flux == SHK_FLUX_GODUNOV || s->flux == SHK_FLUX_EO)                  \
                 return dispatch_upwind<T>(s, f);                                        \
         }                                                                               \
+        if constexpr (EQ == SHK_EQ_BURGERS && sizeof(T) == 8) {                         \
+            if (fixed_flux_scheme(s))                                                   \
+                return f.template operator()<T, EQ, SHK_REC_WENOJS53, kFluxRusanovFx>(); \
+        }                                                                               \
         if (s->rec == SHK_REC_CONSTANT)                                                 \
             return f.template operator()<T, EQ, SHK_REC_CONSTANT, SHK_FLUX_RUSANOV>();  \
         if (s->rec == SHK_REC_WENOJS32)                                                 \
@@ -655,7 +661,7 @@ struct ApplyOpLaunch {
     const double* u; double* out; int64_t n; int g; int tile; double dx; const double* amax;
     OpParams<double> p; size_t smem; int blocks; cudaStream_t st; shk_boundary bc;
     template <class T, int EQ, int REC, int FLUX> int operator()() {
-        auto k = apply_operator_kernel<T, EQ, REC, FLUX>;
+        auto k = apply_operator_kernel<T, EQ, REC, FLUX == kFluxRusanovFx ? SHK_FLUX_RUSANOV : FLUX>;
         SHK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k<<<blocks, kThreads, smem, st>>>(u, out, n, g, tile, dx, amax, p, nullptr, bc);
         return cuda_check(cudaGetLastError());
@@ -822,7 +828,7 @@ int launch_step(shk_plan* P, const void* uin, void* uout, cudaStream_t st) {
             }
         }
     }
-    const size_t smem = Smem<T>::step_bytes(P->tile + 2 * step_halo<T>(), P->scheme.rec);
+    const size_t smem = Smem<T>::step_bytes(P->tile + 2 * step_halo<T>(), P->scheme.rec, fixed_flux_scheme(&P->scheme));
     OpParams<T> p = make_params<T>(&P->scheme);
     BatchedStepLaunch<T> f{D, static_cast<const T*>(uin), static_cast<T*>(uout), p, smem, P->grid, st};
     return dispatch_scheme<T>(&P->scheme, f);
@@ -928,7 +934,7 @@ int shk_ssprk33_step_bc_f64(const shk_scheme* scheme, const shk_boundary* bc, co
     cudaStream_t st = as_stream(stream);
     const int tile = 512;
     const int W = tile + 2 * step_halo<double>();
-    const size_t smem = Smem<double>::step_bytes(W, scheme->rec);
+    const size_t smem = Smem<double>::step_bytes(W, scheme->rec, fixed_flux_scheme(scheme));
     const int blocks = static_cast<int>((n + tile - 1) / tile);
     OpParams<double> p = make_params<double>(scheme);
     p.dx = dx;
@@ -1059,7 +1065,7 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
     int per_sm = opts && opts->ctas_per_sm > 0 ? opts->ctas_per_sm : 0;
     if (per_sm == 0) {
         const size_t smem = lf ? Smem<double>::host_bytes(tile + 2 * op_halo<double>())
-                               : (dtype == SHK_F64 ? Smem<double>::step_bytes(tile + 2 * step_halo<double>(), scheme->rec)
+                               : (dtype == SHK_F64 ? Smem<double>::step_bytes(tile + 2 * step_halo<double>(), scheme->rec, fixed_flux_scheme(scheme))
                                                    : Smem<float>::step_bytes(tile + 2 * step_halo<float>(), scheme->rec));
         int resident = 0;
         const int r = dtype == SHK_F64 ? dispatch_scheme<double>(scheme, StepOccupancy{smem, &resident})

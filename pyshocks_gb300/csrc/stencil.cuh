@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include "device.cuh"
+#include "fixed_flux.cuh"
 #include "learned.cuh"
 
 namespace shk {
@@ -28,6 +29,16 @@ constexpr int kLearnedScratch = (kThreads / 32) * kWarpScratch + 4;
 // length of the face-flux array D of the mixed step's layout (the learned
 // phase's scratch before it takes the fluxes)
 __host__ __device__ constexpr int mixed_d_len(int W) { return W > kLearnedScratch ? W : kLearnedScratch; }
+
+// The FLUX code of kernels whose Rusanov flux runs on fixed_flux.cuh: double
+// states, Burgers, WENO-JS5, nu = 1 (fixed_flux_scheme). nu enters that flux as
+// 24 a with an integer a; other nu and the other equations keep the FP64
+// formula.
+constexpr int kFluxRusanovFx = 100;
+inline bool fixed_flux_scheme(const shk_scheme* s) {
+    return s->flux == SHK_FLUX_RUSANOV && s->rec == SHK_REC_WENOJS53 &&
+           s->equation == SHK_EQ_BURGERS && s->nu == 1.0;
+}
 
 // halo of a window: 9 cells are needed for three fused stages, rounded up so
 // that the window start stays 16-byte aligned for cp.async.bulk
@@ -55,6 +66,8 @@ __device__ __forceinline__ Win<float> learned_scratch(PR region, int nfloats) {
 // ---------------------------------------------------------------------------
 // shared-memory layout of one work item (window of W cells)
 // ---------------------------------------------------------------------------
+constexpr int kFxCounters = 4;  // one per stage, padded
+
 template <class T>
 struct Smem {
     Win<T> U;   // u at the start of the step (window)
@@ -66,6 +79,7 @@ struct Smem {
     Win<T> UR;  // ur (value at the right face of the cell)
     Win<T> I;   // float states: stage increments (see step_tile); null for double
     Win<float> scr;  // the learned phase's warp scratch (free in that phase)
+    Win<int> fx;     // kFluxRusanovFx: counters of the listed faces, then the lists' storage
     int W;      // window length (cells) of every array
 
     // float states carry one more array (the stage increments)
@@ -73,7 +87,10 @@ struct Smem {
     __host__ static size_t host_bytes(int W) { return size_t(kArrays) * W * sizeof(T); }
     // the step tile of a double state with the learned reconstruction runs in
     // mixed precision (step_tile_mixed) on the double window and 6 float arrays
-    __host__ static size_t step_bytes(int W, int rec) {
+    // (kFluxRusanovFx: U, S, D = fluxes, and the list
+    // of faces left to the FP64 formula)
+    __host__ static size_t step_bytes(int W, int rec, bool fixed = false) {
+        if (sizeof(T) == 8 && fixed) return size_t(3) * W * sizeof(T) + size_t(W + kFxCounters) * sizeof(int);
         if (sizeof(T) == 8 && rec == SHK_REC_LEARNED)
             return size_t(W) * sizeof(double) + size_t(5 * W + mixed_d_len(W)) * sizeof(float);
         if (sizeof(T) == 4 && rec == SHK_REC_WENOJS53) return size_t(6) * W * sizeof(T);
@@ -88,6 +105,15 @@ struct Smem {
         H = Q = Win<T>();
         scr = Win<float>();
         this->W = W;
+    }
+    __device__ void carve_fixed(unsigned char* base, int W) {
+        T* p = reinterpret_cast<T*>(base);
+        U = make_win(p, W); S = make_win(p + W, W); D = make_win(p + 2 * W, W);
+        fx = make_win(reinterpret_cast<int*>(p + 3 * W), W + kFxCounters);
+        H = Q = UL = UR = I = Win<T>();
+        scr = Win<float>();
+        this->W = W;
+        if (threadIdx.x < kFxCounters) fx[threadIdx.x] = 0;  // (the caller's barrier follows)
     }
     // compact layout of that mixed step: U (double window), then as float
     // arrays S (2W: uf, k), I (increments), UL, UR and D (mixed_d_len(W)
@@ -128,12 +154,14 @@ struct OpParams {
     T lim_param;           // its theta / van Albada variant
     T atol;                // MUSCL slope-ratio cut
     T dx;                  // cell size (the MUSCLS van Albada variant 2 slope)
+    float e4h, e4l;        // 4 eps as the sum of two floats (kFluxRusanovFx)
 };
 
 // shared-memory layout of a step tile (see Smem::step_bytes)
-template <class T, int REC>
+template <class T, int REC, int FLUX = SHK_FLUX_RUSANOV>
 __device__ __forceinline__ void carve_step(Smem<T>& sm, unsigned char* base, int W) {
-    if constexpr (sizeof(T) == 8 && REC == SHK_REC_LEARNED) sm.carve_mixed(base, W);
+    if constexpr (FLUX == kFluxRusanovFx) sm.carve_fixed(base, W);
+    else if constexpr (sizeof(T) == 8 && REC == SHK_REC_LEARNED) sm.carve_mixed(base, W);
     else if constexpr (sizeof(T) == 4 && REC == SHK_REC_WENOJS53) sm.carve_compact(base, W);
     else sm.carve(base, W);
 }
@@ -232,6 +260,8 @@ __host__ __device__ inline OpParams<float> float_params(const OpParams<T>& p) {
     f.lim_param = static_cast<float>(p.lim_param);
     f.atol = static_cast<float>(p.atol);
     f.dx = static_cast<float>(p.dx);
+    f.e4h = p.e4h;
+    f.e4l = p.e4l;
     return f;
 }
 
@@ -699,6 +729,174 @@ __device__ unsigned int step_tile_f32_weno(const Smem<float>& sm, Win<float> gou
     return mx;
 }
 
+// ---------------------------------------------------------------------------
+// double state, Burgers + Rusanov (nu = 1) + WENO-JS5: the stages on the fluxes
+// of fixed_flux.cuh
+// ---------------------------------------------------------------------------
+// face value at the right of the middle cell of v (WENO-JS5 in product form, the
+// middle sub-stencil's value plus weighted third differences)
+__device__ __forceinline__ double weno53_side_d(double vm2, double vm1, double v, double vp1, double vp2,
+                                                double eps4) {
+    const double dm2 = vm1 - vm2, dm1 = v - vm1, d0 = vp1 - v, dp1 = vp2 - vp1;
+    const double Em = dm1 - dm2, E0 = d0 - dm1, Ep = dp1 - d0;
+    const double h0 = fma(2.0, dm1, Em), h1 = d0 + dm1, h2 = fma(-2.0, d0, Ep);
+    double s0 = fma(h0, h0, fma((13.0 / 3.0) * Em, Em, eps4)); s0 = s0 * s0;
+    double s1 = fma(h1, h1, fma((13.0 / 3.0) * E0, E0, eps4)); s1 = s1 * s1;
+    double s2 = fma(h2, h2, fma((13.0 / 3.0) * Ep, Ep, eps4)); s2 = s2 * s2;
+    const double P0 = s1 * s2, P1 = s0 * s2, P2 = s0 * s1;
+    const double cr0 = fma(2.0, h0, -dm1), cr1 = fma(12.0, d0, 6.0 * dm1), cr2 = 3.0 * (d0 - h2);
+    const double nr = fma(P0, cr0, fma(P1, cr1, P2 * cr2));
+    const double dr = fma(6.0, P0, fma(18.0, P2, 36.0 * P1));
+    return fma(nr, rcp_nr(dr), v);
+}
+
+// what the listed faces need; two lanes per face, one for each side's value
+template <class PV, class FaceOut>
+__device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list, int cnt, double eps,
+                                             FaceOut out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const double eps4 = 4.0 * eps;
+    for (int q0 = 16 * warp; q0 < cnt; q0 += 16 * nw) {
+        const int q = q0 + (lane >> 1);
+        const int j = list[q < cnt ? q : q0];
+        const int c = j + (lane & 1), o = (lane & 1) ? -1 : 1;  // cell and direction of this side
+        const double w = weno53_side_d(v[c - 2 * o], v[c - o], v[c], v[c + o], v[c + 2 * o], eps4);
+        const double w1 = __shfl_xor_sync(0xffffffffu, w, 1);
+        const double R = (lane & 1) ? w1 : w, L = (lane & 1) ? w : w1;
+        if (q < cnt && (lane & 1) == 0) {
+            double g;
+            if (!fx::listed_flux(R, L, v[j], v[j + 1], g)) {
+                const auto ab = abs_bits(v[j]) > abs_bits(v[j + 1]) ? abs_bits(v[j]) : abs_bits(v[j + 1]);
+                g = 72.0 * fma(L, L, fma(R, R, twice_abs_bits(ab) * (R - L)));
+            }
+            G[j] = g;
+            out(j, R, L);
+        }
+    }
+}
+
+struct NoFaces {
+    static constexpr bool kStore = false;
+    __device__ void operator()(int, double, double) const {}
+};
+// face values of the cells [lo, hi) of a window to ul, ur (indexed from the
+// cell `at`)
+template <class PO>
+struct StoreFaces {
+    static constexpr bool kStore = true;
+    PO ul, ur;
+    int lo, hi, at;
+    __device__ void operator()(int j, double R, double L) const {
+        if (j >= lo && j < hi) ur[j - at] = R;
+        if (j + 1 >= lo && j + 1 < hi) ul[j + 1 - at] = L;
+    }
+};
+
+// 288 F of the faces [jlo, jhi) into sm.D from v (valid on [jlo-2, jhi+3)): two
+// adjacent cells per lane, a warp covers 64 cells and the 60 faces of lanes
+// 1..30, neighbours' terms by shuffle. Faces that fixed_flux.cuh leaves go to
+// the list of counter `slot` and are evaluated after a barrier. Ends with a
+// barrier. The counter of the next stage is cleared on the way: its last
+// readers are past this stage's first barrier.
+template <class PV, class FaceOut>
+__device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<double>& sm,
+                                          const OpParams<double>& p, int slot, const FaceOut& out) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const Win<int> list = sm.fx + kFxCounters;
+    const fx::FF eps4{fx::dup(p.e4h), fx::dup(p.e4l)};
+    for (int r0 = (jlo & ~1) - 2 + 60 * warp; r0 + 2 < jhi; r0 += 60 * nw) {
+        const int c0 = r0 + 2 * lane;
+        // (positions outside the window only feed faces that are not stored)
+        const int ca = c0 < 0 ? 0 : (c0 < sm.W - 2 ? c0 : sm.W - 2);
+        const int cb = ca < sm.W - 4 ? ca + 2 : sm.W - 2;
+        const double2 a = *reinterpret_cast<const double2*>(win_span(v, ca, 2));
+        const double2 b = *reinterpret_cast<const double2*>(win_span(v, cb, 2));
+        const fx::Lane s = fx::lane_begin(v[ca > 0 ? ca - 1 : 0], a.x, a.y, b.x, b.y, eps4);
+        const float amh = __shfl_up_sync(kFull, fx::p2y(s.a.h), 1), aml = __shfl_up_sync(kFull, fx::p2y(s.a.l), 1);
+        const float gph = __shfl_down_sync(kFull, fx::p2x(s.g.h), 1), gpl = __shfl_down_sync(kFull, fx::p2x(s.g.l), 1);
+        const float Tmh = __shfl_up_sync(kFull, fx::p2y(s.T.h), 1), Tml = __shfl_up_sync(kFull, fx::p2y(s.T.l), 1);
+        fx::FF pR, pL;
+        fx::lane_cells(s, amh, aml, gph, gpl, Tmh, Tml, pR, pL);
+        const float nLh = __shfl_down_sync(kFull, fx::p2x(pL.h), 1), nLl = __shfl_down_sync(kFull, fx::p2x(pL.l), 1);
+        auto face = [&](int j, const fx::Cell& c, float Rh, float Rl, float Lh, float Ll) {
+            if (lane < 1 || lane > 30 || j < jlo || j >= jhi) return;
+            int64_t Z, D;
+            if (fx::face_sums(c, Rh, Rl, Lh, Ll, Z, D)) {
+                sm.D[j] = fx::face_flux(c.A, c.k, Z, D);
+                if constexpr (FaceOut::kStore)
+                    out(j, fx::to_double(Z + D, c.kz) * (1.0 / 12.0), fx::to_double(Z - D, c.kz) * (1.0 / 12.0));
+            } else {
+                list[atomicAdd(&sm.fx[slot], 1)] = j;
+            }
+        };
+        face(c0, s.x, fx::p2x(pR.h), fx::p2x(pR.l), fx::p2y(pL.h), fx::p2y(pL.l));
+        face(c0 + 1, s.y, fx::p2y(pR.h), fx::p2y(pR.l), nLh, nLl);
+    }
+    __syncthreads();
+    const int cnt = sm.fx[slot];
+    if (threadIdx.x == 0) {
+        sm.fx[slot == 2 ? 0 : slot + 1] = 0;
+        if (slot == 1) sm.fx[0] = 0;  // (a step may end before its third stage)
+    }
+    if (cnt > 0) {
+        fx_listed_faces(v, sm.D, list, cnt, p.eps, out);
+        __syncthreads();
+    }
+}
+
+// the reference's stage formulas (timestepping.py:312-320) on those fluxes
+__device__ __forceinline__ unsigned long long step_tile_fx(const Smem<double>& sm, Win<double> gout, int te,
+                                                           double dtdx, const OpParams<double>& p,
+                                                           const BcView& bc, int64_t g0, int64_t n,
+                                                           const StageOut<double>& so) {
+    constexpr int HL = step_halo<double>();
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const bool np = !bc.periodic();
+    if (np) apply_bc(sm.U, g0, n, 0, te + 2 * HL, bc, 0);
+    const double c = dtdx * (1.0 / 288.0);
+    auto fluxes = [&](const Win<double>& v, int lo, int hi, int slot, Win<double> ul, Win<double> ur) {
+        if (ul) fx_fluxes(v, lo - 1, hi, sm, p, slot, StoreFaces<Win<double>>{ul, ur, HL, HL + te, HL});
+        else fx_fluxes(v, lo - 1, hi, sm, p, slot, NoFaces());
+    };
+    {
+        const int lo = HL - 6, hi = HL + te + 6;
+        fluxes(sm.U, lo, hi, 0, so.ulu, so.uru);
+        for (int i = lo + tid; i < hi; i += nt) {
+            sm.S[i] = fma(c, sm.D[i - 1] - sm.D[i], sm.U[i]);
+        }
+        __syncthreads();
+        if (np) apply_bc(sm.S, g0, n, lo, hi, bc, 1);
+        store_interior(so.k1, sm.S, HL, te);
+    }
+    {
+        const int lo = HL - 3, hi = HL + te + 3;
+        fluxes(sm.S, lo, hi, 1, so.ul1, so.ur1);
+        for (int i = lo + tid; i < hi; i += nt) {
+            const double k = fma(c, sm.D[i - 1] - sm.D[i], sm.S[i]);
+            sm.S[i] = fma(1.0 / 4.0, k, (3.0 / 4.0) * sm.U[i]);
+        }
+        __syncthreads();
+        if (np) apply_bc(sm.S, g0, n, lo, hi, bc, 2);
+        store_interior(so.k2, sm.S, HL, te);
+    }
+    unsigned long long mx = 0;
+    if (!gout && !so.ul2) return mx;
+    {
+        const int lo = HL, hi = HL + te;
+        fluxes(sm.S, lo, hi, 2, so.ul2, so.ur2);
+        if (!gout) return mx;
+        for (int i = lo + tid; i < hi; i += nt) {
+            const double k = fma(c, sm.D[i - 1] - sm.D[i], sm.S[i]);
+            const double un = fma(2.0 / 3.0, k, (1.0 / 3.0) * sm.U[i]);
+            gout[i - HL] = un;
+            const unsigned long long b = abs_bits(un);
+            mx = b > mx ? b : mx;
+        }
+    }
+    return mx;
+}
+
 // g0: global cell of window position 0 (s - HL); n: cells of the instance;
 // bc: its boundary (periodic: nothing to overwrite)
 // so: what the reverse sweep keeps of this step (StageOut); gout may then be
@@ -708,6 +906,9 @@ __device__ typename Bits<T>::type step_tile(const Smem<T>& sm, Win<T> gout, int 
                                             const OpParams<T>& p, const BcView& bc = BcView(),
                                             int64_t g0 = 0, int64_t n = 0,
                                             const StageOut<stage_t<T, REC>>& so = StageOut<stage_t<T, REC>>()) {
+    if constexpr (FLUX == kFluxRusanovFx) {
+        return step_tile_fx(sm, gout, te, dtdx, p, bc, g0, n, so);
+    } else {
     if constexpr (sizeof(T) == 8 && REC == SHK_REC_LEARNED)
         return step_tile_mixed<EQ, FLUX>(sm, gout, te, dtdx, p, bc, g0, n, so);
     if constexpr (sizeof(T) == 4 && REC == SHK_REC_WENOJS53 && FLUX == SHK_FLUX_RUSANOV)
@@ -804,6 +1005,7 @@ __device__ typename Bits<T>::type step_tile(const Smem<T>& sm, Win<T> gout, int 
         }
     }
     return mx;
+    }
 }
 
 // device view of a batched plan (see shk_plan in forward.cu)
