@@ -64,6 +64,11 @@ SHK_FX P2 operator*(P2 a, P2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
     return r;
 }
+SHK_FX P2 operator-(P2 a, P2 b) {
+    P2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
+    return r;
+}
 SHK_FX P2 fma2(P2 a, P2 b, P2 c) {
     P2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.b) : "l"(a.b), "l"(b.b), "l"(c.b));
@@ -78,6 +83,7 @@ SHK_FX uint32_t fbits(float x) { return __float_as_uint(x); }
 SHK_FX float bitsf(uint32_t x) { return __uint_as_float(x); }
 SHK_FX int32_t f2i(float x) { return __float2int_rn(x); }
 SHK_FX uint32_t umulhi(uint32_t a, uint32_t b) { return __umulhi(a, b); }
+SHK_FX uint32_t clz32(uint32_t a) { return static_cast<uint32_t>(__clz(static_cast<int>(a))); }
 SHK_FX int dhi(double x) { return __double2hiint(x); }
 SHK_FX uint32_t dlo(double x) { return static_cast<uint32_t>(__double2loint(x)); }
 SHK_FX double hilo(int hi, uint32_t lo) { return __hiloint2double(hi, static_cast<int>(lo)); }
@@ -94,12 +100,14 @@ SHK_FX P2 p2(float x, float y) { return P2{x, y}; }
 SHK_FX float p2x(P2 a) { return a.x; }
 SHK_FX float p2y(P2 a) { return a.y; }
 SHK_FX P2 operator+(P2 a, P2 b) { return P2{a.x + b.x, a.y + b.y}; }
+SHK_FX P2 operator-(P2 a, P2 b) { return P2{a.x - b.x, a.y - b.y}; }
 SHK_FX P2 operator*(P2 a, P2 b) { return P2{a.x * b.x, a.y * b.y}; }
 SHK_FX P2 fma2(P2 a, P2 b, P2 c) { return P2{std::fmaf(a.x, b.x, c.x), std::fmaf(a.y, b.y, c.y)}; }
 SHK_FX float rcp1(float x) { return 1.0f / x; }
 SHK_FX uint32_t fbits(float x) { uint32_t r; std::memcpy(&r, &x, 4); return r; }
 SHK_FX float bitsf(uint32_t x) { float r; std::memcpy(&r, &x, 4); return r; }
 SHK_FX int32_t f2i(float x) { return x == x ? static_cast<int32_t>(std::nearbyintf(x)) : 0; }
+SHK_FX uint32_t clz32(uint32_t a) { return a ? static_cast<uint32_t>(__builtin_clz(a)) : 32u; }
 SHK_FX uint32_t umulhi(uint32_t a, uint32_t b) { return static_cast<uint32_t>((uint64_t(a) * b) >> 32); }
 SHK_FX int dhi(double x) { int64_t r; std::memcpy(&r, &x, 8); return static_cast<int>(r >> 32); }
 SHK_FX uint32_t dlo(double x) { uint64_t r; std::memcpy(&r, &x, 8); return static_cast<uint32_t>(r); }
@@ -113,7 +121,6 @@ SHK_FX uint64_t shr64(uint64_t x, uint32_t s) { return s >= 64 ? 0 : x >> s; }
 #endif
 SHK_FX P2 dup(float x) { return p2(x, x); }
 SHK_FX P2 neg(P2 a) { return a * dup(-1.0f); }
-SHK_FX P2 sub(P2 a, P2 b) { return fma2(b, dup(-1.0f), a); }  // exactly rounded a - b
 
 // ---- unevaluated sums h + l of two floats (error-free transformations of
 // Dekker and Knuth) -------------------------------------------------------------
@@ -122,8 +129,14 @@ struct FF {
 };
 SHK_FX FF add(FF a, FF b) {
     const P2 s = a.h + b.h;
-    const P2 bb = sub(s, a.h);
-    const P2 e = sub(a.h, sub(s, bb)) + sub(b.h, bb);
+    const P2 bb = s - a.h;
+    const P2 e = (a.h - (s - bb)) + (b.h - bb);
+    return FF{s, e + (a.l + b.l)};
+}
+// |a| >= |b|
+SHK_FX FF add_ordered(FF a, FF b) {
+    const P2 s = a.h + b.h;
+    const P2 e = b.h - (s - a.h);
     return FF{s, e + (a.l + b.l)};
 }
 SHK_FX FF mul(FF a, FF b) {
@@ -179,7 +192,7 @@ SHK_FX FF to_ff(int64_t X, int64_t Y, P2 u36, P2 u12, P2 u0) {
     const P2 l = p2(static_cast<float>(static_cast<uint32_t>(X) & 0xfffu),
                     static_cast<float>(static_cast<uint32_t>(Y) & 0xfffu));
     const P2 s = fma2(m, u12, h);           // |h| >= |m u12| or h = 0
-    const P2 e = fma2(m, u12, sub(h, s));   // exact
+    const P2 e = fma2(m, u12, h - s);   // exact
     return FF{s, fma2(l, u0, e)};
 }
 // (third differences, |X| < 2^50: two pieces)
@@ -189,7 +202,7 @@ SHK_FX FF to_ff50(int64_t X, int64_t Y, P2 u26, P2 u0) {
     const P2 l = p2(static_cast<float>(static_cast<uint32_t>(X) & 0x3ffffffu),
                     static_cast<float>(static_cast<uint32_t>(Y) & 0x3ffffffu)) * u0;
     const P2 s = h + l;
-    return FF{s, l + sub(h, s)};
+    return FF{s, l + (h - s)};
 }
 
 // one cell c of a lane: integers in units of 2^(exm - 1079), the scale taken
@@ -260,9 +273,10 @@ SHK_FX Lane lane_begin(double vm, double v0, double v1, double v2, double v3, FF
     const FF Q = sqr(Sf), W = sqr(Ef), C = mul(Sf, Ef);
     const FF c133{dup(4.33333349f), dup(-1.58945718e-07f)};  // 13/3
     s.b = add(add(Q, mul(W, c133)), eps4);
-    const FF base = add(s.b, scale(W, dup(4.0f)));
-    s.a = add(base, scale(C, dup(4.0f)));
-    s.g = add(base, scale(C, dup(-4.0f)));
+    // (b >= 13/3 W, and b + 4 W >= 2 sqrt(25/3) |S E| > 4 |S E|)
+    const FF base = add_ordered(s.b, scale(W, dup(4.0f)));
+    s.a = add_ordered(base, scale(C, dup(4.0f)));
+    s.g = add_ordered(base, scale(C, dup(-4.0f)));
     s.g.h = p2(s.x.in ? p2x(s.g.h) : nan, s.y.in ? p2y(s.g.h) : nan);
     return s;
 }
@@ -282,54 +296,73 @@ SHK_FX void lane_cells(const Lane& s, float amh, float aml, float gph, float gpl
     pL = quot(add(X2, A), add(Y6, twice(r0)), 1.0f);
 }
 
-// p (1.0 = iu units) to units; |p| < 2^52 units
-SHK_FX int64_t p_units(float h, float l, float iu) {
-    const float x = h * iu;
-    const float magic = 0x1.8p53f;  // rounds to multiples of 2^30
-    const float t = x + magic;
-    const int32_t n = static_cast<int32_t>(fbits(t) - fbits(magic));
-    const float r = (x - (t - magic)) + l * iu;
-    return int64_t(n) * (int64_t(1) << 30) + f2i(r);
+// the sums and differences of the corrections of a lane's two faces, pR + pL
+// and pR - pL, in units: n 2^30 + r each, |p| < 2^52 units
+struct Sums {
+    P2 xR, xL;  // pR, pL in units
+    P2 tR, tL;  // rounded to multiples of 2^30, plus the rounding constant
+    P2 rs, rd;  // sum and difference of the rests
+};
+constexpr float kRound30 = 0x1.8p53f;
+SHK_FX Sums face_units(FF pR, FF pL, P2 iu) {
+    Sums u;
+    u.xR = pR.h * iu;
+    u.xL = pL.h * iu;
+    u.tR = u.xR + dup(kRound30);
+    u.tL = u.xL + dup(kRound30);
+    const P2 rR = fma2(pR.l, iu, u.xR - (u.tR - dup(kRound30)));
+    const P2 rL = fma2(pL.l, iu, u.xL - (u.tL - dup(kRound30)));
+    u.rs = rR + rL;
+    u.rd = rR - rL;
+    return u;
 }
 
-// Z = 6 (R + L) and D = 6 (R - L) of face c + 1/2 from its two cells'
-// corrections; false where the face is left to the FP64 formula
-SHK_FX bool face_sums(const Cell& c, float Rh, float Rl, float Lh, float Ll, int64_t& Z, int64_t& D) {
-    const float lim = 0x1p52f * c.u0;
-    const int64_t pr = p_units(Rh, Rl, c.iu), pl = p_units(Lh, Ll, c.iu);
-    Z = 6 * c.VV - c.EE + pr + pl;
-    D = c.T + pr - pl;
+// Z = 6 (R + L), D = 6 (R - L) and Q = D + 24 a of face c + 1/2; false where the
+// face is left to the FP64 formula
+SHK_FX bool face_sums(const Cell& c, float xR, float xL, float tR, float tL, float rs, float rd, int64_t& Z,
+                      int64_t& D, int64_t& Q) {
+    const int32_t bR = static_cast<int32_t>(fbits(tR)), bL = static_cast<int32_t>(fbits(tL));
+    const int32_t ns = bR + (bL - 2 * static_cast<int32_t>(0x5a400000)), nd = bR - bL;
+    Z = int64_t(ns) * (int64_t(1) << 30) + (6 * c.VV - c.EE) + f2i(rs);
+    D = int64_t(nd) * (int64_t(1) << 30) + c.T + f2i(rd);
+    Q = D + static_cast<int64_t>(24u * c.A);
 #ifdef __CUDACC__
-    const bool fin = fabsf(Rh) <= lim && fabsf(Lh) <= lim;
+    const float x = fabsf(xR) + fabsf(xL);
 #else
-    const bool fin = std::fabs(Rh) <= lim && std::fabs(Lh) <= lim;
+    const float x = std::fabs(xR) + std::fabs(xL);
 #endif
-    return fin && D + static_cast<int64_t>(24u * c.A) >= 0;
+    return x <= 0x1p52f && Q >= 0;
 }
 
-// a 64-bit integer X in units of 2^k as a double (two roundings at most)
+// a 64-bit integer X in units of 2^k as a double, rounded to nearest (ties
+// away), on the integer pipe
+SHK_FX double pack_double(uint32_t hi, uint32_t lo, int e, uint32_t sign) {
+    const uint32_t n = clz32(hi);
+    const uint64_t t = ((uint64_t(hi) << 32) | lo) << n;  // top bit set
+    // the top bit adds one to the exponent field, a rounding carry likewise
+    const uint64_t bits = (t >> 11) + ((t >> 10) & 1u) + (uint64_t(uint32_t(e) - n) << 52);
+    return hilo(static_cast<int>(static_cast<uint32_t>(bits >> 32) | sign), static_cast<uint32_t>(bits));
+}
 SHK_FX double to_double(int64_t X, int k) {
-    // (2^84 + 2^63 + hi 2^32) - (2^84 + 2^63 + 2^52) + (2^52 + lo), times 2^k
-    const int ke = k * (1 << 20);
-    const double y = hilo(0x45300000 + ke, static_cast<uint32_t>(X >> 32) ^ 0x80000000u);
-    const double x = hilo(0x43300000 + ke, static_cast<uint32_t>(X));
-    const double c = hilo(0x45300000 + ke, 0x80100000u);
-    return (y - c) + x;
+    const int e = 1022 + 63 + k;
+    if (static_cast<int32_t>(X >> 32) > 0)
+        return pack_double(static_cast<uint32_t>(X >> 32), static_cast<uint32_t>(X), e, 0u);
+    const uint32_t s = X < 0 ? 0x80000000u : 0u;
+    const uint64_t m = X < 0 ? -static_cast<uint64_t>(X) : static_cast<uint64_t>(X);
+    const uint32_t hi = static_cast<uint32_t>(m >> 32), lo = static_cast<uint32_t>(m);
+    if (hi != 0u) return pack_double(hi, lo, e, s);
+    return lo != 0u ? pack_double(lo, 0u, e - 32, s) : 0.0;
 }
 
-// 288 F = Z^2 + D (D + 24 a), a = A units, in units of 2^k; needs |Z| < 2^63
-// and D + 24 A >= 0. The products keep their upper 64 of 128 bits.
-SHK_FX double face_flux(uint64_t A, int k, int64_t Z, int64_t D) {
-    const uint64_t z = Z < 0 ? -static_cast<uint64_t>(Z) : static_cast<uint64_t>(Z);
-    const uint32_t zh = static_cast<uint32_t>(z >> 32), zl = static_cast<uint32_t>(z);
-    const uint64_t zz = uint64_t(zh) * zh + ((uint64_t(zh) * zl) >> 31);
-    const int64_t s = D >> 63;
-    const uint64_t dm = static_cast<uint64_t>((D ^ s) - s);
-    const uint64_t q = static_cast<uint64_t>(D) + 24u * A;
-    const uint32_t dh = static_cast<uint32_t>(dm >> 32), dl = static_cast<uint32_t>(dm);
-    const uint32_t qh = static_cast<uint32_t>(q >> 32), ql = static_cast<uint32_t>(q);
-    const uint64_t t = uint64_t(dh) * qh + umulhi(dl, qh) + umulhi(dh, ql);
-    return to_double(static_cast<int64_t>(zz) + ((static_cast<int64_t>(t) ^ s) - s), k);
+// 288 F = Z^2 + D Q, in units of 2^k: the upper 64 of 128 bits of each product
+// (0 <= Q < 2^63)
+SHK_FX double face_flux(int k, int64_t Z, int64_t D, int64_t Q) {
+    const int32_t zh = static_cast<int32_t>(Z >> 32), dh = static_cast<int32_t>(D >> 32);
+    const int32_t zl = static_cast<int32_t>(static_cast<uint32_t>(Z) >> 1);
+    const int32_t qh = static_cast<int32_t>(Q >> 32), ql = static_cast<int32_t>(static_cast<uint32_t>(Q) >> 1);
+    const int64_t zz = int64_t(zh) * zh + ((int64_t(zh) * zl) >> 30);
+    const int64_t dq = int64_t(dh) * qh + ((int64_t(dh) * ql) >> 31) + umulhi(static_cast<uint32_t>(D), static_cast<uint32_t>(qh));
+    return to_double(zz + dq, k);
 }
 
 // 288 F from face values R, L formed in double (v0, v1: the face's cells), with
@@ -345,9 +378,9 @@ SHK_FX bool listed_flux(double R, double L, double v0, double v1, double& G) {
     if (exm - (1023u - 60u) > 120u) return false;
     const int64_t x = with_sign(fix_abs(r, exm), r), y = with_sign(fix_abs(l, exm), l);
     const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm), A = A0 > A1 ? A0 : A1;
-    const int64_t D = 6 * (x - y);
-    if (D + static_cast<int64_t>(24u * A) < 0) return false;
-    G = face_flux(A, 2 * static_cast<int>(exm) - 2094, 6 * (x + y), D);
+    const int64_t D = 6 * (x - y), Q = D + static_cast<int64_t>(24u * A);
+    if (Q < 0) return false;
+    G = face_flux(2 * static_cast<int>(exm) - 2094, 6 * (x + y), D, Q);
     return true;
 }
 

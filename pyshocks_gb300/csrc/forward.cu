@@ -55,7 +55,7 @@ __device__ void finalize_step(const PlanDev& P, int64_t k) {
 }
 
 template <class T, int EQ, int REC, int FLUX>
-__global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : (REC == SHK_REC_WENOJS53 ? (sizeof(T) == 8 ? 3 : 4) : 1)) batched_step_kernel(PlanDev P, const T* __restrict__ uin,
+__global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ? 8 : (REC == SHK_REC_LEARNED ? 3 : (REC == SHK_REC_WENOJS53 ? (sizeof(T) == 8 ? 3 : 4) : 1))) batched_step_kernel(PlanDev P, const T* __restrict__ uin,
                                                                 T* __restrict__ uout, OpParams<T> p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
@@ -512,7 +512,7 @@ int default_tile(const shk_scheme* s, int dtype, int max_steps) {
     if (s->rec == SHK_REC_LEARNED) return max_steps > 0 ? 1024 : 2048;
     if (s->rec == SHK_REC_WENOJS53 && s->flux == SHK_FLUX_RUSANOV) {
         if (dtype == SHK_F32) return max_steps > 0 ? 1024 : 2048;
-        return max_steps > 0 ? 512 : kDefaultTile;
+        return max_steps > 0 ? 512 : (fixed_flux_scheme(s) ? 946 : kDefaultTile);
     }
     return kDefaultTile;
 }
@@ -692,7 +692,7 @@ struct BatchedStepLaunch {
         } else {
             auto k = batched_step_kernel<T, EQ, REC, FLUX>;
             SHK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k<<<grid, kThreads, smem, st>>>(D, uin, uout, p);
+            k<<<grid, flux_threads<FLUX>(), smem, st>>>(D, uin, uout, p);
             return cuda_check(cudaGetLastError());
         }
     }
@@ -735,7 +735,7 @@ struct StepOccupancy {
         } else {
             auto k = batched_step_kernel<T, EQ, REC, FLUX>;
             SHK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            SHK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, kThreads, smem));
+            SHK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, flux_threads<FLUX>(), smem));
             return SHK_OK;
         }
     }

@@ -17,6 +17,7 @@
 namespace shk {
 
 constexpr int kThreads = 256;
+
 constexpr int kDefaultTile = 1024;
 // shortest tile of a plan with the learned reconstruction: its warp scratch
 // (8 warps x 128 floats forward, x 192 in the reverse step) lives in window
@@ -35,6 +36,9 @@ __host__ __device__ constexpr int mixed_d_len(int W) { return W > kLearnedScratc
 // 24 a with an integer a; other nu and the other equations keep the FP64
 // formula.
 constexpr int kFluxRusanovFx = 100;
+constexpr int kFxThreads = 128;
+template <int FLUX>
+__host__ __device__ constexpr int flux_threads() { return FLUX == kFluxRusanovFx ? kFxThreads : kThreads; }
 inline bool fixed_flux_scheme(const shk_scheme* s) {
     return s->flux == SHK_FLUX_RUSANOV && s->rec == SHK_REC_WENOJS53 &&
            s->equation == SHK_EQ_BURGERS && s->nu == 1.0;
@@ -770,20 +774,15 @@ __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list,
                 g = 72.0 * fma(L, L, fma(R, R, twice_abs_bits(ab) * (R - L)));
             }
             G[j] = g;
-            out(j, R, L);
+            if (out.ul) out(j, R, L);
         }
     }
 }
 
-struct NoFaces {
-    static constexpr bool kStore = false;
-    __device__ void operator()(int, double, double) const {}
-};
 // face values of the cells [lo, hi) of a window to ul, ur (indexed from the
-// cell `at`)
+// cell `at`; null: not wanted)
 template <class PO>
 struct StoreFaces {
-    static constexpr bool kStore = true;
     PO ul, ur;
     int lo, hi, at;
     __device__ void operator()(int j, double R, double L) const {
@@ -819,19 +818,31 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
         fx::FF pR, pL;
         fx::lane_cells(s, amh, aml, gph, gpl, Tmh, Tml, pR, pL);
         const float nLh = __shfl_down_sync(kFull, fx::p2x(pL.h), 1), nLl = __shfl_down_sync(kFull, fx::p2x(pL.l), 1);
-        auto face = [&](int j, const fx::Cell& c, float Rh, float Rl, float Lh, float Ll) {
-            if (lane < 1 || lane > 30 || j < jlo || j >= jhi) return;
-            int64_t Z, D;
-            if (fx::face_sums(c, Rh, Rl, Lh, Ll, Z, D)) {
-                sm.D[j] = fx::face_flux(c.A, c.k, Z, D);
-                if constexpr (FaceOut::kStore)
+        // faces c0 and c0 + 1: R from the lane's two cells, L from cell c0 + 1 and
+        // the next lane's first
+        const fx::Sums u = fx::face_units(pR, fx::FF{fx::p2(fx::p2y(pL.h), nLh), fx::p2(fx::p2y(pL.l), nLl)},
+                                          fx::p2(s.x.iu, s.y.iu));
+        const bool inner = lane >= 1 && lane <= 30;
+        const bool m0 = inner && c0 >= jlo && c0 < jhi, m1 = inner && c0 + 1 >= jlo && c0 + 1 < jhi;
+        // (the flux of a face left to the list is overwritten after the barrier)
+        auto face = [&](int j, const fx::Cell& c, bool mine, float xR, float xL, float tR, float tL, float rs,
+                        float rd) -> double {
+            int64_t Z, D, Q;
+            const bool ok = fx::face_sums(c, xR, xL, tR, tL, rs, rd, Z, D, Q);
+            if (mine) {
+                if (!ok) list[atomicAdd(&sm.fx[slot], 1)] = j;
+                else if (out.ul)
                     out(j, fx::to_double(Z + D, c.kz) * (1.0 / 12.0), fx::to_double(Z - D, c.kz) * (1.0 / 12.0));
-            } else {
-                list[atomicAdd(&sm.fx[slot], 1)] = j;
             }
+            return fx::face_flux(c.k, Z, D, Q);
         };
-        face(c0, s.x, fx::p2x(pR.h), fx::p2x(pR.l), fx::p2y(pL.h), fx::p2y(pL.l));
-        face(c0 + 1, s.y, fx::p2y(pR.h), fx::p2y(pR.l), nLh, nLl);
+        const double f0 = face(c0, s.x, m0, fx::p2x(u.xR), fx::p2x(u.xL), fx::p2x(u.tR), fx::p2x(u.tL),
+                               fx::p2x(u.rs), fx::p2x(u.rd));
+        const double f1 = face(c0 + 1, s.y, m1, fx::p2y(u.xR), fx::p2y(u.xL), fx::p2y(u.tR), fx::p2y(u.tL),
+                               fx::p2y(u.rs), fx::p2y(u.rd));
+        if (m0 && m1) *reinterpret_cast<double2*>(win_span(sm.D, c0, 2)) = make_double2(f0, f1);
+        else if (m0) sm.D[c0] = f0;
+        else if (m1) sm.D[c0 + 1] = f1;
     }
     __syncthreads();
     const int cnt = sm.fx[slot];
@@ -845,7 +856,9 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
     }
 }
 
-// the reference's stage formulas (timestepping.py:312-320) on those fluxes
+// the reference's stage formulas (timestepping.py:312-320) on those fluxes, in
+// one loop over the stages: the flux code is long, and three copies of it
+// missed the instruction cache
 __device__ __forceinline__ unsigned long long step_tile_fx(const Smem<double>& sm, Win<double> gout, int te,
                                                            double dtdx, const OpParams<double>& p,
                                                            const BcView& bc, int64_t g0, int64_t n,
@@ -855,44 +868,52 @@ __device__ __forceinline__ unsigned long long step_tile_fx(const Smem<double>& s
     const bool np = !bc.periodic();
     if (np) apply_bc(sm.U, g0, n, 0, te + 2 * HL, bc, 0);
     const double c = dtdx * (1.0 / 288.0);
-    auto fluxes = [&](const Win<double>& v, int lo, int hi, int slot, Win<double> ul, Win<double> ur) {
-        if (ul) fx_fluxes(v, lo - 1, hi, sm, p, slot, StoreFaces<Win<double>>{ul, ur, HL, HL + te, HL});
-        else fx_fluxes(v, lo - 1, hi, sm, p, slot, NoFaces());
-    };
-    {
-        const int lo = HL - 6, hi = HL + te + 6;
-        fluxes(sm.U, lo, hi, 0, so.ulu, so.uru);
-        for (int i = lo + tid; i < hi; i += nt) {
-            sm.S[i] = fma(c, sm.D[i - 1] - sm.D[i], sm.U[i]);
-        }
-        __syncthreads();
-        if (np) apply_bc(sm.S, g0, n, lo, hi, bc, 1);
-        store_interior(so.k1, sm.S, HL, te);
-    }
-    {
-        const int lo = HL - 3, hi = HL + te + 3;
-        fluxes(sm.S, lo, hi, 1, so.ul1, so.ur1);
-        for (int i = lo + tid; i < hi; i += nt) {
-            const double k = fma(c, sm.D[i - 1] - sm.D[i], sm.S[i]);
-            sm.S[i] = fma(1.0 / 4.0, k, (3.0 / 4.0) * sm.U[i]);
-        }
-        __syncthreads();
-        if (np) apply_bc(sm.S, g0, n, lo, hi, bc, 2);
-        store_interior(so.k2, sm.S, HL, te);
-    }
     unsigned long long mx = 0;
-    if (!gout && !so.ul2) return mx;
-    {
-        const int lo = HL, hi = HL + te;
-        fluxes(sm.S, lo, hi, 2, so.ul2, so.ur2);
-        if (!gout) return mx;
-        for (int i = lo + tid; i < hi; i += nt) {
-            const double k = fma(c, sm.D[i - 1] - sm.D[i], sm.S[i]);
-            const double un = fma(2.0 / 3.0, k, (1.0 / 3.0) * sm.U[i]);
-            gout[i - HL] = un;
-            const unsigned long long b = abs_bits(un);
-            mx = b > mx ? b : mx;
+#pragma unroll 1
+    for (int s = 0; s < 3; ++s) {
+        if (s == 2 && !gout && !so.ul2) break;
+        const int lo = HL - 6 + 3 * s, hi = HL + te + 6 - 3 * s;
+        const Win<double> v = s == 0 ? sm.U : sm.S;
+        const Win<double> ul = s == 0 ? so.ulu : (s == 1 ? so.ul1 : so.ul2);
+        const Win<double> ur = s == 0 ? so.uru : (s == 1 ? so.ur1 : so.ur2);
+        fx_fluxes(v, lo - 1, hi, sm, p, s, StoreFaces<Win<double>>{ul, ur, HL, HL + te, HL});
+        if (s == 2 && !gout) break;
+        // the stage formula at the cells i, i + 1 (i even; hi <= W - 4): one value
+        // per cell, vector accesses
+        auto ld2 = [](const Win<double>& a, int i) { return *reinterpret_cast<const double2*>(win_span(a, i, 2)); };
+        for (int i = (lo & ~1) + 2 * tid; i < hi; i += 2 * nt) {
+            const double2 f = ld2(sm.D, i), u = ld2(sm.U, i);
+            const double r0 = sm.D[i - 1] - f.x, r1 = f.x - f.y;
+            double2 w;
+            if (s == 0) {
+                w = make_double2(fma(c, r0, u.x), fma(c, r1, u.y));
+            } else {
+                const double2 k = ld2(sm.S, i);
+                const double a = s == 1 ? 1.0 / 4.0 : 2.0 / 3.0, b = s == 1 ? 3.0 / 4.0 : 1.0 / 3.0;
+                w = make_double2(fma(a, fma(c, r0, k.x), b * u.x), fma(a, fma(c, r1, k.y), b * u.y));
+            }
+            const bool v0 = i >= lo, v1 = i + 1 < hi;
+            if (s < 2) {
+                if (v0 && v1) *reinterpret_cast<double2*>(win_span(sm.S, i, 2)) = w;
+                else if (v0) sm.S[i] = w.x;
+                else sm.S[i + 1] = w.y;
+            } else {
+                if (v0) {
+                    gout[i - HL] = w.x;
+                    const unsigned long long b0 = abs_bits(w.x);
+                    mx = b0 > mx ? b0 : mx;
+                }
+                if (v1) {
+                    gout[i + 1 - HL] = w.y;
+                    const unsigned long long b1 = abs_bits(w.y);
+                    mx = b1 > mx ? b1 : mx;
+                }
+            }
         }
+        if (s == 2) break;
+        __syncthreads();
+        if (np) apply_bc(sm.S, g0, n, lo, hi, bc, s + 1);
+        store_interior(s == 0 ? so.k1 : so.k2, sm.S, HL, te);
     }
     return mx;
 }
