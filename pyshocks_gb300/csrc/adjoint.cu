@@ -544,17 +544,14 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED || FLUX == kF
     uint32_t phase = 0;
     const Win<const T> gpnext = make_win(pnext, total);
     const Win<T> gpout = make_win(pout, total);
-    __shared__ int s_item;
-    for (int item = next_item(P, 2, &s_item); item >= 0; item = next_item(P, 2, &s_item)) {
-        const int b = P.item_inst[item];
-        const int64_t off = P.offsets[b];
-        const int64_t n = P.offsets[b + 1] - off;
-        const int64_t s0 = int64_t(P.item_tile[item]) * P.tile;
-        const int te = static_cast<int>(imin64(P.tile, n - s0));
+    __shared__ int s_item[2];
+    for (ItemQueue items(P, 2, s_item); items.more(); items.end()) {
+        const PlanItem it = items.begin();
+        const int b = it.b, te = it.te;
+        const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
         const double dt = dt_row[b];
         if (dt == 0.0) {  // no step was taken: identity
             for (int i = threadIdx.x; i < te; i += blockDim.x) gpout[off + s0 + i] = gpnext[off + s0 + i];
-            __syncthreads();
             continue;
         }
         if (!adjoint_load<T>(a, um + off, pnext + off, n, s0, te, &bar, phase)) {
@@ -598,18 +595,15 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : (FLUX =
     uint32_t phase = 0;
     const Win<const T> guin = make_win(uin, total);
     const Win<T> guout = make_win(uout, total);
-    __shared__ int s_item;
-    for (int item = next_item(P, 4, &s_item); item >= 0; item = next_item(P, 4, &s_item)) {
-        const int b = P.item_inst[item];
-        const int64_t off = P.offsets[b];
-        const int64_t n = P.offsets[b + 1] - off;
-        const int64_t s0 = int64_t(P.item_tile[item]) * P.tile;
-        const int te = static_cast<int>(imin64(P.tile, n - s0));
+    __shared__ int s_item[2];
+    for (ItemQueue items(P, 4, s_item); items.more(); items.end()) {
+        const PlanItem it = items.begin();
+        const int b = it.b, te = it.te;
+        const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
         const double dt = dt_row[b];
         if (dt == 0.0) {  // no step: the reverse step is the identity, stage states unused
             if (uout)
                 for (int i = threadIdx.x; i < te; i += blockDim.x) guout[off + s0 + i] = guin[off + s0 + i];
-            __syncthreads();
             continue;
         }
         if (!load_window<T>(sm.U, uin + off, n, s0 - HL, te + 2 * HL, &bar, phase)) {

@@ -35,23 +35,27 @@ namespace shk {
 // ---------------------------------------------------------------------------
 // batched persistent stepping kernel
 // ---------------------------------------------------------------------------
-__device__ void finalize_step(const PlanDev& P, int64_t k) {
-    const int cur = static_cast<int>(k & 1);
-    for (int b = threadIdx.x; b < P.B; b += blockDim.x) {
-        unsigned long long* am = P.amax + size_t(cur) * P.B + b;
-        const DtState s = plan_dt(P, k, b, from_bits(*am));
-        double rec = 0.0;
-        if (s.active) {
-            if (s.finite) {
-                P.t[b] = P.t[b] + s.dt;
-                rec = s.dt;
-            } else {
-                atomicOr(P.status, ERR_NONFINITE);
-            }
+// One thread, when a tile of instance b is done in step k (s: the instance's
+// step). The CTA that finishes the instance's last tile advances its time,
+// records dt and clears the consumed maximum (every other tile has read both),
+// so the steps of thousands of instances are not finalised by one CTA after all
+// others are done. True for that last tile.
+__device__ __forceinline__ bool finish_tile(const PlanDev& P, int64_t k, int b, int tiles, const DtState& s) {
+    __threadfence();
+    if (atomicAdd(P.left + b, 1u) != static_cast<unsigned>(tiles) - 1u) return false;
+    P.left[b] = 0u;
+    double rec = 0.0;
+    if (s.active) {
+        if (s.finite) {
+            P.t[b] = P.t[b] + s.dt;
+            rec = s.dt;
+        } else {
+            atomicOr(P.status, ERR_NONFINITE);
         }
-        if (P.dt_hist && k < P.max_steps) P.dt_hist[size_t(k) * P.B + b] = rec;
-        *am = 0ull;
     }
+    if (P.dt_hist && k < P.max_steps) P.dt_hist[size_t(k) * P.B + b] = rec;
+    P.amax[size_t(k & 1) * P.B + b] = 0ull;
+    return true;
 }
 
 template <class T, int EQ, int REC, int FLUX>
@@ -60,7 +64,6 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long red[32];
-    __shared__ int is_last;
     __shared__ DtState item_dt;  // the item's step, computed once per CTA
     __shared__ T item_dtdx, item_dx;
     constexpr int HL = step_halo<T>();
@@ -82,23 +85,26 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
     const Win<const T> guin = make_win(uin, total);
     const Win<T> guout = make_win(uout, total);
 
-    __shared__ int s_item;
-    for (int item = next_item(P, 0, &s_item); item >= 0 && ok; item = next_item(P, 0, &s_item)) {
-        const int b = P.item_inst[item];
-        const int64_t off = P.offsets[b];
-        const int64_t n = P.offsets[b + 1] - off;
-        const int64_t s0 = int64_t(P.item_tile[item]) * P.tile;
-        const int te = static_cast<int>(imin64(P.tile, n - s0));
+    __shared__ int s_item[2];
+    for (ItemQueue items(P, 0, s_item); items.more(); items.end()) {
+        const PlanItem it = items.begin();
+        const int b = it.b, te = it.te;
+        const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
         // one thread evaluates the step (double divisions: a 1/64-rate pipe on
-        // this GPU) and shares it; the previous item's readers are past the
-        // barrier that ended that item
-        if (threadIdx.x == 0) {
-            const DtState d = plan_dt(P, k, b, from_bits(P.amax[size_t(cur) * P.B + b]));
-            item_dt = d;
-            item_dtdx = static_cast<T>(d.dt * P.inv_dx[b]);
-            item_dx = static_cast<T>(1.0 / P.inv_dx[b]);
+        // this GPU) while the window is in flight, and shares it; the previous
+        // item's readers are past the barrier that ended that item
+        ok = load_window<T>(sm.U, uin + off, n, s0 - HL, te + 2 * HL, &bar, phase, [&] {
+            if (threadIdx.x == 32) {
+                const DtState d = plan_dt(P, k, b, from_bits(P.amax[size_t(cur) * P.B + b]));
+                item_dt = d;
+                item_dtdx = static_cast<T>(d.dt * P.inv_dx[b]);
+                item_dx = static_cast<T>(1.0 / P.inv_dx[b]);
+            }
+        });
+        if (!ok) {
+            if (threadIdx.x == 0) atomicOr(P.status, ERR_TIMEOUT);
+            break;
         }
-        __syncthreads();
         const DtState ds = item_dt;
         B mx = 0;
         if (!(ds.active && ds.finite)) {
@@ -110,11 +116,6 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
                 mx = bb > mx ? bb : mx;
             }
         } else {
-            ok = load_window<T>(sm.U, uin + off, n, s0 - HL, te + 2 * HL, &bar, phase);
-            if (!ok) {
-                if (threadIdx.x == 0) atomicOr(P.status, ERR_TIMEOUT);
-                break;
-            }
             const T dtdx = item_dtdx;
             OpParams<T> pb = p;
             pb.dx = item_dx;
@@ -122,24 +123,17 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
                                              s0 - HL, n);
         }
         const B bm = block_max<B>(mx, reinterpret_cast<B*>(red));
-        if (threadIdx.x == 0) atomicMax(P.amax + size_t(nxt) * P.B + b, to_double_bits<T>(bm));
-        __syncthreads();
+        if (threadIdx.x == 0) {
+            atomicMax(P.amax + size_t(nxt) * P.B + b, to_double_bits<T>(bm));
+            finish_tile(P, k, b, it.tiles, ds);
+        }
     }
 
-    // completion: the last CTA of the step advances t, records dt, resets the
-    // consumed maxima and increments the step counter (no host round trip)
-    __syncthreads();
+    // the last CTA of the step increments the step counter (no host round trip)
     if (threadIdx.x == 0) {
         __threadfence();
-        const unsigned prev = atomicAdd(P.done, 1u);
-        is_last = (prev == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (is_last) {
-        __threadfence();
-        finalize_step(P, k);
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        if (atomicAdd(P.done, 1u) == gridDim.x - 1) {
+            __threadfence();
             *reinterpret_cast<volatile unsigned*>(P.done) = 0u;
             atomicExch(P.sched, 0u);  // every CTA has taken its last item
             *reinterpret_cast<volatile int64_t*>(P.step) = k + 1;
@@ -170,7 +164,6 @@ __global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ unsigned long long red[32];
-    __shared__ int is_last;
     __shared__ DtState item_dt;
     __shared__ double item_dtdx, item_amax;
     constexpr int HL = op_halo<double>();
@@ -192,20 +185,23 @@ __global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
     const unsigned long long* ain = STAGE == 1 ? P.amax + size_t(cur) * P.B : amax_in;
     unsigned long long* aout = STAGE == 3 ? P.amax + size_t(cur ^ 1) * P.B : amax_out;
     bool ok = true;
-    __shared__ int s_item;
-    for (int item = next_item(P, 6, &s_item); item >= 0 && ok; item = next_item(P, 6, &s_item)) {
-        const int b = P.item_inst[item];
-        const int64_t off = P.offsets[b];
-        const int64_t n = P.offsets[b + 1] - off;
-        const int64_t s0 = int64_t(P.item_tile[item]) * P.tile;
-        const int te = static_cast<int>(imin64(P.tile, n - s0));
-        if (threadIdx.x == 0) {
-            const DtState d = plan_dt(P, k, b, from_bits(P.amax[size_t(cur) * P.B + b]));
-            item_dt = d;
-            item_dtdx = d.dt * P.inv_dx[b];
-            item_amax = from_bits(ain[b]);
+    __shared__ int s_item[2];
+    for (ItemQueue items(P, 6, s_item); items.more(); items.end()) {
+        const PlanItem it = items.begin();
+        const int b = it.b, te = it.te;
+        const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
+        ok = load_window<double>(sm.U, kin + off, n, s0 - HL, te + 2 * HL, &bar, phase, [&] {
+            if (threadIdx.x == 32) {
+                const DtState d = plan_dt(P, k, b, from_bits(P.amax[size_t(cur) * P.B + b]));
+                item_dt = d;
+                item_dtdx = d.dt * P.inv_dx[b];
+                item_amax = from_bits(ain[b]);
+            }
+        });
+        if (!ok) {
+            if (threadIdx.x == 0) atomicOr(P.status, ERR_TIMEOUT);
+            break;
         }
-        __syncthreads();
         const DtState ds = item_dt;
         unsigned long long mx = 0;
         if (!(ds.active && ds.finite)) {
@@ -217,11 +213,6 @@ __global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
                 mx = bb > mx ? bb : mx;
             }
         } else {
-            ok = load_window<double>(sm.U, kin + off, n, s0 - HL, te + 2 * HL, &bar, phase);
-            if (!ok) {
-                if (threadIdx.x == 0) atomicOr(P.status, ERR_TIMEOUT);
-                break;
-            }
             OpParams<double> pb = p;
             pb.hnu_amax = p.hnu * item_amax;
             face_fluxes<double, EQ, SHK_REC_WENOJS53, SHK_FLUX_LF>(sm.U, HL, HL + te, sm, pb);
@@ -239,33 +230,26 @@ __global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
             }
         }
         const unsigned long long bm = block_max<unsigned long long>(mx, red);
-        if (threadIdx.x == 0) atomicMax(aout + b, bm);
-        __syncthreads();
+        if (threadIdx.x == 0) {
+            atomicMax(aout + b, bm);
+            if constexpr (STAGE == 3) {
+                // the instance's stage maxima are consumed too
+                if (finish_tile(P, k, b, it.tiles, ds)) amax_clear[b] = amax_clear[P.B + b] = 0ull;
+            }
+        }
     }
     if constexpr (STAGE < 3) {
         finish_items(P, 6);
-    } else {
-        // the last CTA of the step: time, dt history, step counter, and the
-        // stage maxima cleared for the next step
-        __syncthreads();
-        if (threadIdx.x == 0) {
+    } else if (threadIdx.x == 0) {
+        // the last CTA of the step increments the step counter
+        __threadfence();
+        if (atomicAdd(P.done, 1u) == gridDim.x - 1) {
             __threadfence();
-            const unsigned prev = atomicAdd(P.done, 1u);
-            is_last = (prev == gridDim.x - 1);
-        }
-        __syncthreads();
-        if (is_last) {
+            *reinterpret_cast<volatile unsigned*>(P.done) = 0u;
+            atomicExch(P.sched + 6, 0u);
+            atomicExch(P.sched + 7, 0u);
+            *reinterpret_cast<volatile int64_t*>(P.step) = k + 1;
             __threadfence();
-            finalize_step(P, k);
-            for (int i = threadIdx.x; i < 2 * P.B; i += blockDim.x) amax_clear[i] = 0ull;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                *reinterpret_cast<volatile unsigned*>(P.done) = 0u;
-                atomicExch(P.sched + 6, 0u);
-                atomicExch(P.sched + 7, 0u);
-                *reinterpret_cast<volatile int64_t*>(P.step) = k + 1;
-                __threadfence();
-            }
         }
     }
 }
@@ -771,7 +755,8 @@ struct shk_plan {
     double* bc_neu = nullptr;  // [B][2], or per-step [bc_steps][3][B][2]
     int64_t bc_steps = 0;      // 0: time-independent boundary data
     size_t bc_dir_cap = 0, bc_neu_cap = 0;  // doubles allocated
-    int32_t* item_order = nullptr;  // [nitems] longest first
+    PlanItem* items = nullptr;  // [nitems] longest first
+    unsigned int* left = nullptr;  // [B] finished tiles of the running step
     unsigned int* sched = nullptr;  // [8] scheduling counters
     // host mirror of the number of steps launched since reset
     int64_t host_steps = 0;
@@ -792,7 +777,7 @@ struct shk_plan {
         P.partial = partial; P.B = B;
         P.dt_fixed = fixed_steps > 0 ? dt_fixed : nullptr; P.fixed_steps = fixed_steps;
         P.bc_left = bc_left; P.bc_right = bc_right; P.bc_dir = bc_dir; P.bc_neu = bc_neu; P.nitems = nitems; P.tile = tile; P.max_steps = max_steps;
-        P.item_order = item_order; P.sched = sched; P.bc_steps = bc_steps;
+        P.items = items; P.left = left; P.sched = sched; P.bc_steps = bc_steps;
         return P;
     }
 };
@@ -959,7 +944,7 @@ int shk_plan_destroy(shk_plan* plan) {
     void* ptrs[] = {plan->item_inst, plan->item_tile, plan->item_first, plan->offsets, plan->cfl,
                     plan->inv_dx, plan->tfinal, plan->amax, plan->t, plan->dt_hist, plan->step,
                     plan->done, plan->status, plan->partial, plan->dt_fixed, plan->bc_dir,
-                    plan->bc_neu, plan->item_order, plan->sched, plan->lf_k1, plan->lf_k2,
+                    plan->bc_neu, plan->items, plan->left, plan->sched, plan->lf_k1, plan->lf_k2,
                     plan->amax_lf};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -1005,6 +990,12 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
         len[i] = std::min<int64_t>(tile, n - int64_t(tl[i]) * tile);
     }
     std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return len[x] > len[y]; });
+    std::vector<PlanItem> items(inst.size());
+    for (size_t q = 0; q < order.size(); ++q) {
+        const int32_t i = order[q], b = inst[i];
+        items[q] = PlanItem{h_offsets[b], h_offsets[b + 1] - h_offsets[b], b, static_cast<int32_t>(len[i]),
+                            tl[i], first[b + 1] - first[b]};
+    }
     auto* P = new (std::nothrow) shk_plan();
     if (!P) return SHK_ENOMEM;
     P->scheme = *scheme;
@@ -1030,7 +1021,8 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
               alloc((void**)&P->step, sizeof(int64_t)) && alloc((void**)&P->done, sizeof(unsigned)) &&
               alloc((void**)&P->status, sizeof(int32_t)) &&
               alloc((void**)&P->partial, sizeof(double) * P->nitems) &&
-              alloc((void**)&P->item_order, sizeof(int32_t) * P->nitems) &&
+              alloc((void**)&P->items, sizeof(PlanItem) * P->nitems) &&
+              alloc((void**)&P->left, sizeof(unsigned) * batch) &&
               alloc((void**)&P->sched, sizeof(unsigned) * 8);
     if (ok && P->max_steps > 0)
         ok = alloc((void**)&P->dt_hist, sizeof(double) * size_t(P->max_steps) * batch);
@@ -1045,7 +1037,8 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
     }
     ok = cudaMemcpy(P->item_inst, inst.data(), sizeof(int32_t) * P->nitems, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(P->item_tile, tl.data(), sizeof(int32_t) * P->nitems, cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(P->item_order, order.data(), sizeof(int32_t) * P->nitems, cudaMemcpyHostToDevice) == cudaSuccess &&
+         cudaMemcpy(P->items, items.data(), sizeof(PlanItem) * P->nitems, cudaMemcpyHostToDevice) == cudaSuccess &&
+         cudaMemset(P->left, 0, sizeof(unsigned) * batch) == cudaSuccess &&
          cudaMemset(P->sched, 0, sizeof(unsigned) * 8) == cudaSuccess &&
          cudaMemcpy(P->item_first, first.data(), sizeof(int32_t) * (batch + 1), cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(P->offsets, h_offsets, sizeof(int64_t) * (batch + 1), cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -1128,6 +1121,7 @@ int shk_plan_reset(shk_plan* plan, const void* u, const double* t0, const double
     SHK_CUDA(cudaMemsetAsync(plan->step, 0, sizeof(int64_t), st));
     SHK_CUDA(cudaMemsetAsync(plan->done, 0, sizeof(unsigned), st));
     SHK_CUDA(cudaMemsetAsync(plan->sched, 0, sizeof(unsigned) * 8, st));
+    SHK_CUDA(cudaMemsetAsync(plan->left, 0, sizeof(unsigned) * B, st));
     SHK_CUDA(cudaMemsetAsync(plan->status, 0, sizeof(int32_t), st));
     if (t0) SHK_CUDA(cudaMemcpyAsync(plan->t, t0, sizeof(double) * B, cudaMemcpyDeviceToDevice, st));
     else SHK_CUDA(cudaMemsetAsync(plan->t, 0, sizeof(double) * B, st));

@@ -435,9 +435,13 @@ __device__ __forceinline__ void face_fluxes(PV v, int lo, int hi, const Smem<T>&
 // when every piece is 16-byte aligned, plain coalesced loads otherwise.
 // Returns false if the bulk copy did not complete within the wait limit.
 // ---------------------------------------------------------------------------
-template <class T>
+// meanwhile() runs on every thread while the copies are in flight.
+struct Nothing {
+    __device__ void operator()() const {}
+};
+template <class T, class F = Nothing>
 __device__ bool load_window(Win<T> dst, const T* base, int64_t n, int64_t g0, int W,
-                            uint64_t* bar, uint32_t& phase) {
+                            uint64_t* bar, uint32_t& phase, F&& meanwhile = F()) {
     const size_t sz = sizeof(T);
     // a window no longer than its instance wraps at most once: one compare
     // instead of a 64-bit remainder per position
@@ -471,6 +475,7 @@ __device__ bool load_window(Win<T> dst, const T* base, int64_t n, int64_t g0, in
             const int64_t src = wrap(g0 + w);
             if (chk_index(src, n)) dst[w] = base[src];
         }
+        meanwhile();
         __syncthreads();
         return true;
     }
@@ -488,6 +493,7 @@ __device__ bool load_window(Win<T> dst, const T* base, int64_t n, int64_t g0, in
             pos += len;
         }
     }
+    meanwhile();
     bool ok = mbar_wait_bounded(bar, phase);
     if (!ok) ok = mbar_wait_bounded(bar, phase);  // second bounded wait for copies in flight
     phase ^= 1u;
@@ -1029,6 +1035,13 @@ __device__ typename Bits<T>::type step_tile(const Smem<T>& sm, Win<T> gout, int 
     }
 }
 
+// one work item: tile `tile` of the `tiles` of instance b (te cells of it), whose n
+// cells start at off
+struct __align__(16) PlanItem {
+    int64_t off, n;
+    int32_t b, te, tile, tiles;
+};
+
 // device view of a batched plan (see shk_plan in forward.cu)
 struct PlanDev {
     const int32_t* item_inst;
@@ -1051,23 +1064,40 @@ struct PlanDev {
     const double* bc_dir;    // [B][2][3] Dirichlet ghost values, or [bc_steps][3][B][2][3]
     const double* bc_neu;    // [B][2] Neumann gradients, or [bc_steps][3][B][2]
     int64_t bc_steps;        // 0: time-independent data; else per-step, per-stage tables
-    const int32_t* item_order;  // [nitems] items longest first (dynamic scheduling)
+    const PlanItem* items;      // [nitems] longest first (dynamic scheduling)
+    unsigned int* left;         // [B] tiles of the running step that are done
     unsigned int* sched;        // [8] item counters of the scheduled kernels
     int32_t B, nitems, tile, max_steps;
 };
 
-// Dynamic item scheduling. A CTA takes the next item of the plan's
-// longest-first order from the counter sched[slot]; uneven items (partial
-// tiles, copied-through instances) then balance over the persistent grid,
-// where a fixed stride would hand some CTAs only long items. Returns the item,
-// or -1 when none is left. Every caller's loop body ends with a barrier, which
-// orders the read of *s_item before thread 0 overwrites it.
-__device__ __forceinline__ int next_item(const PlanDev& P, int slot, int* s_item) {
-    if (threadIdx.x == 0) *s_item = static_cast<int>(atomicAdd(P.sched + slot, 1u));
-    __syncthreads();
-    const int q = *s_item;
-    return q < P.nitems ? P.item_order[q] : -1;
-}
+// Dynamic item scheduling. A CTA takes the items of the plan's longest-first
+// list from the counter sched[slot]; uneven items (partial tiles, copied-through
+// instances) then balance over the persistent grid, where a fixed stride would
+// hand some CTAs only long items. The first item is the CTA's own index; the next
+// one is requested when an item begins, so the counter's latency is behind it.
+// s: two words of shared memory (a thread may still read one when the next is
+// written).
+struct ItemQueue {
+    const PlanDev& P;
+    int slot;
+    int* s;
+    int q, par = 0;
+    unsigned next = 0;
+    __device__ __forceinline__ ItemQueue(const PlanDev& P_, int slot_, int* s_)
+        : P(P_), slot(slot_), s(s_), q(static_cast<int>(blockIdx.x)) {}
+    __device__ __forceinline__ bool more() const { return q < P.nitems; }
+    __device__ __forceinline__ PlanItem begin() {
+        if (threadIdx.x == 0) next = atomicAdd(P.sched + slot, 1u) + gridDim.x;
+        return P.items[q];
+    }
+    // a barrier
+    __device__ __forceinline__ void end() {
+        if (threadIdx.x == 0) s[par] = static_cast<int>(next);
+        __syncthreads();
+        q = s[par];
+        par ^= 1;
+    }
+};
 
 // end of a scheduled launch: the CTA that finishes last (counter
 // sched[slot + 1]) resets both counters for the next launch
