@@ -1,5 +1,5 @@
 // Face fluxes of a double state without the FP64 pipe (Burgers, WENO-JS5,
-// Rusanov with nu = 1).
+// Rusanov or global Lax-Friedrichs with nu = 1).
 //
 // GB300's FP64 pipe takes 16 clocks per warp instruction and SM, 64 times an
 // FP32 or integer instruction's share, so the flux is formed from 64-bit
@@ -8,7 +8,8 @@
 // on the middle sub-stencil's value plus weighted third differences give
 //   Z = 6 (R + L) = 6 (v_j + v_{j+1}) - (E_j + E_{j+1}) + pR_j + pL_{j+1}
 //   D = 6 (R - L) = T_j + pR_j - pL_{j+1}
-//   288 F = Z^2 + D (D + 24 a),  a = max(|v_j|, |v_{j+1}|)
+//   288 F = Z^2 + D (D + 24 a),  a = max(|v_j|, |v_{j+1}|) (Lax-Friedrichs: the
+//                                instance's maximum)
 //   pR = -(2 r0 T_{c-1} + 3 r2 T_c) / (r0 + 6 + 3 r2)
 //   pL =  (2 r2 T_c + 3 r0 T_{c-1}) / (r2 + 6 + 3 r0)
 // with r0 = (e1/e0)^2, r2 = (e1/e2)^2, e_k = 4 (eps + beta_k). Only pR and pL
@@ -213,6 +214,7 @@ struct Cell {
     int64_t T;    // E_{c+1} - E_c
     int64_t S, E; // v_{c+1} - v_{c-1}, E_c
     uint64_t A;   // max(|v_c|, |v_{c+1}|)
+    uint32_t exm;
     float u0;     // 2^(exm - 1079)
     float iu;     // 1 / u0
     int kz, k;    // binary exponents of the units and of the flux units
@@ -226,6 +228,7 @@ SHK_FX Cell cell_begin(const Mag& vm, const Mag& v0, const Mag& v1, const Mag& v
     // scales 2^-60 .. 2^60; a zero state takes the smallest
     c.in = exm - (1023u - 60u) <= 120u || exm == 0u;
     exm = exm == 0u || !c.in ? 1023u - 60u : exm;
+    c.exm = exm;
     c.u0 = bitsf((exm - 952u) << 23);
     c.iu = bitsf((1206u - exm) << 23);
     c.kz = static_cast<int>(exm) - 1079;
@@ -354,30 +357,56 @@ SHK_FX double to_double(int64_t X, int k) {
     return lo != 0u ? pack_double(lo, 0u, e - 32, s) : 0.0;
 }
 
-// 288 F = Z^2 + D Q, in units of 2^k: the upper 64 of 128 bits of each product
-// (0 <= Q < 2^63)
-SHK_FX double face_flux(int k, int64_t Z, int64_t D, int64_t Q) {
-    const int32_t zh = static_cast<int32_t>(Z >> 32), dh = static_cast<int32_t>(D >> 32);
-    const int32_t zl = static_cast<int32_t>(static_cast<uint32_t>(Z) >> 1);
+// the upper 64 of 128 bits of Z^2 and of D Q, 0 <= Q < 2^63
+SHK_FX int64_t square_hi(int64_t Z) {
+    const int32_t zh = static_cast<int32_t>(Z >> 32), zl = static_cast<int32_t>(static_cast<uint32_t>(Z) >> 1);
+    return int64_t(zh) * zh + ((int64_t(zh) * zl) >> 30);
+}
+SHK_FX int64_t product_hi(int64_t D, int64_t Q) {
+    const int32_t dh = static_cast<int32_t>(D >> 32);
     const int32_t qh = static_cast<int32_t>(Q >> 32), ql = static_cast<int32_t>(static_cast<uint32_t>(Q) >> 1);
-    const int64_t zz = int64_t(zh) * zh + ((int64_t(zh) * zl) >> 30);
-    const int64_t dq = int64_t(dh) * qh + ((int64_t(dh) * ql) >> 31) + umulhi(static_cast<uint32_t>(D), static_cast<uint32_t>(qh));
-    return to_double(zz + dq, k);
+    return int64_t(dh) * qh + ((int64_t(dh) * ql) >> 31) + umulhi(static_cast<uint32_t>(D), static_cast<uint32_t>(qh));
+}
+// 288 F = Z^2 + D Q with Q = D + 24 a, in units of 2^k
+SHK_FX double face_flux(int k, int64_t Z, int64_t D, int64_t Q) {
+    return to_double(square_hi(Z) + product_hi(D, Q), k);
 }
 
-// 288 F from face values R, L formed in double (v0, v1: the face's cells), with
-// the integer arithmetic of the other faces: next to a constant state, where R
-// = L = v, the flux equals theirs and the difference vanishes exactly. False
-// where the integers do not hold it.
-SHK_FX bool listed_flux(double R, double L, double v0, double v1, double& G) {
-    const Mag r = mag(R), l = mag(L), a = mag(v0), b = mag(v1);
+// the Lax-Friedrichs speed: 24 a = M units of 2^(e - 1079), M < 2^62
+struct Speed {
+    int64_t M;
+    uint32_t e;
+    bool in;  // the scale is in range
+};
+SHK_FX Speed speed_begin(double a) {
+    const Mag m = mag(a);
+    return Speed{static_cast<int64_t>(24u * fix_abs(m, m.e)), m.e, m.e <= 1023u + 60u};
+}
+// 288 F = Z^2 + D^2 + 24 a D with the speed's own scale (at least the cell's):
+// in units 2^(k + sh), sh the distance of the two scales. dt / dx times the
+// speed is at most 1/2, so a resolution of 2^-57 of (speed x local value) in F
+// is one of 2^-57 of the local value in the state.
+SHK_FX double face_flux_lf(const Cell& c, int64_t Z, int64_t D, const Speed& sp) {
+    const uint32_t d = sp.e > c.exm ? sp.e - c.exm : 0u, sh = d < 63u ? d : 63u;
+    return to_double(((square_hi(Z) + square_hi(D)) >> sh) + product_hi(D, sp.M), c.k + static_cast<int>(d));
+}
+
+// 288 F from face values R, L formed in double (v0, v1: the face's cells, a: the
+// speed if it is the larger), with the integer arithmetic of the other faces:
+// next to a constant state, where R = L = v, the flux equals theirs and the
+// difference vanishes exactly. False where the integers do not hold it.
+SHK_FX bool listed_flux(double R, double L, double v0, double v1, double aglob, double& G) {
+    const Mag r = mag(R), l = mag(L), a = mag(v0), b = mag(v1), g = mag(aglob);
     uint32_t exm = r.e > l.e ? r.e : l.e;
     exm = exm > a.e ? exm : a.e;
     exm = exm > b.e ? exm : b.e;
+    exm = exm > g.e ? exm : g.e;
     if (exm == 0u) exm = 1023u - 60u;
     if (exm - (1023u - 60u) > 120u) return false;
     const int64_t x = with_sign(fix_abs(r, exm), r), y = with_sign(fix_abs(l, exm), l);
-    const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm), A = A0 > A1 ? A0 : A1;
+    const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm), A2 = fix_abs(g, exm);
+    uint64_t A = A0 > A1 ? A0 : A1;
+    A = A > A2 ? A : A2;
     const int64_t D = 6 * (x - y), Q = D + static_cast<int64_t>(24u * A);
     if (Q < 0) return false;
     G = face_flux(2 * static_cast<int>(exm) - 2094, 6 * (x + y), D, Q);

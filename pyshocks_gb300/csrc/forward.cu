@@ -156,8 +156,9 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
 // batched_step_kernel does and clears the stage maxima. float64 states,
 // periodic instances, the reference's stage formulas:
 //   k1 = u + dt L(u),  k2 = 3/4 u + 1/4 (k1 + dt L(k1)),  u+ = 1/3 u + 2/3 (k2 + dt L(k2)).
-template <int EQ, int STAGE>
-__global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
+// FX: the fluxes of fixed_flux.cuh.
+template <int EQ, int STAGE, bool FX>
+__global__ void __launch_bounds__(FX ? kFxThreads : kThreads, FX ? 8 : 1) batched_lf_stage_kernel(
     PlanDev P, const double* __restrict__ u, const double* __restrict__ kin, double* __restrict__ kout,
     const unsigned long long* __restrict__ amax_in, unsigned long long* amax_out,
     unsigned long long* amax_clear, OpParams<double> p) {
@@ -168,7 +169,8 @@ __global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
     __shared__ double item_dtdx, item_amax;
     constexpr int HL = op_halo<double>();
     Smem<double> sm;
-    sm.carve(smem_raw, P.tile + 2 * HL);
+    if constexpr (FX) sm.carve_lf_stage(smem_raw, P.tile + 2 * HL);
+    else sm.carve(smem_raw, P.tile + 2 * HL);
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_mbar_init();
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
     const unsigned long long* ain = STAGE == 1 ? P.amax + size_t(cur) * P.B : amax_in;
     unsigned long long* aout = STAGE == 3 ? P.amax + size_t(cur ^ 1) * P.B : amax_out;
     bool ok = true;
+    [[maybe_unused]] int slot = 0;
     __shared__ int s_item[2];
     for (ItemQueue items(P, 6, s_item); items.more(); items.end()) {
         const PlanItem it = items.begin();
@@ -213,10 +216,18 @@ __global__ void __launch_bounds__(kThreads) batched_lf_stage_kernel(
                 mx = bb > mx ? bb : mx;
             }
         } else {
-            OpParams<double> pb = p;
-            pb.hnu_amax = p.hnu * item_amax;
-            face_fluxes<double, EQ, SHK_REC_WENOJS53, SHK_FLUX_LF>(sm.U, HL, HL + te, sm, pb);
-            const double dtdx = item_dtdx;
+            double dtdx = item_dtdx;
+            if constexpr (FX) {
+                // (the list's counters 0 and 1 alternate)
+                fx_fluxes<true>(sm.U, HL - 1, HL + te, sm, p, slot,
+                                StoreFaces<Win<double>>{Win<double>(), Win<double>(), 0, 0, 0}, item_amax);
+                slot ^= 1;
+                dtdx *= 1.0 / 288.0;
+            } else {
+                OpParams<double> pb = p;
+                pb.hnu_amax = p.hnu * item_amax;
+                face_fluxes<double, EQ, SHK_REC_WENOJS53, SHK_FLUX_LF>(sm.U, HL, HL + te, sm, pb);
+            }
             for (int i = threadIdx.x; i < te; i += blockDim.x) {
                 const int w = HL + i;
                 const double kk = fma(dtdx, sm.D[w - 1] - sm.D[w], sm.U[w]);  // k + dt L(k)
@@ -498,6 +509,7 @@ int default_tile(const shk_scheme* s, int dtype, int max_steps) {
         if (dtype == SHK_F32) return max_steps > 0 ? 1024 : 2048;
         return max_steps > 0 ? 512 : (fixed_flux_scheme(s) ? 946 : kDefaultTile);
     }
+    if (dtype == SHK_F64 && fixed_flux_scheme(s, SHK_FLUX_LF)) return 946;
     return kDefaultTile;
 }
 
@@ -686,18 +698,19 @@ struct BatchedStepLaunch {
 struct BatchedLfLaunch {
     PlanDev D; const double* uin; double* uout; double* k1; double* k2; unsigned long long* amax_lf;
     OpParams<double> p; size_t smem; int grid; cudaStream_t st;
-    template <int EQ> int run() {
-        auto s1 = batched_lf_stage_kernel<EQ, 1>;
-        auto s2 = batched_lf_stage_kernel<EQ, 2>;
-        auto s3 = batched_lf_stage_kernel<EQ, 3>;
+    template <int EQ, bool FX = false> int run() {
+        constexpr int kThr = FX ? kFxThreads : kThreads;
+        auto s1 = batched_lf_stage_kernel<EQ, 1, FX>;
+        auto s2 = batched_lf_stage_kernel<EQ, 2, FX>;
+        auto s3 = batched_lf_stage_kernel<EQ, 3, FX>;
         for (auto k : {s1, s2, s3})
             SHK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const int B = D.B;
-        s1<<<grid, kThreads, smem, st>>>(D, uin, uin, k1, nullptr, amax_lf, amax_lf, p);
+        s1<<<grid, kThr, smem, st>>>(D, uin, uin, k1, nullptr, amax_lf, amax_lf, p);
         SHK_CUDA(cudaGetLastError());
-        s2<<<grid, kThreads, smem, st>>>(D, uin, k1, k2, amax_lf, amax_lf + B, amax_lf, p);
+        s2<<<grid, kThr, smem, st>>>(D, uin, k1, k2, amax_lf, amax_lf + B, amax_lf, p);
         SHK_CUDA(cudaGetLastError());
-        s3<<<grid, kThreads, smem, st>>>(D, uin, k2, uout, amax_lf + B, nullptr, amax_lf, p);
+        s3<<<grid, kThr, smem, st>>>(D, uin, k2, uout, amax_lf + B, nullptr, amax_lf, p);
         return cuda_check(cudaGetLastError());
     }
 };
@@ -705,15 +718,17 @@ struct BatchedLfLaunch {
 // resident CTAs per SM of the step kernel a scheme dispatches to, at the
 // given dynamic shared memory (registers and shared memory both counted)
 struct StepOccupancy {
-    size_t smem; int* out;
+    size_t smem; int* out; bool fixed;  // fixed: a Lax-Friedrichs plan on fixed_flux.cuh
     template <class T, int EQ, int REC, int FLUX> int operator()() {
         if constexpr (FLUX == SHK_FLUX_LF) {
             if constexpr (sizeof(T) != 8) {
                 return SHK_EUNSUPPORTED;
             } else {
-                auto k = batched_lf_stage_kernel<EQ, 2>;
+                auto k = batched_lf_stage_kernel<EQ, 2, false>;
+                if constexpr (EQ == SHK_EQ_BURGERS)
+                    if (fixed) k = batched_lf_stage_kernel<EQ, 2, true>;
                 SHK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                SHK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, kThreads, smem));
+                SHK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, k, fixed ? kFxThreads : kThreads, smem));
                 return SHK_OK;
             }
         } else {
@@ -803,11 +818,12 @@ int launch_step(shk_plan* P, const void* uin, void* uout, cudaStream_t st) {
         if constexpr (sizeof(T) != 8) {
             return SHK_EUNSUPPORTED;
         } else {
-            const size_t smem = Smem<double>::host_bytes(P->tile + 2 * op_halo<double>());
+            const bool fixed = fixed_flux_scheme(&P->scheme, SHK_FLUX_LF);
+            const size_t smem = Smem<double>::lf_stage_bytes(P->tile + 2 * op_halo<double>(), fixed);
             BatchedLfLaunch f{D, static_cast<const double*>(uin), static_cast<double*>(uout), P->lf_k1,
                               P->lf_k2, P->amax_lf, make_params<double>(&P->scheme), smem, P->grid, st};
             switch (P->scheme.equation) {
-                case SHK_EQ_BURGERS: return f.run<SHK_EQ_BURGERS>();
+                case SHK_EQ_BURGERS: return fixed ? f.run<SHK_EQ_BURGERS, true>() : f.run<SHK_EQ_BURGERS>();
                 case SHK_EQ_ADVECTION: return f.run<SHK_EQ_ADVECTION>();
                 default: return f.run<SHK_EQ_LWR>();
             }
@@ -1057,12 +1073,13 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
     // persistent grid: resident CTAs per SM x SMs
     int per_sm = opts && opts->ctas_per_sm > 0 ? opts->ctas_per_sm : 0;
     if (per_sm == 0) {
-        const size_t smem = lf ? Smem<double>::host_bytes(tile + 2 * op_halo<double>())
+        const bool fixed_lf = fixed_flux_scheme(scheme, SHK_FLUX_LF);
+        const size_t smem = lf ? Smem<double>::lf_stage_bytes(tile + 2 * op_halo<double>(), fixed_lf)
                                : (dtype == SHK_F64 ? Smem<double>::step_bytes(tile + 2 * step_halo<double>(), scheme->rec, fixed_flux_scheme(scheme))
                                                    : Smem<float>::step_bytes(tile + 2 * step_halo<float>(), scheme->rec));
         int resident = 0;
-        const int r = dtype == SHK_F64 ? dispatch_scheme<double>(scheme, StepOccupancy{smem, &resident})
-                                       : dispatch_scheme<float>(scheme, StepOccupancy{smem, &resident});
+        const int r = dtype == SHK_F64 ? dispatch_scheme<double>(scheme, StepOccupancy{smem, &resident, fixed_lf})
+                                       : dispatch_scheme<float>(scheme, StepOccupancy{smem, &resident, fixed_lf});
         if (r != SHK_OK || resident < 1) {
             shk_plan_destroy(P);
             return r != SHK_OK ? r : SHK_EINVAL;  // the window does not fit one SM

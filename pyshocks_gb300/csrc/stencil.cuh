@@ -39,9 +39,8 @@ constexpr int kFluxRusanovFx = 100;
 constexpr int kFxThreads = 128;
 template <int FLUX>
 __host__ __device__ constexpr int flux_threads() { return FLUX == kFluxRusanovFx ? kFxThreads : kThreads; }
-inline bool fixed_flux_scheme(const shk_scheme* s) {
-    return s->flux == SHK_FLUX_RUSANOV && s->rec == SHK_REC_WENOJS53 &&
-           s->equation == SHK_EQ_BURGERS && s->nu == 1.0;
+inline bool fixed_flux_scheme(const shk_scheme* s, int flux = SHK_FLUX_RUSANOV) {
+    return s->flux == flux && s->rec == SHK_REC_WENOJS53 && s->equation == SHK_EQ_BURGERS && s->nu == 1.0;
 }
 
 // halo of a window: 9 cells are needed for three fused stages, rounded up so
@@ -109,6 +108,19 @@ struct Smem {
         H = Q = Win<T>();
         scr = Win<float>();
         this->W = W;
+    }
+    // (one Lax-Friedrichs stage: U, D and the list)
+    __host__ static size_t lf_stage_bytes(int W, bool fixed) {
+        return fixed ? size_t(2) * W * sizeof(T) + size_t(W + kFxCounters) * sizeof(int) : host_bytes(W);
+    }
+    __device__ void carve_lf_stage(unsigned char* base, int W) {
+        T* p = reinterpret_cast<T*>(base);
+        U = make_win(p, W); D = make_win(p + W, W);
+        fx = make_win(reinterpret_cast<int*>(p + 2 * W), W + kFxCounters);
+        S = H = Q = UL = UR = I = Win<T>();
+        scr = Win<float>();
+        this->W = W;
+        if (threadIdx.x < kFxCounters) fx[threadIdx.x] = 0;  // (the caller's barrier follows)
     }
     __device__ void carve_fixed(unsigned char* base, int W) {
         T* p = reinterpret_cast<T*>(base);
@@ -763,7 +775,7 @@ __device__ __forceinline__ double weno53_side_d(double vm2, double vm1, double v
 // what the listed faces need; two lanes per face, one for each side's value
 template <class PV, class FaceOut>
 __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list, int cnt, double eps,
-                                             FaceOut out) {
+                                             double aglob, FaceOut out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const double eps4 = 4.0 * eps;
     for (int q0 = 16 * warp; q0 < cnt; q0 += 16 * nw) {
@@ -775,8 +787,9 @@ __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list,
         const double R = (lane & 1) ? w1 : w, L = (lane & 1) ? w : w1;
         if (q < cnt && (lane & 1) == 0) {
             double g;
-            if (!fx::listed_flux(R, L, v[j], v[j + 1], g)) {
-                const auto ab = abs_bits(v[j]) > abs_bits(v[j + 1]) ? abs_bits(v[j]) : abs_bits(v[j + 1]);
+            if (!fx::listed_flux(R, L, v[j], v[j + 1], aglob, g)) {
+                auto ab = abs_bits(v[j]) > abs_bits(v[j + 1]) ? abs_bits(v[j]) : abs_bits(v[j + 1]);
+                ab = ab > abs_bits(aglob) ? ab : abs_bits(aglob);
                 g = 72.0 * fma(L, L, fma(R, R, twice_abs_bits(ab) * (R - L)));
             }
             G[j] = g;
@@ -802,14 +815,18 @@ struct StoreFaces {
 // 1..30, neighbours' terms by shuffle. Faces that fixed_flux.cuh leaves go to
 // the list of counter `slot` and are evaluated after a barrier. Ends with a
 // barrier. The counter of the next stage is cleared on the way: its last
-// readers are past this stage's first barrier.
-template <class PV, class FaceOut>
+// readers are past this stage's first barrier. LF: the global Lax-Friedrichs
+// flux with the speed aglob (at least every |v|).
+template <bool LF = false, class PV, class FaceOut>
 __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<double>& sm,
-                                          const OpParams<double>& p, int slot, const FaceOut& out) {
+                                          const OpParams<double>& p, int slot, const FaceOut& out,
+                                          double aglob = 0.0) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const Win<int> list = sm.fx + kFxCounters;
     const fx::FF eps4{fx::dup(p.e4h), fx::dup(p.e4l)};
+    fx::Speed speed{0, 0u, true};
+    if constexpr (LF) speed = fx::speed_begin(aglob);
     for (int r0 = (jlo & ~1) - 2 + 60 * warp; r0 + 2 < jhi; r0 += 60 * nw) {
         const int c0 = r0 + 2 * lane;
         // (positions outside the window only feed faces that are not stored)
@@ -834,13 +851,14 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
         auto face = [&](int j, const fx::Cell& c, bool mine, float xR, float xL, float tR, float tL, float rs,
                         float rd) -> double {
             int64_t Z, D, Q;
-            const bool ok = fx::face_sums(c, xR, xL, tR, tL, rs, rd, Z, D, Q);
+            const bool ok = fx::face_sums(c, xR, xL, tR, tL, rs, rd, Z, D, Q) && speed.in;
             if (mine) {
                 if (!ok) list[atomicAdd(&sm.fx[slot], 1)] = j;
                 else if (out.ul)
                     out(j, fx::to_double(Z + D, c.kz) * (1.0 / 12.0), fx::to_double(Z - D, c.kz) * (1.0 / 12.0));
             }
-            return fx::face_flux(c.k, Z, D, Q);
+            if constexpr (LF) return fx::face_flux_lf(c, Z, D, speed);
+            else return fx::face_flux(c.k, Z, D, Q);
         };
         const double f0 = face(c0, s.x, m0, fx::p2x(u.xR), fx::p2x(u.xL), fx::p2x(u.tR), fx::p2x(u.tL),
                                fx::p2x(u.rs), fx::p2x(u.rd));
@@ -857,7 +875,7 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
         if (slot == 1) sm.fx[0] = 0;  // (a step may end before its third stage)
     }
     if (cnt > 0) {
-        fx_listed_faces(v, sm.D, list, cnt, p.eps, out);
+        fx_listed_faces(v, sm.D, list, cnt, p.eps, aglob, out);
         __syncthreads();
     }
 }

@@ -37,10 +37,11 @@ def _state(kind, n, rng):
     return np.exp(-27.0 * np.abs(2.0 * x - 1.0)) * np.where(x > 0.5, 1.0, -1.0)
 
 
+@pytest.mark.parametrize("flux", ["rusanov", "lf"])
 @pytest.mark.parametrize(("kind", "amp"), [("smooth", 1.0), ("noise", 1.0), ("front", 1.0),
                                            ("plateaus", 1.0), ("range", 1.0), ("smooth", 1e-22),
                                            ("front", 1e-17), ("smooth", 1e17), ("front", 1e19)])
-def test_steps_match_oracle(kind, amp):
+def test_steps_match_oracle(kind, amp, flux):
     import pyshocks_gb300 as gb
     from pyshocks_gb300 import burgers
     from pyshocks_gb300.batched import BatchedSolver
@@ -53,11 +54,11 @@ def test_steps_match_oracle(kind, amp):
         u = amp * _state(kind, n, rng)
         ug = np.zeros(n + 6)
         ug[3:-3] = u
-        ref, _ = R.evolve(R.SchemeSpec(), og, ug, theta=0.9, maxit=nsteps)
+        ref, _ = R.evolve(R.SchemeSpec(flux_kind=flux), og, ug, theta=0.9, maxit=nsteps)
         u0.append(u)
         refs.append(ref[3:-3])
     rec = gb.reconstruction.make_reconstruction_from_name("wenojs53", eps=1.0e-6)
-    solver = BatchedSolver(burgers.Rusanov(rec=rec), SIZES, [2.0 * amp / n for n in SIZES], theta=0.9)
+    solver = BatchedSolver(burgers.make_scheme_from_name(flux, rec=rec), SIZES, [2.0 * amp / n for n in SIZES], theta=0.9)
     solver.reset(torch.tensor(np.concatenate(u0)))
     solver.step(nsteps)
     assert solver.status() == 0
