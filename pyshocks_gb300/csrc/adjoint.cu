@@ -828,14 +828,12 @@ int shk_plan_forward_checkpointed(shk_plan* plan, void* u_a, void* u_b, int32_t 
     if (!D.dt_hist || D.max_steps < nsteps || hsteps != 0) return SHK_EINVAL;
     const size_t bytes = size_t(total) * (dtype == SHK_F64 ? 8 : 4);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    for (int k = 0; k < nsteps; ++k) {
-        if (k % stride == 0) {
-            // the state before step k is in u_a for even k, u_b for odd k
-            const void* cur = (k % 2 == 0) ? u_a : u_b;
-            ADJ_CUDA(cudaMemcpyAsync(static_cast<char*>(ckpt) + size_t(k / stride) * bytes, cur,
-                                     bytes, cudaMemcpyDeviceToDevice, st));
-        }
-        r = shk_plan_step(plan, u_a, u_b, 1, stream);
+    for (int k = 0; k < nsteps; k += stride) {
+        // the state before step k is in u_a for even k, u_b for odd k
+        const void* cur = (k % 2 == 0) ? u_a : u_b;
+        ADJ_CUDA(cudaMemcpyAsync(static_cast<char*>(ckpt) + size_t(k / stride) * bytes, cur,
+                                 bytes, cudaMemcpyDeviceToDevice, st));
+        r = shk_plan_step(plan, u_a, u_b, std::min(stride, nsteps - k), stream);
         if (r != SHK_OK) return r;
     }
     return SHK_OK;
