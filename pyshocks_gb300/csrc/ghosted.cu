@@ -47,6 +47,13 @@ namespace {
 constexpr int kGhThreads = 256;
 constexpr int kPad = 3;          // zero cells beyond each end of the array
 constexpr int kGhMaxBlocks = 1024;
+// Longest array (cells with ghosts) that one CTA handles. Measured in one CTA
+// against a launch per piece (us, step / transpose): constant reconstruction, LF:
+// 256 cells 14 / 29, 2048 cells 49 / 94 against 75 / 130; WENO-JS5, whose FP64
+// operations one SM carries alone: 256 cells 25 / 72, 1024 cells 78 / 250 against
+// 60 / 125.
+template <int REC>
+constexpr int64_t kGhBlockCells = REC == SHK_REC_CONSTANT ? 3072 : 512;
 
 struct GhArgs {
     int64_t n;   // interior cells
@@ -59,6 +66,10 @@ struct GhArgs {
     shk_boundary bc;
 };
 
+// Every piece is a device function over its elements (a grid-stride loop), so
+// that it runs as a kernel of its own on long arrays, or one after another in one
+// CTA on short ones (gh_step_block_kernel, gh_vjp_block_kernel), where a launch
+// per piece costs more than the piece.
 // ---- boundary fill (scalar.py:397-540) -------------------------------------
 // value at ghosted index i of the filled stage input v: interior unchanged;
 // periodic ghosts take the interior images (right ghosts the first g interior
@@ -78,7 +89,7 @@ __device__ __forceinline__ double gh_fill_value(const GhArgs& A, PV v, int64_t i
 }
 
 // vp[q], q = i + kPad: the filled array with kPad zeros on each side
-__global__ void gh_fill_kernel(GhArgs A, const double* __restrict__ v_, double* __restrict__ vp_,
+__device__ __forceinline__ void gh_fill(GhArgs A, const double* v_, double* vp_,
                                int stage) {
     const Win<const double> v = make_win(v_, A.M);
     const Win<double> vp = make_win(vp_, A.M + 2 * kPad);
@@ -89,11 +100,15 @@ __global__ void gh_fill_kernel(GhArgs A, const double* __restrict__ v_, double* 
         vp[q] = (i < 0 || i >= A.M) ? 0.0 : gh_fill_value(A, v, i, stage);
     }
 }
+__global__ void gh_fill_kernel(GhArgs A, const double* __restrict__ v_, double* __restrict__ vp_,
+                               int stage) {
+    gh_fill(A, v_, vp_, stage);
+}
 
 // ---- reconstruction of every cell (reconstruction.py:153-163, 351-377) -----
 template <int REC>
-__global__ void gh_recon_kernel(GhArgs A, const double* __restrict__ vp_, double* __restrict__ ul_,
-                                double* __restrict__ ur_) {
+__device__ __forceinline__ void gh_recon(GhArgs A, const double* vp_, double* ul_,
+                                double* ur_) {
     const Win<const double> vp = make_win(vp_, A.M + 2 * kPad);
     const Win<double> ul = make_win(ul_, A.M), ur = make_win(ur_, A.M);
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < A.M;
@@ -116,10 +131,15 @@ __global__ void gh_recon_kernel(GhArgs A, const double* __restrict__ vp_, double
         }
     }
 }
+template <int REC>
+__global__ void gh_recon_kernel(GhArgs A, const double* __restrict__ vp_, double* __restrict__ ul_,
+                                double* __restrict__ ur_) {
+    gh_recon<REC>(A, vp_, ul_, ur_);
+}
 
 // ---- global max of |f'| over the filled array and the cells attaining it ---
 template <int EQ>
-__global__ void gh_max_kernel(GhArgs A, const double* __restrict__ vp_, unsigned long long* amax) {
+__device__ __forceinline__ void gh_max(GhArgs A, const double* vp_, unsigned long long* amax) {
     const Win<const double> vp = make_win(vp_, A.M + 2 * kPad);
     __shared__ unsigned long long red[32];
     unsigned long long mx = 0;
@@ -132,7 +152,11 @@ __global__ void gh_max_kernel(GhArgs A, const double* __restrict__ vp_, unsigned
     if (threadIdx.x == 0) atomicMax(amax, bm);
 }
 template <int EQ>
-__global__ void gh_count_kernel(GhArgs A, const double* __restrict__ vp_,
+__global__ void gh_max_kernel(GhArgs A, const double* __restrict__ vp_, unsigned long long* amax) {
+    gh_max<EQ>(A, vp_, amax);
+}
+template <int EQ>
+__device__ __forceinline__ void gh_count(GhArgs A, const double* vp_,
                                 const unsigned long long* amax, unsigned int* count) {
     const Win<const double> vp = make_win(vp_, A.M + 2 * kPad);
     unsigned int cnt = 0;
@@ -142,6 +166,11 @@ __global__ void gh_count_kernel(GhArgs A, const double* __restrict__ vp_,
         cnt += abs_bits(wave_speed<EQ>(vp[i + kPad], A.c)) == m ? 1u : 0u;
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(count, cnt);
+}
+template <int EQ>
+__global__ void gh_count_kernel(GhArgs A, const double* __restrict__ vp_,
+                                const unsigned long long* amax, unsigned int* count) {
+    gh_count<EQ>(A, vp_, amax, count);
 }
 
 // wave speed of face j (between cells j-1 and j)
@@ -154,9 +183,9 @@ __device__ __forceinline__ double gh_face_speed(const GhArgs& A, double vl, doub
 
 // ---- fluxes and the stage update -------------------------------------------
 template <int EQ, int FLUX>
-__global__ void gh_flux_kernel(GhArgs A, const double* __restrict__ vp_, const double* __restrict__ ul_,
-                               const double* __restrict__ ur_, const unsigned long long* amax,
-                               double* __restrict__ F_) {
+__device__ __forceinline__ void gh_flux(GhArgs A, const double* vp_, const double* ul_,
+                               const double* ur_, const unsigned long long* amax,
+                               double* F_) {
     const Win<const double> vp = make_win(vp_, A.M + 2 * kPad);
     const Win<const double> ul = make_win(ul_, A.M), ur = make_win(ur_, A.M);
     const Win<double> F = make_win(F_, A.M + 1);
@@ -172,11 +201,17 @@ __global__ void gh_flux_kernel(GhArgs A, const double* __restrict__ vp_, const d
         F[j] = fma(0.5, phys_flux<EQ>(L, A.c) + phys_flux<EQ>(R, A.c), -((A.hnu * a) * (L - R)));
     }
 }
+template <int EQ, int FLUX>
+__global__ void gh_flux_kernel(GhArgs A, const double* __restrict__ vp_, const double* __restrict__ ul_,
+                               const double* __restrict__ ur_, const unsigned long long* amax,
+                               double* __restrict__ F_) {
+    gh_flux<EQ, FLUX>(A, vp_, ul_, ur_, amax, F_);
+}
 
 // out = cu u + ck (k + dt L),  L_i = -(F_{i+1} - F_i) / dx  (schemes.py:346,
 // timestepping.py:318-320)
-__global__ void gh_stage_kernel(GhArgs A, const double* __restrict__ u_, const double* __restrict__ k_,
-                                const double* __restrict__ F_, double* __restrict__ out_, double dt,
+__device__ __forceinline__ void gh_stage(GhArgs A, const double* u_, const double* k_,
+                                const double* F_, double* out_, double dt,
                                 double cu, double ck) {
     const Win<const double> u = make_win(u_, A.M), k = make_win(k_, A.M), F = make_win(F_, A.M + 1);
     const Win<double> out = make_win(out_, A.M);
@@ -186,14 +221,22 @@ __global__ void gh_stage_kernel(GhArgs A, const double* __restrict__ u_, const d
         out[i] = cu * u[i] + ck * (k[i] + dt * L);
     }
 }
+__global__ void gh_stage_kernel(GhArgs A, const double* __restrict__ u_, const double* __restrict__ k_,
+                                const double* __restrict__ F_, double* __restrict__ out_, double dt,
+                                double cu, double ck) {
+    gh_stage(A, u_, k_, F_, out_, dt, cu, ck);
+}
 
 // L_i = -(F_{i+1} - F_i) / dx on every cell, ghosts included (schemes.py:346)
-__global__ void gh_rhs_kernel(GhArgs A, const double* __restrict__ F_, double* __restrict__ out_) {
+__device__ __forceinline__ void gh_rhs(GhArgs A, const double* F_, double* out_) {
     const Win<const double> F = make_win(F_, A.M + 1);
     const Win<double> out = make_win(out_, A.M);
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < A.M;
          i += int64_t(gridDim.x) * blockDim.x)
         out[i] = -(F[i + 1] - F[i]) / A.dx;
+}
+__global__ void gh_rhs_kernel(GhArgs A, const double* __restrict__ F_, double* __restrict__ out_) {
+    gh_rhs(A, F_, out_);
 }
 
 // ---- transpose of one operator evaluation ----------------------------------
@@ -201,10 +244,10 @@ __global__ void gh_rhs_kernel(GhArgs A, const double* __restrict__ F_, double* _
 // w_{j-1}) / dx; gl[j] / gr[j-1]: cotangents of ul_j / ur_{j-1} through F_j;
 // ga[j]: of F_j's wave speed.
 template <int EQ, int FLUX>
-__global__ void gh_seed_kernel(GhArgs A, const double* __restrict__ vp_, const double* __restrict__ ul_,
-                               const double* __restrict__ ur_, const unsigned long long* amax,
-                               const double* __restrict__ w_, double dt, double* __restrict__ gl_,
-                               double* __restrict__ gr_, double* __restrict__ ga_) {
+__device__ __forceinline__ void gh_seed(GhArgs A, const double* vp_, const double* ul_,
+                               const double* ur_, const unsigned long long* amax,
+                               const double* w_, double dt, double* gl_,
+                               double* gr_, double* ga_) {
     const Win<const double> vp = make_win(vp_, A.M + 2 * kPad);
     const Win<const double> ul = make_win(ul_, A.M), ur = make_win(ur_, A.M), w = make_win(w_, A.M);
     const Win<double> gl = make_win(gl_, A.M), gr = make_win(gr_, A.M), ga = make_win(ga_, A.M + 1);
@@ -228,13 +271,20 @@ __global__ void gh_seed_kernel(GhArgs A, const double* __restrict__ vp_, const d
         ga[j] = -(fb * A.hnu) * (L - R);
     }
 }
+template <int EQ, int FLUX>
+__global__ void gh_seed_kernel(GhArgs A, const double* __restrict__ vp_, const double* __restrict__ ul_,
+                               const double* __restrict__ ur_, const unsigned long long* amax,
+                               const double* __restrict__ w_, double dt, double* __restrict__ gl_,
+                               double* __restrict__ gr_, double* __restrict__ ga_) {
+    gh_seed<EQ, FLUX>(A, vp_, ul_, ur_, amax, w_, dt, gl_, gr_, ga_);
+}
 
 // per-cell reconstruction backward: contributions t_o to the cotangents of
 // v_{c-2+o} (T[o * M + c]); constant: t_2 = gl + gr
 template <int REC>
-__global__ void gh_recon_vjp_kernel(GhArgs A, const double* __restrict__ vp_,
-                                    const double* __restrict__ gl_, const double* __restrict__ gr_,
-                                    double* __restrict__ T_) {
+__device__ __forceinline__ void gh_recon_vjp(GhArgs A, const double* vp_,
+                                    const double* gl_, const double* gr_,
+                                    double* T_) {
     const Win<const double> vp = make_win(vp_, A.M + 2 * kPad);
     const Win<const double> gl = make_win(gl_, A.M), gr = make_win(gr_, A.M);
     const Win<double> T = make_win(T_, 5 * A.M);
@@ -260,10 +310,16 @@ __global__ void gh_recon_vjp_kernel(GhArgs A, const double* __restrict__ vp_,
         }
     }
 }
+template <int REC>
+__global__ void gh_recon_vjp_kernel(GhArgs A, const double* __restrict__ vp_,
+                                    const double* __restrict__ gl_, const double* __restrict__ gr_,
+                                    double* __restrict__ T_) {
+    gh_recon_vjp<REC>(A, vp_, gl_, gr_, T_);
+}
 
 // sum of the face-speed cotangents of the global Lax-Friedrichs flux: fixed
 // per-block partial sums, then one ordered sum (deterministic)
-__global__ void gh_sum_partial_kernel(GhArgs A, const double* __restrict__ ga_, double* __restrict__ part) {
+__device__ __forceinline__ void gh_sum_partial(GhArgs A, const double* ga_, double* part) {
     const Win<const double> ga = make_win(ga_, A.M + 1);
     __shared__ double red[32];
     double s = 0.0;
@@ -279,12 +335,18 @@ __global__ void gh_sum_partial_kernel(GhArgs A, const double* __restrict__ ga_, 
         part[blockIdx.x] = r;
     }
 }
-__global__ void gh_sum_final_kernel(const double* __restrict__ part, int nparts, double* __restrict__ out) {
+__global__ void gh_sum_partial_kernel(GhArgs A, const double* __restrict__ ga_, double* __restrict__ part) {
+    gh_sum_partial(A, ga_, part);
+}
+__device__ __forceinline__ void gh_sum_final(const double* part, int nparts, double* out) {
     if (threadIdx.x == 0) {
         double r = 0.0;
         for (int b = 0; b < nparts; ++b) r += part[b];
         *out = r;
     }
+}
+__global__ void gh_sum_final_kernel(const double* __restrict__ part, int nparts, double* __restrict__ out) {
+    gh_sum_final(part, nparts, out);
 }
 
 // z_i: cotangent of the filled state at cell i (recon taps, face speeds, the
@@ -320,11 +382,11 @@ __device__ double gh_z(const GhArgs& A, Win<const double> vp, Win<const double> 
 }
 
 template <int EQ, int REC, int FLUX>
-__global__ void gh_gather_kernel(GhArgs A, const double* __restrict__ vp_, const double* __restrict__ T_,
-                                 const double* __restrict__ ga_, const unsigned long long* amax,
+__device__ __forceinline__ void gh_gather(GhArgs A, const double* vp_, const double* T_,
+                                 const double* ga_, const unsigned long long* amax,
                                  const unsigned int* count, const double* gsum, int mode,
-                                 const double* __restrict__ p_, double* __restrict__ cb_,
-                                 double* __restrict__ acc_, double* __restrict__ out_) {
+                                 const double* p_, double* cb_,
+                                 double* acc_, double* out_) {
     const Win<const double> vp = make_win(vp_, A.M + 2 * kPad);
     const Win<const double> T = make_win(T_, 5 * A.M), ga = make_win(ga_, A.M + 1);
     const Win<const double> p = make_win(p_, A.M);
@@ -362,21 +424,14 @@ __global__ void gh_gather_kernel(GhArgs A, const double* __restrict__ vp_, const
         }
     }
 }
-
-// ---- host side ----------------------------------------------------------------
-
-int gh_cuda(cudaError_t e) {
-    if (e != cudaSuccess) {
-        std::fprintf(stderr, "libshocks: CUDA error %s\n", cudaGetErrorString(e));
-        return SHK_ECUDA;
-    }
-    return SHK_OK;
+template <int EQ, int REC, int FLUX>
+__global__ void gh_gather_kernel(GhArgs A, const double* __restrict__ vp_, const double* __restrict__ T_,
+                                 const double* __restrict__ ga_, const unsigned long long* amax,
+                                 const unsigned int* count, const double* gsum, int mode,
+                                 const double* __restrict__ p_, double* __restrict__ cb_,
+                                 double* __restrict__ acc_, double* __restrict__ out_) {
+    gh_gather<EQ, REC, FLUX>(A, vp_, T_, ga_, amax, count, gsum, mode, p_, cb_, acc_, out_);
 }
-#define GH_CUDA(call)                       \
-    do {                                    \
-        const int _st = gh_cuda(call);      \
-        if (_st != SHK_OK) return _st;      \
-    } while (0)
 
 // workspace carve (doubles unless noted), P = M + 2 kPad
 struct GhWork {
@@ -397,6 +452,89 @@ struct GhWork {
     unsigned long long* amax;  // 3
     unsigned int* count;       // 3
 };
+
+// ---- one step, or its transpose, of a short array in one CTA ----------------
+// A step is 18 pieces and a transpose 30, each well under the 2 to 3 us that a
+// launch of its own takes at a few hundred cells; between them a block barrier
+// orders the workspace in global memory.
+constexpr int kGhBlockThreads = 512;
+
+template <int EQ, int REC, int FLUX>
+__device__ __forceinline__ void gh_block_operator(const GhArgs& A, const GhWork& W, const double* v, int stage,
+                                                  bool count) {
+    gh_fill(A, v, W.vp[stage], stage);
+    __syncthreads();
+    gh_recon<REC>(A, W.vp[stage], W.ul[stage], W.ur[stage]);
+    if constexpr (FLUX == SHK_FLUX_LF) {
+        gh_max<EQ>(A, W.vp[stage], W.amax + stage);
+        __syncthreads();
+        if (count) gh_count<EQ>(A, W.vp[stage], W.amax + stage, W.count + stage);
+    }
+    __syncthreads();
+}
+template <int EQ, int REC, int FLUX>
+__device__ __forceinline__ void gh_block_stage(const GhArgs& A, const GhWork& W, const double* u, const double* k,
+                                               double* out, int stage, double dt, double cu, double ck, bool count) {
+    gh_block_operator<EQ, REC, FLUX>(A, W, k, stage, count);
+    gh_flux<EQ, FLUX>(A, W.vp[stage], W.ul[stage], W.ur[stage], W.amax + stage, W.F);
+    __syncthreads();
+    gh_stage(A, u, k, W.F, out, dt, cu, ck);
+    __syncthreads();
+}
+__device__ __forceinline__ void gh_block_clear(const GhWork& W) {
+    if (threadIdx.x < 3) {
+        W.amax[threadIdx.x] = 0ull;
+        W.count[threadIdx.x] = 0u;
+    }
+    __syncthreads();
+}
+template <int EQ, int REC, int FLUX>
+__global__ void __launch_bounds__(kGhBlockThreads) gh_step_block_kernel(GhArgs A, GhWork W, const double* u,
+                                                                        double* out, double dt) {
+    gh_block_clear(W);
+    gh_block_stage<EQ, REC, FLUX>(A, W, u, u, W.k1, 0, dt, 0.0, 1.0, false);
+    gh_block_stage<EQ, REC, FLUX>(A, W, u, W.k1, W.k2, 1, dt, 3.0 / 4.0, 1.0 / 4.0, false);
+    gh_block_stage<EQ, REC, FLUX>(A, W, u, W.k2, out, 2, dt, 1.0 / 3.0, 2.0 / 3.0, false);
+}
+template <int EQ, int REC, int FLUX>
+__global__ void __launch_bounds__(kGhBlockThreads) gh_vjp_block_kernel(GhArgs A, GhWork W, const double* u,
+                                                                       const double* p, double* out, double dt) {
+    gh_block_clear(W);
+    gh_block_stage<EQ, REC, FLUX>(A, W, u, u, W.k1, 0, dt, 0.0, 1.0, true);
+    gh_block_stage<EQ, REC, FLUX>(A, W, u, W.k1, W.k2, 1, dt, 3.0 / 4.0, 1.0 / 4.0, true);
+    gh_block_operator<EQ, REC, FLUX>(A, W, W.k2, 2, true);
+#pragma unroll 1
+    for (int stage = 2; stage >= 0; --stage) {
+        const double* w = stage == 2 ? p : W.cb;
+        gh_seed<EQ, FLUX>(A, W.vp[stage], W.ul[stage], W.ur[stage], W.amax + stage, w, dt, W.gl, W.gr, W.ga);
+        __syncthreads();
+        gh_recon_vjp<REC>(A, W.vp[stage], W.gl, W.gr, W.T);
+        if constexpr (FLUX == SHK_FLUX_LF) {
+            gh_sum_partial(A, W.ga, W.part);
+            __syncthreads();
+            gh_sum_final(W.part, 1, W.gsum);
+        }
+        __syncthreads();
+        gh_gather<EQ, REC, FLUX>(A, W.vp[stage], W.T, W.ga, W.amax + stage, W.count + stage, W.gsum, stage + 1, p,
+                                 W.cb, W.acc, out);
+        __syncthreads();
+    }
+}
+
+// ---- host side ----------------------------------------------------------------
+
+int gh_cuda(cudaError_t e) {
+    if (e != cudaSuccess) {
+        std::fprintf(stderr, "libshocks: CUDA error %s\n", cudaGetErrorString(e));
+        return SHK_ECUDA;
+    }
+    return SHK_OK;
+}
+#define GH_CUDA(call)                       \
+    do {                                    \
+        const int _st = gh_cuda(call);      \
+        if (_st != SHK_OK) return _st;      \
+    } while (0)
 
 int64_t gh_bytes(int64_t M) {
     const int64_t P = M + 2 * kPad;
@@ -469,7 +607,7 @@ struct GhLaunch {
 };
 
 template <int EQ, int REC, int FLUX>
-int gh_operator(const GhLaunch& L, const double* v, int stage) {
+int launch_operator(const GhLaunch& L, const double* v, int stage) {
     // fill, reconstruct and (LF) the global max of the stage input v
     const GhArgs& A = L.A;
     const GhWork& W = L.W;
@@ -488,9 +626,9 @@ int gh_operator(const GhLaunch& L, const double* v, int stage) {
 }
 
 template <int EQ, int REC, int FLUX>
-int gh_stage(const GhLaunch& L, const double* u, const double* k, double* out, int stage, double dt,
+int launch_stage(const GhLaunch& L, const double* u, const double* k, double* out, int stage, double dt,
              double cu, double ck) {
-    int r = gh_operator<EQ, REC, FLUX>(L, k, stage);
+    int r = launch_operator<EQ, REC, FLUX>(L, k, stage);
     if (r != SHK_OK) return r;
     gh_flux_kernel<EQ, FLUX><<<L.blocks, kGhThreads, 0, L.st>>>(L.A, L.W.vp[stage], L.W.ul[stage],
                                                                L.W.ur[stage], L.W.amax + stage, L.W.F);
@@ -506,10 +644,14 @@ struct GhStep {
     double dt;
     template <int EQ, int REC, int FLUX>
     int run() {
+        if (L.A.M <= kGhBlockCells<REC>) {
+            gh_step_block_kernel<EQ, REC, FLUX><<<1, kGhBlockThreads, 0, L.st>>>(L.A, L.W, u, out, dt);
+            return gh_cuda(cudaGetLastError());
+        }
         GH_CUDA(cudaMemsetAsync(L.W.amax, 0, sizeof(unsigned long long) * 3 + sizeof(unsigned int) * 4, L.st));
-        int r = gh_stage<EQ, REC, FLUX>(L, u, u, L.W.k1, 0, dt, 0.0, 1.0);
-        if (r == SHK_OK) r = gh_stage<EQ, REC, FLUX>(L, u, L.W.k1, L.W.k2, 1, dt, 3.0 / 4.0, 1.0 / 4.0);
-        if (r == SHK_OK) r = gh_stage<EQ, REC, FLUX>(L, u, L.W.k2, out, 2, dt, 1.0 / 3.0, 2.0 / 3.0);
+        int r = launch_stage<EQ, REC, FLUX>(L, u, u, L.W.k1, 0, dt, 0.0, 1.0);
+        if (r == SHK_OK) r = launch_stage<EQ, REC, FLUX>(L, u, L.W.k1, L.W.k2, 1, dt, 3.0 / 4.0, 1.0 / 4.0);
+        if (r == SHK_OK) r = launch_stage<EQ, REC, FLUX>(L, u, L.W.k2, out, 2, dt, 1.0 / 3.0, 2.0 / 3.0);
         return r;
     }
 };
@@ -521,7 +663,7 @@ struct GhRhs {
     template <int EQ, int REC, int FLUX>
     int run() {
         GH_CUDA(cudaMemsetAsync(L.W.amax, 0, sizeof(unsigned long long) * 3 + sizeof(unsigned int) * 4, L.st));
-        int r = gh_operator<EQ, REC, FLUX>(L, u, 0);
+        int r = launch_operator<EQ, REC, FLUX>(L, u, 0);
         if (r != SHK_OK) return r;
         gh_flux_kernel<EQ, FLUX><<<L.blocks, kGhThreads, 0, L.st>>>(L.A, L.W.vp[0], L.W.ul[0], L.W.ur[0],
                                                                    L.W.amax, L.W.F);
@@ -559,11 +701,15 @@ struct GhVjp {
     }
     template <int EQ, int REC, int FLUX>
     int run() {
+        if (L.A.M <= kGhBlockCells<REC>) {
+            gh_vjp_block_kernel<EQ, REC, FLUX><<<1, kGhBlockThreads, 0, L.st>>>(L.A, L.W, u, p, out, dt);
+            return gh_cuda(cudaGetLastError());
+        }
         GH_CUDA(cudaMemsetAsync(L.W.amax, 0, sizeof(unsigned long long) * 3 + sizeof(unsigned int) * 4, L.st));
         // forward recompute: k1, k2 and the filled states of u, k1, k2
-        int r = gh_stage<EQ, REC, FLUX>(L, u, u, L.W.k1, 0, dt, 0.0, 1.0);
-        if (r == SHK_OK) r = gh_stage<EQ, REC, FLUX>(L, u, L.W.k1, L.W.k2, 1, dt, 3.0 / 4.0, 1.0 / 4.0);
-        if (r == SHK_OK) r = gh_operator<EQ, REC, FLUX>(L, L.W.k2, 2);
+        int r = launch_stage<EQ, REC, FLUX>(L, u, u, L.W.k1, 0, dt, 0.0, 1.0);
+        if (r == SHK_OK) r = launch_stage<EQ, REC, FLUX>(L, u, L.W.k1, L.W.k2, 1, dt, 3.0 / 4.0, 1.0 / 4.0);
+        if (r == SHK_OK) r = launch_operator<EQ, REC, FLUX>(L, L.W.k2, 2);
         // reverse: stage 3 at BC(k2) with w = p, stage 2 at BC(k1) with w = k2b,
         // stage 1 at BC(u) with w = k1b
         if (r == SHK_OK) r = reverse_stage<EQ, REC, FLUX>(2, p, 3);
