@@ -228,8 +228,10 @@ def check(status: int, what: str = "") -> None:
 
 
 def stream_handle(stream: torch.cuda.Stream | None = None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return int(s.cuda_stream)
+    if stream is not None:
+        return int(stream.cuda_stream)
+    # the current stream's handle without a Stream object (several us per call)
+    return int(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t: torch.Tensor | None) -> int | None:

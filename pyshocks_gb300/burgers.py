@@ -230,31 +230,30 @@ def c_boundary(bc: Boundary, grid: Grid, times) -> L.ShkBoundary | None:
     if isinstance(bc, PeriodicBoundary):
         return None
     out = L.ShkBoundary()
-    g, n = grid.nghosts, grid.ncells
-    h = float(grid.dx_min)
+    values, at = [], []  # Dirichlet data and its place in out.dirichlet
     for side, b in ((0, bc.left), (1, bc.right)):
         kind = L.SHK_BC_DIRICHLET if isinstance(b, DirichletBoundary) else L.SHK_BC_NEUMANN
         if side == 0:
             out.left = kind
-            idx = [g - 1 - k for k in range(min(g, 3))]
         else:
             out.right = kind
-            idx = [g + n + k for k in range(min(g, 3))]
-        x = grid.x[torch.tensor(idx, device=grid.x.device)].double()
-        if g < 3:
-            # cells beyond a grid with fewer than 3 ghosts (their values reach
-            # only ghost outputs): centres continued outward
-            x0 = float(grid.f[g]) if side == 0 else float(grid.f[g + n])
-            sgn = -1.0 if side == 0 else 1.0
-            extra = [x0 + sgn * (k + 0.5) * h for k in range(g, 3)]
-            x = torch.cat([x, torch.tensor(extra, dtype=x.dtype, device=x.device)])
-        for s_, ts in enumerate(times):
-            if kind == L.SHK_BC_DIRICHLET:
-                vals = torch.as_tensor(b.g(ts, x), dtype=torch.float64).reshape(-1).cpu()
-                for k in range(3):
-                    out.dirichlet[(s_ * 2 + side) * 3 + k] = float(vals[k])
-            else:
+        if kind == L.SHK_BC_NEUMANN:
+            for s_, ts in enumerate(times):
                 out.neumann[s_ * 2 + side] = float(b.g(ts))
+            continue
+        x = grid.ghost_centres(side)
+        for s_, ts in enumerate(times):
+            v = torch.as_tensor(b.g(ts, x), dtype=torch.float64).reshape(-1)
+            if v.numel() < 3:
+                raise IndexError(f"boundary data of 3 ghost cells expected, got {v.numel()}")
+            values.append(v[:3])
+            at.append((s_ * 2 + side) * 3)
+    if values:
+        # one copy to the host for all of it
+        same = all(v.device == values[0].device for v in values)
+        rows = torch.cat(values).tolist() if same else [w for v in values for w in v.tolist()]
+        for i, o in enumerate(at):
+            out.dirichlet[o : o + 3] = rows[3 * i : 3 * i + 3]
     return out
 
 
@@ -312,12 +311,17 @@ def _apply_operator_gpu(scheme, grid: Grid, bc: Boundary, t: Any, u: torch.Tenso
 def _predict_timestep_gpu(scheme, grid: Grid, bc: Boundary, t: Any, u: torch.Tensor):
     """``0.5 dx^(2-alpha) / max|f'(u_i)|`` (``src/pyshocks/burgers/schemes.py:121-127``)
     as a 0-d device tensor."""
+    return scaled_timestep(scheme, grid, 1.0, u)
+
+
+def scaled_timestep(scheme, grid: Grid, theta: float, u: torch.Tensor) -> torch.Tensor:
+    """``theta * predict_timestep`` (the driver's closure) in one library call."""
     _check_state(grid, u)
     lib = L.lib()
     dt = torch.empty((), dtype=torch.float64, device=u.device)
     L.check(
         lib.shk_predict_timestep_f64(scheme.c_scheme(grid.dx_min), u.data_ptr(), grid.ncells, grid.nghosts,
-                                     scheme.cfl_constant(grid.dx_min), 1.0, dt.data_ptr(),
+                                     scheme.cfl_constant(grid.dx_min), float(theta), dt.data_ptr(),
                                      L.stream_handle()),
         "predict_timestep",
     )

@@ -73,6 +73,12 @@ class TwoSidedBoundary(Boundary):
 
 @apply_boundary.register(TwoSidedBoundary)
 def _apply_boundary_two_sided(bc, grid, t, u):
+    if (type(bc.left) is NeumannBoundary and type(bc.right) is NeumannBoundary
+            and apply_boundary.dispatch(NeumannBoundary) is _apply_boundary_neumann):
+        u = u.clone()  # one copy for both sides
+        _fill_neumann(bc.left, grid, t, u)
+        _fill_neumann(bc.right, grid, t, u)
+        return u
     u = apply_boundary(bc.left, grid, t, u)
     return apply_boundary(bc.right, grid, t, u)
 
@@ -120,16 +126,21 @@ class NeumannBoundary(OneSidedBoundary):
 def _apply_boundary_neumann(bc, grid, t, u):
     """``src/pyshocks/scalar.py:467-495``."""
     u = u.clone()
+    _fill_neumann(bc, grid, t, u)
+    return u
+
+
+def _fill_neumann(bc, grid, t, u) -> None:
+    """The ghost cells of *u* (overwritten): the interior cells next to the
+    boundary mirrored, plus distance x gradient (none for a zero gradient)."""
     g = grid.nghosts
     n = u.shape[0]
-    ifrom = torch.arange(*grid.gi_[bc.side].indices(n), device=u.device)
-    if bc.side == -1:
-        ito = torch.arange(g - 1, -1, -1, device=u.device)
-    else:
-        ito = torch.arange(n - 1, n - g - 1, -1, device=u.device)
+    inner, ghost = (slice(g, 2 * g), slice(0, g)) if bc.side == -1 else (slice(n - 2 * g, n - g), slice(n - g, n))
     gn = float(bc.g(t))
-    u[ito] = u[ifrom] + bc.side * (grid.x[ifrom] - grid.x[ito]) * gn
-    return u
+    v = u[inner]
+    if gn != 0.0:
+        v = v + (grid.x[inner] - grid.x[ghost].flip(0)) * (bc.side * gn)
+    u[ghost] = v.flip(0)
 
 
 def make_neumann_boundary(ga: Callable, gb: Callable | None = None) -> TwoSidedBoundary:

@@ -89,8 +89,12 @@ class TimestepPredictor:
     theta: float = 1.0
 
     def __call__(self, t, u):
+        from pyshocks_gb300 import burgers
         from pyshocks_gb300.schemes import predict_timestep
 
+        if predict_timestep.dispatch(type(self.scheme)) is burgers._predict_timestep_gpu:
+            # the product is formed by the kernel that forms the estimate
+            return burgers.scaled_timestep(self.scheme, self.grid, self.theta, u)
         return self.theta * predict_timestep(self.scheme, self.grid, self.bc, t, u)
 
 
