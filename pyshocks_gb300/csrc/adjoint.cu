@@ -173,6 +173,163 @@ __device__ void vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<T>& a,
     __syncthreads();
 }
 
+// vjp_stage for the schemes of fixed_flux_scheme. The FP64 pipe bounded the
+// reverse step at 159 operations per cell and stage, most of them in the
+// reconstruction's backward. Its linear (ideal-weight) part, the flux seeds and
+// the sums stay in FP64 (25 operations); the rest, small where the state is
+// smooth, is formed in pairs of floats two cells per lane (lane_grad). Cells
+// with a weight change |x0| + |x2| above 1/8 or a third difference out of range
+// are listed and take the FP64 backward, less the linear part. In units of
+// g / 60: GR, GL, GA hold the flux seeds of the faces; a.H takes the pair part of
+// z, a.D the list, a.Q the flags of the listed cells, T0..T4 their taps.
+constexpr float kSmoothWeights = 0.125f;
+template <class PV, class PW, class PZ, class PC>
+__device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<double>& a, const OpParams<double>& p,
+                             double dtdx, PC UL, PC UR) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const Win<int> list = win_cast<int>(a.D), flag = win_cast<int>(a.Q);  // list[0]: count, from list[4]
+    if (tid == 0) list[0] = 0;
+    const double cf = dtdx * (1.0 / 120.0);
+    for (int j = lo - 3 + tid; j < hi + 2; j += nt) {
+        const double fb = (w[j + 1] - w[j]) * cf;
+        const double L = UL[j + 1], R = UR[j], s = absmax(v[j], v[j + 1]);
+        a.GL[j] = fb * (L - s);
+        a.GR[j] = fb * (R + s);
+        a.GA[j] = fb * (R - L);
+    }
+    __syncthreads();
+    const fx::FF eps4{fx::dup(p.e4h), fx::dup(p.e4l)};
+    // a warp takes 64 cells and finishes z of 58 (those at 4 .. 61)
+    const int first = (lo & ~1) - 4;
+    for (int r0 = first + 58 * warp; r0 + 4 < hi; r0 += 58 * nw) {
+        const int c0 = r0 + 2 * lane;
+        const int ca = c0 < a.W - 2 ? c0 : a.W - 2, cb = ca < a.W - 4 ? ca + 2 : a.W - 2;
+        auto ld2 = [](const auto& q, int i) { return *reinterpret_cast<const double2*>(win_span(q, i, 2)); };
+        const double2 va = ld2(v, ca), vb = ld2(v, cb), gr = ld2(a.GR, ca);
+        const double gl0 = a.GL[ca - 1], gl1 = a.GL[ca];
+        // the seeds relative to a power of two of the warp's largest (exact: the
+        // backward is linear in them)
+        unsigned em = 0;
+        {
+            auto top = [&](double q) {
+                const unsigned e = (static_cast<unsigned>(__double2hiint(q)) & 0x7fffffffu) >> 20;
+                em = e > em ? e : em;
+            };
+            if (c0 >= lo - 2 && c0 + 1 < hi + 2) {
+                top(gr.x);
+                top(gr.y);
+                top(gl0);
+                top(gl1);
+            }
+            em = __reduce_max_sync(kFull, em);
+        }
+        const bool out_of_range = em > 1846u;
+        em = em < 200u ? 200u : (out_of_range ? 1846u : em);
+        fx::CellGrad g;
+        {
+            fx::Cell x, y;
+            {
+                const fx::Mag m0 = fx::mag(v[ca - 1]), m1 = fx::mag(va.x), m2 = fx::mag(va.y), m3 = fx::mag(vb.x),
+                              m4 = fx::mag(vb.y);
+                x = fx::cell_begin(m0, m1, m2, m3);
+                y = fx::cell_begin(m1, m2, m3, m4);
+            }
+            const fx::P2 u0 = fx::p2(x.u0, y.u0), u12 = u0 * fx::dup(0x1p12f), u36 = u0 * fx::dup(0x1p36f);
+            const float nan = fx::bitsf(0x7fffffffu);
+            fx::FF T0 = fx::to_ff50(x.T, y.T, u0 * fx::dup(0x1p26f), u0);
+            T0.h = fx::p2(x.ok ? fx::p2x(T0.h) : nan, y.ok ? fx::p2y(T0.h) : nan);
+            const float Tmh = __shfl_up_sync(kFull, fx::p2y(T0.h), 1), Tml = __shfl_up_sync(kFull, fx::p2y(T0.l), 1);
+            const fx::FF Tm{fx::p2(Tmh, fx::p2x(T0.h)), fx::p2(Tml, fx::p2x(T0.l))};
+            float h0, l0, h1, l1;
+            fx::split_double(gr.x, em, h0, l0);
+            fx::split_double(gr.y, em, h1, l1);
+            const fx::FF gR{fx::p2(h0, h1), fx::p2(l0, l1)};
+            fx::split_double(gl0, em, h0, l0);
+            fx::split_double(gl1, em, h1, l1);
+            const fx::FF gL{fx::p2(h0, h1), fx::p2(l0, l1)};
+            g = fx::lane_grad(fx::to_ff(x.S, y.S, u36, u12, u0), fx::to_ff(x.E, y.E, u36, u12, u0), Tm, T0, eps4, gR,
+                              gL);
+        }
+        // listed cells: nothing here
+        const bool b0 = !(fx::p2x(g.x) <= kSmoothWeights) || out_of_range;
+        const bool b1 = !(fx::p2y(g.x) <= kSmoothWeights) || out_of_range;
+        auto keep = [&](fx::P2 q) { return fx::p2(b0 ? 0.0f : fx::p2x(q), b1 ? 0.0f : fx::p2y(q)); };
+        auto keep2 = [&](fx::FF q) { return fx::FF{keep(q.h), keep(q.l)}; };
+        const fx::FF tm = keep2(g.tm), t0 = keep2(g.t0), sg = keep2(g.sg), et = keep2(g.et);
+        auto mark = [&](int q, int c, bool bad) {
+            const bool mine = (q >= 4 && q < 62) || (r0 == first && q >= 2 && q < 4) || (r0 + 62 >= hi && q >= 62);
+            if (mine && c >= lo - 2 && c < hi + 2) {
+                flag[c] = bad ? 1 : 0;
+                if (bad) list[4 + atomicAdd(&list[0], 1)] = c;
+            }
+        };
+        mark(2 * lane, c0, b0);
+        mark(2 * lane + 1, c0 + 1, b1);
+        // transposes of T, E and S: the cotangent of T_c, of E_c, then z (neighbours'
+        // values from the lanes beside)
+        auto dn = [&](float q) { return __shfl_down_sync(kFull, q, 1); };
+        auto up = [&](float q) { return __shfl_up_sync(kFull, q, 1); };
+        const fx::FF tn{fx::p2(fx::p2y(tm.h), dn(fx::p2x(tm.h))), fx::p2(fx::p2y(tm.l), dn(fx::p2x(tm.l)))};
+        const fx::FF th = fx::add(t0, tn);
+        const fx::FF tp{fx::p2(up(fx::p2y(th.h)), fx::p2x(th.h)), fx::p2(up(fx::p2y(th.l)), fx::p2x(th.l))};
+        const fx::FF H = fx::add(et, fx::sub(tp, th));
+        const fx::FF P = fx::add(H, sg), M = fx::sub(H, sg);
+        const fx::FF Pp{fx::p2(up(fx::p2y(P.h)), fx::p2x(P.h)), fx::p2(up(fx::p2y(P.l)), fx::p2x(P.l))};
+        const fx::FF Mn{fx::p2(fx::p2y(M.h), dn(fx::p2x(M.h))), fx::p2(fx::p2y(M.l), dn(fx::p2x(M.l)))};
+        const fx::FF zz = fx::sub(fx::add(Pp, Mn), fx::twice(H));
+        const fx::P2 zh = zz.h + zz.l, zl = zz.l - (zh - zz.h);
+        if (lane >= 2 && lane <= 30) {
+            if (c0 >= lo && c0 < hi) a.H[c0] = fx::join_double(fx::p2x(zh), fx::p2x(zl), em);
+            if (c0 + 1 >= lo && c0 + 1 < hi) a.H[c0 + 1] = fx::join_double(fx::p2y(zh), fx::p2y(zl), em);
+        }
+    }
+    __syncthreads();
+    const int cnt = list[0];
+    for (int q = tid; q < cnt; q += nt) {
+        const int c = list[4 + q];
+        const double Hm2 = 0.5 * (v[c - 1] - v[c - 2]), Hm1 = 0.5 * (v[c] - v[c - 1]);
+        const double H0 = 0.5 * (v[c + 1] - v[c]), Hp1 = 0.5 * (v[c + 2] - v[c + 1]);
+        const double Dm1 = Hm1 - Hm2, D0 = H0 - Hm1, Dp1 = Hp1 - H0;
+        const double R = a.GR[c], L = a.GL[c - 1];
+        double t0, t1, t2, t3, t4;
+        weno53_cell_vjp<double>(Hm2, Hm1, H0, Hp1, Dm1, D0, Dp1, (13.0 / 3.0 * Dm1) * Dm1, (13.0 / 3.0 * D0) * D0,
+                                (13.0 / 3.0 * Dp1) * Dp1, p.eps, 60.0 * R, 60.0 * L, t0, t1, t2, t3, t4);
+        a.T0[c] = t0 - fma(2.0, R, -3.0 * L);
+        a.T1[c] = t1 - fma(-13.0, R, 27.0 * L);
+        a.T2[c] = t2 - 47.0 * (R + L);
+        a.T3[c] = t3 - fma(27.0, R, -13.0 * L);
+        a.T4[c] = t4 - fma(-3.0, R, 2.0 * L);
+    }
+    if (cnt > 0) __syncthreads();
+    for (int i = lo + tid; i < hi; i += nt) {
+        // ideal weights: taps (2, -13, 47, 27, -3) of the right face values, mirrored
+        // of the left ones
+        double s = fma(2.0, a.GR[i + 2] + a.GL[i - 3], 47.0 * (a.GR[i] + a.GL[i - 1]));
+        s = fma(-13.0, a.GR[i + 1] + a.GL[i - 2], s);
+        s = fma(27.0, a.GR[i - 1] + a.GL[i], s);
+        s = fma(-3.0, a.GR[i - 2] + a.GL[i + 1], s);
+        s = fma(10.0, a.H[i], s);
+        // wave speed terms of the two faces, 60 GA d max(|v_i|, |v_i+-1|) / dv_i
+        const double vi = v[i];
+        const auto bi = abs_bits(vi), bm = abs_bits(v[i - 1]), bp = abs_bits(v[i + 1]);
+        const double gm = a.GA[i - 1], gp = a.GA[i];
+        double q = bi > bm ? gm : (bi == bm ? 0.5 * gm : 0.0);
+        q += bi > bp ? gp : (bi == bp ? 0.5 * gp : 0.0);
+        s = fma(vi > 0.0 ? 60.0 : (vi < 0.0 ? -60.0 : 0.0), q, s);
+        if (cnt > 0) {
+            if (flag[i + 2]) s += a.T0[i + 2];
+            if (flag[i + 1]) s += a.T1[i + 1];
+            if (flag[i]) s += a.T2[i];
+            if (flag[i - 1]) s += a.T3[i - 1];
+            if (flag[i - 2]) s += a.T4[i - 2];
+        }
+        z[i] = s;
+    }
+    __syncthreads();
+}
+
 // Stage storage of one replayed step: k1, k2 (learned or float steps, in
 // float), plus the face values of u and k1 (double WENO-JS5 steps, in double),
 // each an array of the plan's `total` cells.
@@ -449,10 +606,15 @@ __device__ void adjoint_tile(const AdjSmem<T>& a, Win<T> gout, int te, T dtdx, c
     }
     }
     }
+    auto vjp = [&](auto v, auto w, auto z, int lo, int hi, const AdjSmem<T>& a_, const OpParams<T>& p_, T dtdx_,
+                   Win<T> ul, Win<T> ur) {
+        if constexpr (FLUX == kFluxRusanovFx) fx_vjp_stage(v, w, z, lo, hi, a_, p_, dtdx_, ul, ur);
+        else vjp_stage<T, EQ, REC>(v, w, z, lo, hi, a_, p_, dtdx_, ul, ur);
+    };
     // reverse stage 3: k2b = 2/3 (p + dt J(k2)^T p) on [HU-6, HU+te+6)
     {
         const int lo = HU - 6, hi = HU + te + 6;
-        vjp_stage<T, EQ, REC>(a.K2, a.PB, a.Z, lo, hi, a, p, dtdx, kCache ? a.UL : Win<T>(),
+        vjp(a.K2, a.PB, a.Z, lo, hi, a, p, dtdx, kCache ? a.UL : Win<T>(),
                               kCache ? a.UR : Win<T>());
         if (np) bc_transpose(a.Z, g0, n, lo, hi, bc);
         for (int i = lo + tid; i < hi; i += nt) a.CB[i] = T(2.0 / 3.0) * (a.PB[i] + a.Z[i]);
@@ -464,7 +626,7 @@ __device__ void adjoint_tile(const AdjSmem<T>& a, Win<T> gout, int te, T dtdx, c
     // reverse stage 2: k1b = 1/4 (k2b + dt J(k1)^T k2b) on [HU-3, HU+te+3)
     {
         const int lo = HU - 3, hi = HU + te + 3;
-        vjp_stage<T, EQ, REC>(a.K1, a.CB, a.Z, lo, hi, a, p, dtdx, kCache ? a.CL1 : Win<T>(),
+        vjp(a.K1, a.CB, a.Z, lo, hi, a, p, dtdx, kCache ? a.CL1 : Win<T>(),
                               kCache ? a.CR1 : Win<T>());
         if (np) bc_transpose(a.Z, g0, n, lo, hi, bc);
         for (int i = lo + tid; i < hi; i += nt) a.CB[i] = T(1.0 / 4.0) * (a.CB[i] + a.Z[i]);
@@ -483,7 +645,7 @@ __device__ void adjoint_tile(const AdjSmem<T>& a, Win<T> gout, int te, T dtdx, c
             if (g0 + HU == 0) lo -= 3;
             if (g0 + HU + te == n) hi += 3;
         }
-        vjp_stage<T, EQ, REC>(a.U, a.CB, a.Z, lo, hi, a, p, dtdx, kCache ? a.CLu : Win<T>(),
+        vjp(a.U, a.CB, a.Z, lo, hi, a, p, dtdx, kCache ? a.CLu : Win<T>(),
                               kCache ? a.CRu : Win<T>());
         if (np) bc_transpose(a.Z, g0, n, lo, hi, bc);
         for (int i = HU + tid; i < HU + te; i += nt) gout[i - HU] = a.ACC[i] + (a.CB[i] + a.Z[i]);

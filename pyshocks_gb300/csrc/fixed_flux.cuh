@@ -134,6 +134,12 @@ SHK_FX FF add(FF a, FF b) {
     const P2 e = (a.h - (s - bb)) + (b.h - bb);
     return FF{s, e + (a.l + b.l)};
 }
+SHK_FX FF sub(FF a, FF b) {
+    const P2 s = a.h - b.h;
+    const P2 bb = s - a.h;
+    const P2 e = (a.h - (s - bb)) - (b.h + bb);
+    return FF{s, e + (a.l - b.l)};
+}
 // |a| >= |b|
 SHK_FX FF add_ordered(FF a, FF b) {
     const P2 s = a.h + b.h;
@@ -299,6 +305,95 @@ SHK_FX void lane_cells(const Lane& s, float amh, float aml, float gph, float gpl
     pL = quot(add(X2, A), add(Y6, twice(r0)), 1.0f);
 }
 
+// ---- reverse mode of a lane's two cells --------------------------------------------
+// The smoothness sums and weights' derivatives of both face values of a cell as
+// cotangents of S, E, T_{c-1} and T_c. The linear (ideal-weight) part of the
+// reconstruction is left to the caller: with x_k = r_k - 1, formed without
+// cancellation from e_1 - e_0 = T_{c-1} (2S - T_{c-1} + 13/3 (2E - T_{c-1})) and
+// e_1 - e_2 = T_c (2S - T_c - 13/3 (2E + T_c)), the remaining weights
+//   r0/D_R - 1/10 = 3 (3 x0 - x2) / 10 D_R,  r2/D_R - 1/10 = (7 x2 - x0) / 10 D_R
+// (and mirrored on the left) are small where the state is smooth, and every term
+// below carries one of them or a third difference. gR, gL: 1/6 of the cotangents
+// of the face values; `x`: |x0| + |x2|, the caller's measure of smooth.
+struct CellGrad {
+    FF tm, t0, sg, et;
+    P2 x;
+};
+// a times a constant of few bits
+SHK_FX FF mul_const(FF a, float c) {
+    const P2 C = dup(c);
+    const P2 p = a.h * C;
+    return FF{p, fma2(a.l, C, fma2(a.h, C, neg(p)))};
+}
+SHK_FX P2 abs2(P2 a) { return p2(bitsf(fbits(p2x(a)) & 0x7fffffffu), bitsf(fbits(p2y(a)) & 0x7fffffffu)); }
+SHK_FX CellGrad lane_grad(FF S, FF E, FF Tm, FF T0, FF eps4, FF gR, FF gL) {
+    const FF c133{dup(4.33333349f), dup(-1.58945718e-07f)};  // 13/3
+    const FF c263{dup(8.66666698f), dup(-3.17891436e-07f)};  // 26/3
+    const FF c03{dup(0.300000012f), dup(-1.19209291e-08f)};  // 3/10
+    const FF one{dup(1.0f), dup(0.0f)}, ten{dup(10.0f), dup(0.0f)};
+    CellGrad g;
+    const FF h0 = sub(S, Tm), h2 = sub(S, T0), E0 = sub(E, Tm), E2 = add(E, T0);
+    const FF e1 = add(add(sqr(S), mul(sqr(E), c133)), eps4);
+    const FF e0 = add(add(sqr(h0), mul(sqr(E0), c133)), eps4);
+    const FF e2 = add(add(sqr(h2), mul(sqr(E2), c133)), eps4);
+    const FF b0 = mul(Tm, add(add(S, h0), mul(add(E, E0), c133)));
+    const FF b2 = mul(T0, sub(add(S, h2), mul(add(E, E2), c133)));
+    const FF x0 = mul(quot(b0, e0, 1.0f), quot(add(e1, e0), e0, 1.0f));
+    const FF x2 = mul(quot(b2, e2, 1.0f), quot(add(e1, e2), e2, 1.0f));
+    g.x = abs2(x0.h) + abs2(x2.h);
+    const FF X = add(ten, add(x0, x2));
+    const FF DR = add(X, twice(x2)), DL = add(X, twice(x0));
+    const FF r0 = add(one, x0), r2 = add(one, x2);
+    const FF A = mul(r0, Tm), B = mul(r2, T0), X2 = twice(add(A, B));
+    const FF pR = quot(add(X2, B), DR, -1.0f), pL = quot(add(X2, A), DL, 1.0f);
+    const FF a = quot(gR, DR, 1.0f), b = quot(gL, DL, 1.0f);
+    const FF a3 = add_ordered(twice(a), a), b3 = add_ordered(twice(b), b);
+    const FF u0 = sub(b3, twice(a)), u2 = sub(twice(b), a3);
+    // cotangents of r0, r2, then of e0, e1, e2
+    const FF m0 = add(mul(a, pR), mul(b3, pL)), m2 = add(mul(a3, pR), mul(b, pL));
+    const FF w0 = twice(mul(r0, sub(mul(Tm, u0), m0))), w2 = twice(mul(r2, sub(mul(T0, u2), m2)));
+    const FF k0 = quot(w0, e0, -1.0f), k2 = quot(w2, e2, -1.0f), k1 = quot(add(w0, w2), e1, 1.0f);
+    const FF hk0 = twice(mul(h0, k0)), hk2 = twice(mul(h2, k2));
+    const FF Ek0 = mul(mul(E0, k0), c263), Ek2 = mul(mul(E2, k2), c263);
+    // the weights beyond the ideal ones
+    const FF d = sub(x0, x2);
+    const FF y0 = add(twice(x0), d), y2 = sub(twice(x2), d);                        // 3 x0 - x2, 3 x2 - x0
+    const FF z0 = add(mul_const(x0, 4.0f), y0), z2 = add(mul_const(x2, 4.0f), y2);  // 7 x0 - x2, 7 x2 - x0
+    const FF o0 = mul(sub(mul(z0, b), twice(mul(y0, a))), c03);
+    const FF o2 = mul(sub(twice(mul(y2, b)), mul(z2, a)), c03);
+    g.sg = add(twice(mul(S, k1)), add(hk0, hk2));
+    g.et = add(mul(mul(E, k1), c263), add(Ek0, Ek2));
+    g.tm = sub(o0, add(hk0, Ek0));
+    g.t0 = add(o2, sub(Ek2, hk2));
+    return g;
+}
+
+// v 2^(1023 - em) as two floats (truncated upper part, exact rest), on the integer
+// pipe; em the biased exponent of the largest value of the warp, 200 .. 1846. 2^-120
+// below it and less: zero.
+SHK_FX void split_double(double v, uint32_t em, float& h, float& l) {
+    const uint32_t hi = static_cast<uint32_t>(dhi(v)), lo = dlo(v);
+    const uint32_t mag = hi & 0x7fffffffu;
+    const uint32_t fb = ((hi << 3) | (lo >> 29)) + ((0x400u - em + 0x7fu) << 23);
+    const uint32_t b = mag < ((em - 120u) << 20) ? 0u : ((fb & 0x7fffffffu) | (hi & 0x80000000u));
+    h = bitsf(b);
+    // the lower 29 bits of the mantissa, in units of 2^-52 of the upper part's
+    // power of two
+    l = (static_cast<float>(lo & 0x1fffffffu) * 0x1p-52f) * bitsf(b & 0xff800000u);
+}
+// (h + l) 2^(em - 1023) as a double, |l| at most a unit of h, on the integer pipe
+SHK_FX double join_double(float h, float l, uint32_t em) {
+    const uint32_t b = fbits(h), e = (b >> 23) & 0xffu;
+    const uint32_t es = 306u - (e > 60u ? e : 60u);
+    const int32_t li = f2i(l * bitsf(es << 23));
+    const int64_t u = (static_cast<int32_t>(b) < 0) ? -int64_t(li) : int64_t(li);
+    const uint64_t d = (uint64_t(((b & 0x7fffffffu) >> 3) + ((em - 127u) << 20)) << 32 | uint64_t(b << 29)) +
+                       static_cast<uint64_t>(u);
+    const bool zero = (b & 0x7fffffffu) == 0u;
+    return hilo(zero ? 0 : static_cast<int>(static_cast<uint32_t>(d >> 32) | (b & 0x80000000u)),
+                zero ? 0u : static_cast<uint32_t>(d));
+}
+
 // the sums and differences of the corrections of a lane's two faces, pR + pL
 // and pR - pL, in units: n 2^30 + r each, |p| < 2^52 units
 struct Sums {
@@ -306,7 +401,7 @@ struct Sums {
     P2 tR, tL;  // rounded to multiples of 2^30, plus the rounding constant
     P2 rs, rd;  // sum and difference of the rests
 };
-constexpr float kRound30 = 0x1.8p53f;
+constexpr float kRound30 = 0x1.8p53f;  // bits 0x5a400000
 SHK_FX Sums face_units(FF pR, FF pL, P2 iu) {
     Sums u;
     u.xR = pR.h * iu;
@@ -324,8 +419,8 @@ SHK_FX Sums face_units(FF pR, FF pL, P2 iu) {
 // face is left to the FP64 formula
 SHK_FX bool face_sums(const Cell& c, float xR, float xL, float tR, float tL, float rs, float rd, int64_t& Z,
                       int64_t& D, int64_t& Q) {
-    const int32_t bR = static_cast<int32_t>(fbits(tR)), bL = static_cast<int32_t>(fbits(tL));
-    const int32_t ns = bR + (bL - 2 * static_cast<int32_t>(0x5a400000)), nd = bR - bL;
+    const uint32_t bR = fbits(tR), bL = fbits(tL);
+    const int32_t ns = static_cast<int32_t>(bR + bL - 2u * 0x5a400000u), nd = static_cast<int32_t>(bR - bL);
     Z = int64_t(ns) * (int64_t(1) << 30) + (6 * c.VV - c.EE) + f2i(rs);
     D = int64_t(nd) * (int64_t(1) << 30) + c.T + f2i(rd);
     Q = D + static_cast<int64_t>(24u * c.A);

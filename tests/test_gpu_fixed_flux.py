@@ -65,3 +65,37 @@ def test_steps_match_oracle(kind, amp, flux):
     for b, n in enumerate(SIZES):
         err = np.max(np.abs(solver.instance(b).cpu().numpy() - refs[b])) / np.max(np.abs(u0[b]))
         assert err < 1.0e-13, (n, err)
+
+
+@pytest.mark.parametrize("kind", ["smooth", "noise", "front", "range"])
+@pytest.mark.parametrize("scale", [1.0, 1e-250, 1e-30, 1e200, 1e280])
+def test_transposed_step_matches_autograd(kind, scale):
+    """One reverse step (``fx_vjp_stage``) around a warp's 58 cells and the
+    tile of 512, with cotangents of any scale (the pairs of floats work relative
+    to the warp's largest). The oracle's step is differentiated at its own
+    rounding of the stages; the operator's second derivative is at most about
+    1 / sqrt(eps) = 1e3 per unit, so 1e-11 of the largest entry leaves two
+    digits over 1e3 times a step's roundings."""
+    import pyshocks_gb300 as gb
+    from pyshocks_gb300 import _lib as L
+    from pyshocks_gb300 import burgers
+
+    from oracle import torch_ref as T
+
+    rec = gb.reconstruction.make_reconstruction_from_name("wenojs53", eps=1.0e-6)
+    scheme = burgers.Rusanov(rec=rec)
+    rng = np.random.default_rng(5)
+    for n in [13, 57, 58, 59, 116, 117, 500, 512, 513, 1025]:
+        dx = 2.0 / n
+        u = torch.tensor(_state(kind, n, rng))
+        p = torch.tensor(rng.standard_normal(n)) * torch.tensor(np.exp(-0.05 * np.arange(n)))
+        dt = 0.4 * dx / float(u.abs().max())
+        ref = T.step_vjp(u[None], p[None], dt, dx)[0]
+        ud = torch.cat([u[-3:], u, u[:3]]).cuda()
+        pd = torch.cat([p[-3:], p, p[:3]]).cuda() * scale
+        out = torch.empty_like(ud)
+        st = L.lib().shk_ssprk33_vjp_f64(scheme.c_scheme(dx), ud.data_ptr(), pd.data_ptr(), out.data_ptr(), n, 3, dx,
+                                         dt, L.stream_handle())
+        assert st == 0, L.errstr(st)
+        got = (out / scale).cpu()[3:-3]
+        assert float((got - ref).abs().max()) <= 1.0e-11 * float(ref.abs().max()), n
