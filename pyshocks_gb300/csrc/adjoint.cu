@@ -303,6 +303,13 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         a.T4[c] = t4 - fma(-3.0, R, 2.0 * L);
     }
     if (cnt > 0) __syncthreads();
+    // the cotangent of max(x, y) that x takes, by the magnitudes' bits: all, half at
+    // a tie, none
+    auto share = [](double g, unsigned long long x, unsigned long long y) {
+        const int h = __double2hiint(g);
+        const int half = (h & 0x7ff00000) > 0x00100000 ? h - 0x00100000 : 0;
+        return __hiloint2double(x > y ? h : (x == y ? half : 0), x >= y ? __double2loint(g) : 0);
+    };
     for (int i = lo + tid; i < hi; i += nt) {
         // ideal weights: taps (2, -13, 47, 27, -3) of the right face values, mirrored
         // of the left ones
@@ -312,12 +319,12 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         s = fma(-3.0, a.GR[i - 2] + a.GL[i + 1], s);
         s = fma(10.0, a.H[i], s);
         // wave speed terms of the two faces, 60 GA d max(|v_i|, |v_i+-1|) / dv_i
+        // (compared, halved and signed on the integer pipe)
         const double vi = v[i];
         const auto bi = abs_bits(vi), bm = abs_bits(v[i - 1]), bp = abs_bits(v[i + 1]);
-        const double gm = a.GA[i - 1], gp = a.GA[i];
-        double q = bi > bm ? gm : (bi == bm ? 0.5 * gm : 0.0);
-        q += bi > bp ? gp : (bi == bp ? 0.5 * gp : 0.0);
-        s = fma(vi > 0.0 ? 60.0 : (vi < 0.0 ? -60.0 : 0.0), q, s);
+        const double q = share(a.GA[i - 1], bi, bm) + share(a.GA[i], bi, bp);
+        const int sgn60 = bi == 0 ? 0 : 0x404e0000 | (__double2hiint(vi) & static_cast<int>(0x80000000u));
+        s = fma(__hiloint2double(sgn60, 0), q, s);
         if (cnt > 0) {
             if (flag[i + 2]) s += a.T0[i + 2];
             if (flag[i + 1]) s += a.T1[i + 1];
@@ -732,13 +739,89 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED || FLUX == kF
     finish_items(P, 2);
 }
 
+// The reverse step of a periodic instance of a fixed_flux_scheme plan from the
+// replay's stored stages: one loop over the reverse stages, each loading its own
+// state and face values, in 13 windows (batched_adjoint_kernel keeps 24, for its
+// recompute) so that three CTAs fit an SM. UL/UR hold T0/T1 once the seeds are
+// formed; the cotangent is updated in place; Z overwrites the pair part.
+constexpr int kAdjFxArrays = 13;
+constexpr int kAdjFxThreads = 256, kAdjFxCtas = 3;
+__device__ __forceinline__ void carve_adjoint_fx(AdjSmem<double>& a, unsigned char* base, int W) {
+    double* p = reinterpret_cast<double*>(base);
+    Win<double>* slots[kAdjFxArrays] = {&a.U, &a.UL, &a.UR, &a.CB, &a.ACC, &a.GL, &a.GR,
+                                        &a.GA, &a.H, &a.D, &a.T2, &a.T3, &a.T4};
+    for (int i = 0; i < kAdjFxArrays; ++i) *slots[i] = make_win(p + size_t(i) * W, W);
+    a.T0 = a.UL;
+    a.T1 = a.UR;
+    a.Z = a.H;
+    // the list and the flags share one window: W ints each
+    Win<double> d = a.D;
+    a.Q = make_win(win_raw(d) + W / 2, W / 2);
+    a.D = make_win(win_raw(d), W / 2);
+    a.W = W;
+}
+__global__ void __launch_bounds__(kAdjFxThreads, kAdjFxCtas) batched_adjoint_fx_kernel(PlanDev P, const double* __restrict__ um,
+                                                                         const double* __restrict__ pnext,
+                                                                         double* __restrict__ pout,
+                                                                         const double* __restrict__ dt_row,
+                                                                         OpParams<double> p, const void* stages,
+                                                                         int64_t total) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int HU = adj_uhalo<double>();
+    AdjSmem<double> a;
+    carve_adjoint_fx(a, smem_raw, P.tile + 2 * HU);
+    const Win<const double> gum = make_win(um, total), gpnext = make_win(pnext, total);
+    const Win<double> gpout = make_win(pout, total);
+    __shared__ int s_item[2];
+    for (ItemQueue items(P, 2, s_item); items.more(); items.end()) {
+        const PlanItem it = items.begin();
+        const int b = it.b, te = it.te;
+        const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
+        const double dt = dt_row[b];
+        if (dt == 0.0) {  // no step was taken: identity
+            for (int i = threadIdx.x; i < te; i += blockDim.x) gpout[off + s0 + i] = gpnext[off + s0 + i];
+            continue;
+        }
+        const double dtdx = dt * P.inv_dx[b];
+        const int64_t g0 = s0 - HU;
+        const StageOut<const double> st =
+            as_const(stage_out<double, SHK_REC_WENOJS53>(const_cast<void*>(stages), total, off));
+        load_stage(a.CB, gpnext + off, n, g0, HU - 9, HU + te + 9);
+#pragma unroll 1
+        for (int s = 2; s >= 0; --s) {
+            // z on [lo, hi) from the state on 6 and the face values on 3 cells more
+            const int lo = HU - 3 * s, hi = HU + te + 3 * s;
+            load_stage(a.U, s == 2 ? st.k2 : (s == 1 ? st.k1 : gum + off), n, g0, lo - 6, hi + 6);
+            load_stage(a.UL, s == 2 ? st.ul2 : (s == 1 ? st.ul1 : st.ulu), n, g0, lo - 3, hi + 3);
+            load_stage(a.UR, s == 2 ? st.ur2 : (s == 1 ? st.ur1 : st.uru), n, g0, lo - 3, hi + 3);
+            __syncthreads();
+            fx_vjp_stage(a.U, a.CB, a.Z, lo, hi, a, p, dtdx, a.UL, a.UR);
+            for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+                const double q = a.CB[i], z = a.Z[i];
+                if (s == 2) {
+                    // k2b = 2/3 (p + Z), acc = 3/4 k2b + 1/3 p
+                    const double k = (2.0 / 3.0) * (q + z);
+                    a.CB[i] = k;
+                    a.ACC[i] = fma(3.0 / 4.0, k, (1.0 / 3.0) * q);
+                } else if (s == 1) {
+                    a.CB[i] = (1.0 / 4.0) * (q + z);
+                } else {
+                    gpout[off + s0 + i - HU] = a.ACC[i] + (q + z);
+                }
+            }
+            __syncthreads();
+        }
+    }
+    finish_items(P, 2);
+}
+
 // forward step with a recorded dt (no CFL, no time update): recompute of the
 // states between checkpoints
 // stages (optional): the step's stage storage, kStageArrays<T, REC> arrays of
 // P's cells in the stage precision (stage_arrays), for a reverse step that
 // skips its forward recompute; uout may then be null.
 template <class T, int EQ, int REC, int FLUX>
-__global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED ? 3 : (FLUX == kFluxRusanovFx ? 2 : 1)) replay_step_kernel(PlanDev P, const T* __restrict__ uin,
+__global__ void __launch_bounds__(flux_threads<FLUX>(), REC == SHK_REC_LEARNED ? 3 : (FLUX == kFluxRusanovFx ? 6 : 1)) replay_step_kernel(PlanDev P, const T* __restrict__ uin,
                                                                T* __restrict__ uout,
                                                                const double* __restrict__ dt_row,
                                                                OpParams<T> p, void* stages,
@@ -924,7 +1007,8 @@ struct ReplayLaunch {
         if constexpr (kHasFixed<T, EQ, REC>)
             if (fixed) k = replay_step_kernel<T, EQ, REC, kFluxRusanovFx>;
         ADJ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<grid, kThreads, smem, st>>>(D, static_cast<const T*>(uin), static_cast<T*>(uout), dt_row, p,
+        const int threads = kHasFixed<T, EQ, REC> && fixed ? kFxThreads : kThreads;
+        k<<<grid, threads, smem, st>>>(D, static_cast<const T*>(uin), static_cast<T*>(uout), dt_row, p,
                                          stages, total, step);
         return acuda(cudaGetLastError());
     }
@@ -1063,7 +1147,16 @@ int shk_plan_adjoint_staged(shk_plan* plan, const void* ckpt, int32_t stride, in
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int per_sm = std::max(1, static_cast<int>((220 * 1024) / std::max<size_t>(asmem, 1)));
+    int per_sm = std::max(1, static_cast<int>((220 * 1024) / std::max<size_t>(asmem, 1)));
+    // stored stages of a fixed-flux plan: batched_adjoint_fx_kernel
+    const bool fixed_stored = stages && dtype == SHK_F64 && fixed_flux_scheme(&sch);
+    const size_t xsmem = sizeof(double) * kAdjFxArrays * size_t(W);
+    if (fixed_stored) {
+        ADJ_CUDA(cudaFuncSetAttribute(batched_adjoint_fx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(xsmem)));
+        ADJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_adjoint_fx_kernel, kAdjFxThreads, xsmem));
+        per_sm = std::max(1, per_sm);
+    }
     const int agrid = std::max(1, std::min(D.nitems, per_sm * sms));
     auto seg_at = [&](int j) { return static_cast<char*>(seg) + size_t(j) * bytes; };
     // stage storage of segment step j
@@ -1096,7 +1189,12 @@ int shk_plan_adjoint_staged(shk_plan* plan, const void* ckpt, int32_t stride, in
         }
         for (int j = cnt - 1; j >= 0; --j) {
             const double* row = D.dt_hist + size_t(base + j) * D.B;
-            if (dtype == SHK_F64) {
+            if (fixed_stored) {
+                batched_adjoint_fx_kernel<<<agrid, kAdjFxThreads, xsmem, st>>>(
+                    D, reinterpret_cast<const double*>(seg_at(j)), static_cast<const double*>(cur),
+                    static_cast<double*>(nxt), row, adj_params<double>(&sch), stage_at(j), total);
+                r = acuda(cudaGetLastError());
+            } else if (dtype == SHK_F64) {
                 AdjLaunch<double> f{D, seg_at(j), cur, nxt, row, adj_params<double>(&sch), asmem, agrid, st,
                                     stage_at(j), total, base + j, fixed_flux_scheme(&sch)};
                 r = by_scheme<double>(sch, f);

@@ -612,7 +612,8 @@ int default_tile(const shk_scheme* s, int dtype, int max_steps) {
     if (s->rec == SHK_REC_LEARNED) return max_steps > 0 ? 1024 : 2048;
     if (s->rec == SHK_REC_WENOJS53 && s->flux == SHK_FLUX_RUSANOV) {
         if (dtype == SHK_F32) return max_steps > 0 ? 1024 : 2048;
-        return max_steps > 0 ? 512 : (fixed_flux_scheme(s) ? 946 : kDefaultTile);
+        if (fixed_flux_scheme(s)) return max_steps > 0 ? 448 : 946;
+        return max_steps > 0 ? 512 : kDefaultTile;
     }
     if (dtype == SHK_F64 && fixed_flux_scheme(s, SHK_FLUX_LF)) return 946;
     return kDefaultTile;
