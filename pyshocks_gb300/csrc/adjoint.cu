@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED || FLUX == kF
     const Win<const T> gpnext = make_win(pnext, total);
     const Win<T> gpout = make_win(pout, total);
     __shared__ int s_item[2];
-    for (ItemQueue items(P, 2, s_item); items.more(); items.end()) {
+    for (ItemQueue<REC != SHK_REC_LEARNED> items(P, 2, s_item); items.more(); items.end()) {
         const PlanItem it = items.begin();
         const int b = it.b, te = it.te;
         const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(kAdjFxThreads, kAdjFxCtas) batched_adjoint_fx_
     const Win<const double> gum = make_win(um, total), gpnext = make_win(pnext, total);
     const Win<double> gpout = make_win(pout, total);
     __shared__ int s_item[2];
-    for (ItemQueue items(P, 2, s_item); items.more(); items.end()) {
+    for (ItemQueue<> items(P, 2, s_item); items.more(); items.end()) {
         const PlanItem it = items.begin();
         const int b = it.b, te = it.te;
         const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), REC == SHK_REC_LEARNED ?
     const Win<const T> guin = make_win(uin, total);
     const Win<T> guout = make_win(uout, total);
     __shared__ int s_item[2];
-    for (ItemQueue items(P, 4, s_item); items.more(); items.end()) {
+    for (ItemQueue<REC != SHK_REC_LEARNED> items(P, 4, s_item); items.more(); items.end()) {
         const PlanItem it = items.begin();
         const int b = it.b, te = it.te;
         const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;

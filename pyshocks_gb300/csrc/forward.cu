@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
     const Win<T> guout = make_win(uout, total);
 
     __shared__ int s_item[2];
-    for (ItemQueue items(P, 0, s_item); items.more(); items.end()) {
+    for (ItemQueue<REC != SHK_REC_LEARNED> items(P, 0, s_item); items.more(); items.end()) {
         const PlanItem it = items.begin();
         const int b = it.b, te = it.te;
         const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(FX ? kFxThreads : kThreads, FX ? 8 : 1) batche
     bool ok = true;
     [[maybe_unused]] int slot = 0;
     __shared__ int s_item[2];
-    for (ItemQueue items(P, 6, s_item); items.more(); items.end()) {
+    for (ItemQueue<> items(P, 6, s_item); items.more(); items.end()) {
         const PlanItem it = items.begin();
         const int b = it.b, te = it.te;
         const int64_t off = it.off, n = it.n, s0 = int64_t(it.tile) * P.tile;
@@ -355,31 +355,55 @@ __global__ void __launch_bounds__(FX ? kFxThreads : kThreads, FX ? 8 : 1) batche
     }
 }
 
-__global__ void fill_kernel(double* x, int n, double v) {
+// plan reset in one launch (a memset per array cost the host stepper's chunks more
+// than their steps): counters, maxima and per-instance times; t0 / tfinal null: 0 /
+// no final time
+__global__ void reset_kernel(PlanDev P, unsigned long long* amax_lf, double* tfinal_dev, const double* t0,
+                             const double* tfinal) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[i] = v;
+    if (i < 2 * P.B) {
+        P.amax[i] = 0ull;
+        if (amax_lf) amax_lf[i] = 0ull;
+    }
+    if (i < P.B) {
+        P.left[i] = 0u;
+        P.t[i] = t0 ? t0[i] : 0.0;
+        tfinal_dev[i] = tfinal ? tfinal[i] : DBL_MAX;
+    }
+    if (i < 8) P.sched[i] = 0u;
+    if (i == 0) {
+        *P.step = 0;
+        *P.done = 0u;
+        *P.status = 0;
+    }
 }
 
-// max |f'(u)| per instance into amax[cur] (plan reset / priming)
+// max |f'(u)| per instance into amax[cur] (plan reset / priming): one read of the
+// state, eight loads in flight per thread (one at a time: 21 us for 22 MB)
 template <class T, int EQ>
 __global__ void __launch_bounds__(kThreads) batched_max_kernel(PlanDev P, const T* __restrict__ u, T c,
                                                                int slot) {
     __shared__ unsigned long long red[32];
     using B = typename Bits<T>::type;
-    for (int item = blockIdx.x; item < P.nitems; item += gridDim.x) {
-        const int b = P.item_inst[item];
-        const int64_t off = P.offsets[b];
-        const int64_t n = P.offsets[b + 1] - off;
-        const int64_t s0 = int64_t(P.item_tile[item]) * P.tile;
-        const int te = static_cast<int>(imin64(P.tile, n - s0));
+    for (int q = blockIdx.x; q < P.nitems; q += gridDim.x) {
+        const PlanItem it = P.items[q];
+        const T* v = u + it.off + int64_t(it.tile) * P.tile;
         B mx = 0;
-        for (int i = threadIdx.x; i < te; i += blockDim.x) {
-            const B bb = abs_bits(wave_speed<EQ>(u[off + s0 + i], c));
-            mx = bb > mx ? bb : mx;
+        for (int i0 = threadIdx.x; i0 < it.te; i0 += 8 * kThreads) {
+            T x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int i = i0 + k * kThreads;
+                x[k] = v[i < it.te ? i : i0];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const B bb = abs_bits(wave_speed<EQ>(x[k], c));
+                mx = bb > mx ? bb : mx;
+            }
         }
         const B bm = block_max<B>(mx, reinterpret_cast<B*>(red));
-        if (threadIdx.x == 0) atomicMax(P.amax + size_t(slot) * P.B + b, to_double_bits<T>(bm));
-        __syncthreads();
+        if (threadIdx.x == 0) atomicMax(P.amax + size_t(slot) * P.B + it.b, to_double_bits<T>(bm));
     }
 }
 
@@ -605,17 +629,36 @@ int cuda_check(cudaError_t e) {
         if (_st != SHK_OK) return _st;                  \
     } while (0)
 
-// the library's tile when the caller gives none: the shapes the autotuner
-// picks on the bench batches (plans that keep a dt history are tuned for
-// their reverse step, whose shared memory grows with the tile)
-int default_tile(const shk_scheme* s, int dtype, int max_steps) {
-    if (s->rec == SHK_REC_LEARNED) return max_steps > 0 ? 1024 : 2048;
-    if (s->rec == SHK_REC_WENOJS53 && s->flux == SHK_FLUX_RUSANOV) {
-        if (dtype == SHK_F32) return max_steps > 0 ? 1024 : 2048;
-        if (fixed_flux_scheme(s)) return max_steps > 0 ? 448 : 946;
-        return max_steps > 0 ? 512 : kDefaultTile;
+// The library's tile when the caller gives none, by the plan's cells: long tiles
+// waste the least on halos, short ones give a small batch more CTAs and a shorter
+// step. Where the lines lie (us per step, or per forward + reverse step of plans
+// that keep a dt history; 152 SMs):
+//   integer fluxes, forward: 65 k cells 20.7 (tile 226) / 22.8 (466) / 28.9 (946);
+//     442 k 50 / 39.8 / 43.2; 819 k 69 / 68 / 57 (706: 55.5); 4.1 M 253 / 221 / 213
+//   Lax-Friedrichs stages: 131 k 39.6 / 41.6 / 48.2; 1.2 M 134 / 111 / 119
+//   float32, forward: 65 k 10.7 (484) / 12.6 (2048); 819 k 22.8 / 16.7
+//   learned, forward: 65 k 20.6 (512) / 26.9 (1024) / 41.0 (2048); 262 k 48 / 36.5 /
+//     41; 3.3 M 279 / 255 / 240
+//   with history: integer fluxes 65 k 92 (216) / 104 (448), 262 k 187 / 206, 819 k
+//     429 / 403; float32 65 k 37.0 (512) / 42.3 (1024), 262 k 56 / 50; learned 65 k
+//     74 (512) / 98 (1024), 262 k 161 / 130
+// The integer-flux tiles are 60 faces (reverse: 58 cells) a warp in full rounds.
+int default_tile(const shk_scheme* s, int dtype, int max_steps, int64_t cells) {
+    const bool history = max_steps > 0;
+    if (s->rec == SHK_REC_LEARNED) {
+        if (cells <= 100000) return 512;
+        return history || cells <= 500000 ? 1024 : 2048;
     }
-    if (dtype == SHK_F64 && fixed_flux_scheme(s, SHK_FLUX_LF)) return 946;
+    if (dtype == SHK_F64 && fixed_flux_scheme(s)) {
+        if (history) return cells <= 400000 ? 216 : 448;
+        return cells <= 140000 ? 226 : (cells <= 600000 ? 466 : (cells <= 3000000 ? 706 : 946));
+    }
+    if (dtype == SHK_F64 && fixed_flux_scheme(s, SHK_FLUX_LF))
+        return cells <= 140000 ? 226 : (cells <= 2000000 ? 466 : 946);
+    if (s->rec == SHK_REC_WENOJS53 && s->flux == SHK_FLUX_RUSANOV) {
+        if (dtype == SHK_F32) return cells <= 120000 ? (history ? 512 : 484) : (history ? 1024 : 2048);
+        return history ? 512 : kDefaultTile;
+    }
     return kDefaultTile;
 }
 
@@ -936,10 +979,11 @@ int launch_max(shk_plan* P, const void* u, int slot, cudaStream_t st) {
     const PlanDev D = P->dev();
     const T c = static_cast<T>(P->scheme.speed);
     const T* uu = static_cast<const T*>(u);
+    const int grid = std::min(P->nitems, 8 * sm_count());
     switch (P->scheme.equation) {
-        case SHK_EQ_BURGERS: batched_max_kernel<T, SHK_EQ_BURGERS><<<P->grid, kThreads, 0, st>>>(D, uu, c, slot); break;
-        case SHK_EQ_ADVECTION: batched_max_kernel<T, SHK_EQ_ADVECTION><<<P->grid, kThreads, 0, st>>>(D, uu, c, slot); break;
-        default: batched_max_kernel<T, SHK_EQ_LWR><<<P->grid, kThreads, 0, st>>>(D, uu, c, slot); break;
+        case SHK_EQ_BURGERS: batched_max_kernel<T, SHK_EQ_BURGERS><<<grid, kThreads, 0, st>>>(D, uu, c, slot); break;
+        case SHK_EQ_ADVECTION: batched_max_kernel<T, SHK_EQ_ADVECTION><<<grid, kThreads, 0, st>>>(D, uu, c, slot); break;
+        default: batched_max_kernel<T, SHK_EQ_LWR><<<grid, kThreads, 0, st>>>(D, uu, c, slot); break;
     }
     return cuda_check(cudaGetLastError());
 }
@@ -1140,7 +1184,8 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
     // global Lax-Friedrichs: float64 stage states kept between the stage launches
     const bool lf = scheme->flux == SHK_FLUX_LF;
     if (lf && dtype != SHK_F64) return SHK_EUNSUPPORTED;
-    int tile = (opts && opts->tile > 0) ? opts->tile : default_tile(scheme, dtype, opts ? opts->max_steps : 0);
+    int tile = (opts && opts->tile > 0) ? opts->tile : default_tile(scheme, dtype, opts ? opts->max_steps : 0,
+                                                                  h_offsets[batch] - h_offsets[0]);
     const int align = dtype == SHK_F64 ? 2 : 4;
     if (tile % align || tile < 16 || tile > 8192) return SHK_EINVAL;
     // the learned phase's warp scratch lives in the window's free arrays
@@ -1315,21 +1360,10 @@ int shk_plan_reset(shk_plan* plan, const void* u, const double* t0, const double
     if (!plan || !u) return SHK_EINVAL;
     cudaStream_t st = as_stream(stream);
     const int B = plan->B;
-    SHK_CUDA(cudaMemsetAsync(plan->amax, 0, sizeof(unsigned long long) * 2 * B, st));
-    if (plan->amax_lf) SHK_CUDA(cudaMemsetAsync(plan->amax_lf, 0, sizeof(unsigned long long) * 2 * B, st));
-    SHK_CUDA(cudaMemsetAsync(plan->step, 0, sizeof(int64_t), st));
-    SHK_CUDA(cudaMemsetAsync(plan->done, 0, sizeof(unsigned), st));
-    SHK_CUDA(cudaMemsetAsync(plan->sched, 0, sizeof(unsigned) * 8, st));
-    SHK_CUDA(cudaMemsetAsync(plan->left, 0, sizeof(unsigned) * B, st));
-    SHK_CUDA(cudaMemsetAsync(plan->status, 0, sizeof(int32_t), st));
-    if (t0) SHK_CUDA(cudaMemcpyAsync(plan->t, t0, sizeof(double) * B, cudaMemcpyDeviceToDevice, st));
-    else SHK_CUDA(cudaMemsetAsync(plan->t, 0, sizeof(double) * B, st));
-    if (tfinal) {
-        SHK_CUDA(cudaMemcpyAsync(plan->tfinal, tfinal, sizeof(double) * B, cudaMemcpyDeviceToDevice, st));
-    } else {  // no final time; a kernel, so that a reset never waits on the host
-        fill_kernel<<<(B + kThreads - 1) / kThreads, kThreads, 0, st>>>(plan->tfinal, B, DBL_MAX);
-        SHK_CUDA(cudaGetLastError());
-    }
+    const int threads = std::max(8, 2 * B);
+    reset_kernel<<<(threads + kThreads - 1) / kThreads, kThreads, 0, st>>>(plan->dev(), plan->amax_lf, plan->tfinal,
+                                                                         t0, tfinal);
+    SHK_CUDA(cudaGetLastError());
     if (plan->dt_hist)
         SHK_CUDA(cudaMemsetAsync(plan->dt_hist, 0, sizeof(double) * size_t(plan->max_steps) * B, st));
     plan->host_steps = 0;

@@ -1091,10 +1091,13 @@ struct PlanDev {
 // Dynamic item scheduling. A CTA takes the items of the plan's longest-first
 // list from the counter sched[slot]; uneven items (partial tiles, copied-through
 // instances) then balance over the persistent grid, where a fixed stride would
-// hand some CTAs only long items. The first item is the CTA's own index; the next
-// one is requested when an item begins, so the counter's latency is behind it.
+// hand some CTAs only long items. The first item is the CTA's own index. EARLY:
+// the next one is requested when an item begins, so the counter's latency is
+// behind it; kernels with few, long and unequal items take it when an item ends
+// (bound early, the learned reverse step lost 12 % to the imbalance).
 // s: two words of shared memory (a thread may still read one when the next is
 // written).
+template <bool EARLY = true>
 struct ItemQueue {
     const PlanDev& P;
     int slot;
@@ -1105,12 +1108,12 @@ struct ItemQueue {
         : P(P_), slot(slot_), s(s_), q(static_cast<int>(blockIdx.x)) {}
     __device__ __forceinline__ bool more() const { return q < P.nitems; }
     __device__ __forceinline__ PlanItem begin() {
-        if (threadIdx.x == 0) next = atomicAdd(P.sched + slot, 1u) + gridDim.x;
+        if (EARLY && threadIdx.x == 0) next = atomicAdd(P.sched + slot, 1u) + gridDim.x;
         return P.items[q];
     }
     // a barrier
     __device__ __forceinline__ void end() {
-        if (threadIdx.x == 0) s[par] = static_cast<int>(next);
+        if (threadIdx.x == 0) s[par] = static_cast<int>(EARLY ? next : atomicAdd(P.sched + slot, 1u) + gridDim.x);
         __syncthreads();
         q = s[par];
         par ^= 1;
