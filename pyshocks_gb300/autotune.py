@@ -26,6 +26,11 @@ import torch
 
 #: candidate tile lengths (multiples of 16 cells keep every window 16-byte aligned)
 TILES = (512, 1024, 2048, 4096)
+#: float64 WENO-JS5 plans add the tiles that fill whole rounds of the integer-flux
+#: kernels' warps (60 faces each; 58 outputs each in the reverse step): 4096
+#: instances, 25.9 M cells, per step: tile 946 1129 us, 706 1164, 466 1246
+TILES_F64 = (226, 466, 706, 946)
+TILES_F64_ADJOINT = (216, 448)
 #: candidate resident CTAs per SM (0: the plan's own choice from shared memory)
 CTAS_PER_SM = (0, 1, 2, 3, 4)
 #: the shared memory one SM offers to resident CTAs (bytes)
@@ -96,7 +101,10 @@ def candidates(dtype: torch.dtype, max_cells: int, learned: bool = False,
     than twice the largest instance are skipped (they only add idle lanes);
     with ``adjoint`` only tiles whose reverse step fits too."""
     out = []
-    for tile in TILES:
+    tiles = TILES
+    if dtype == torch.float64 and weno5:
+        tiles = (TILES_F64_ADJOINT if adjoint else TILES_F64) + TILES
+    for tile in tiles:
         if tile > max(2 * max_cells, TILES[0]):
             continue
         if adjoint and _adjoint_smem_bytes(tile, dtype, learned) > SMEM_PER_SM:
@@ -148,7 +156,8 @@ def tune(scheme, sizes: Sequence[int], dx, *, dtype: torch.dtype = torch.float64
     """
     from pyshocks_gb300.batched import BatchedSolver, pack_offsets
 
-    key = shape_key(scheme, sizes, dtype, device) + (":adjoint" if adjoint else "")
+    # (v2: shapes timed on kernels with other CTA sizes are not taken from the file)
+    key = shape_key(scheme, sizes, dtype, device) + (":adjoint" if adjoint else "") + ":v2"
     if use_cache:
         if key in _MEMO:
             return _MEMO[key]

@@ -58,12 +58,46 @@ __device__ __forceinline__ bool finish_tile(const PlanDev& P, int64_t k, int b, 
     return true;
 }
 
+// A tile whose maximum and completion are still to be reported. kDefer: the atomics
+// (one returns a value, behind a fence) run while the next item's window is in flight
+// instead of before its load. Measured, 4096 instances (25.9 M cells), ten float32
+// steps: 2491 -> 2413 us; learned float64: 1051 -> 1039 us. The integer-flux kernel
+// reports at once: eight CTAs on an SM hide each other's atomics already (4096
+// instances, two steps: 2398 us, deferred 2413; 300 ragged instances, ten steps:
+// 693 us, deferred 731). wmax: the warps' maxima of |f'|, as double bits.
+template <int FLUX>
+inline constexpr bool kDefer = FLUX != kFluxRusanovFx;
+struct PendingTile {
+    unsigned long long wmax[32];
+    DtState dt;
+    int b, tiles;  // b < 0: none
+};
+__device__ __forceinline__ void pending_fill(PendingTile& pt, unsigned long long mx, int b, int tiles,
+                                             const DtState& dt) {
+    mx = warp_max(mx);
+    if ((threadIdx.x & 31) == 0) pt.wmax[threadIdx.x >> 5] = mx;
+    if (threadIdx.x == 0) {
+        pt.dt = dt;
+        pt.b = b;
+        pt.tiles = tiles;
+    }
+}
+// thread 0, after a barrier
+__device__ __forceinline__ void pending_flush(PendingTile& pt, const PlanDev& P, int64_t k, unsigned long long* amax) {
+    if (pt.b < 0) return;
+    unsigned long long m = pt.wmax[0];
+    for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) m = pt.wmax[w] > m ? pt.wmax[w] : m;
+    atomicMax(amax + pt.b, m);
+    finish_tile(P, k, pt.b, pt.tiles, pt.dt);
+}
+
 template <class T, int EQ, int REC, int FLUX>
 __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ? 8 : (REC == SHK_REC_LEARNED ? 3 : (REC == SHK_REC_WENOJS53 ? (sizeof(T) == 8 ? 3 : 4) : 1))) batched_step_kernel(PlanDev P, const T* __restrict__ uin,
                                                                 T* __restrict__ uout, OpParams<T> p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
-    __shared__ unsigned long long red[32];
+    __shared__ PendingTile pending;         // kDefer
+    __shared__ unsigned long long red[32];  // else
     __shared__ DtState item_dt;  // the item's step, computed once per CTA
     __shared__ T item_dtdx, item_dx;
     constexpr int HL = step_halo<T>();
@@ -72,6 +106,7 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
     Smem<T> sm;
     carve_step<T, REC, FLUX>(sm, smem_raw, P.tile + 2 * HL);
     if (threadIdx.x == 0) {
+        if constexpr (kDefer<FLUX>) pending.b = -1;
         mbar_init(&bar, 1);
         fence_mbar_init();
     }
@@ -94,6 +129,9 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
         // this GPU) while the window is in flight, and shares it; the previous
         // item's readers are past the barrier that ended that item
         ok = load_window<T>(sm.U, uin + off, n, s0 - HL, te + 2 * HL, &bar, phase, [&] {
+            if constexpr (kDefer<FLUX>) {
+                if (threadIdx.x == 0) pending_flush(pending, P, k, P.amax + size_t(nxt) * P.B);
+            }
             if (threadIdx.x == 32) {
                 const DtState d = plan_dt(P, k, b, from_bits(P.amax[size_t(cur) * P.B + b]));
                 item_dt = d;
@@ -102,7 +140,10 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
             }
         });
         if (!ok) {
-            if (threadIdx.x == 0) atomicOr(P.status, ERR_TIMEOUT);
+            if (threadIdx.x == 0) {
+                atomicOr(P.status, ERR_TIMEOUT);
+                if constexpr (kDefer<FLUX>) pending.b = -1;
+            }
             break;
         }
         const DtState ds = item_dt;
@@ -122,15 +163,20 @@ __global__ void __launch_bounds__(flux_threads<FLUX>(), FLUX == kFluxRusanovFx ?
             mx = step_tile<T, EQ, REC, FLUX>(sm, guout + (off + s0), te, dtdx, pb, plan_bc(P, b, k),
                                              s0 - HL, n);
         }
-        const B bm = block_max<B>(mx, reinterpret_cast<B*>(red));
-        if (threadIdx.x == 0) {
-            atomicMax(P.amax + size_t(nxt) * P.B + b, to_double_bits<T>(bm));
-            finish_tile(P, k, b, it.tiles, ds);
+        if constexpr (kDefer<FLUX>) {
+            pending_fill(pending, to_double_bits<T>(mx), b, it.tiles, ds);
+        } else {
+            const B bm = block_max<B>(mx, reinterpret_cast<B*>(red));
+            if (threadIdx.x == 0) {
+                atomicMax(P.amax + size_t(nxt) * P.B + b, to_double_bits<T>(bm));
+                finish_tile(P, k, b, it.tiles, ds);
+            }
         }
     }
 
     // the last CTA of the step increments the step counter (no host round trip)
     if (threadIdx.x == 0) {
+        if constexpr (kDefer<FLUX>) pending_flush(pending, P, k, P.amax + size_t(nxt) * P.B);
         __threadfence();
         if (atomicAdd(P.done, 1u) == gridDim.x - 1) {
             __threadfence();

@@ -69,3 +69,29 @@ def test_predicted_timestep(n):
         assert st == 0
         assert float(dt) == 0.5 * (0.125 / 1.7)
 
+
+@pytest.mark.parametrize("ctas", [1, 0])
+@pytest.mark.parametrize(("dtype", "flux"), [("float32", "burgers"), ("float32", "lwr"), ("float64", "lwr")])
+def test_many_items_per_cta_report_every_maximum(dtype, flux, ctas):
+    """A CTA's tiles report their maximum and completion with its next item (or
+    after its last): with 64-cell tiles a CTA takes up to about forty, of instances
+    that end at every point of its list, and states and times must equal, bit for
+    bit, those of one CTA per tile."""
+    from test_gpu_adjoint import _scheme
+
+    from pyshocks_gb300.batched import BatchedSolver
+
+    sizes = [n for n in (20011, 7, 333, 64, 65, 4097, 15, 1999) for _ in range(12)]
+    rng = np.random.default_rng(61)
+    u0 = torch.tensor(np.concatenate([0.5 + 0.3 * np.sin(2 * np.pi * (np.arange(n) / n + rng.uniform()))
+                                      * rng.uniform(0.2, 1.0) for n in sizes]))
+    out = []
+    for tile, c in ((64, ctas), (2048, 0)):
+        s = BatchedSolver(_scheme(*(("lwr",) if flux == "lwr" else ())), sizes, [2.0 / n for n in sizes], tile=tile,
+                          ctas_per_sm=c, dtype=getattr(torch, dtype))
+        s.reset(u0)
+        s.step(5)
+        assert s.status() == 0
+        out.append((s.u.clone(), s.time()))
+    assert torch.equal(out[0][0], out[1][0])
+    assert torch.equal(out[0][1], out[1][1])
