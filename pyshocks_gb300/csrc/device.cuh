@@ -10,7 +10,8 @@
 //   ES-WENO flux src/pyshocks/burgers/schemes.py:230-256
 //   SSPRK33      src/pyshocks/timestepping.py:312-320
 // reorganised to cut the FP64 instruction count (the FP64 pipe, not HBM,
-// bounds this path on GB300):
+// bounds these formulas on GB300; double Burgers states with WENO-JS5 and the
+// Rusanov or Lax-Friedrichs flux leave that pipe, see fixed_flux.cuh):
 //   * one set of smoothness indicators per cell serves both faces: the
 //     mirrored left reconstruction sees beta_k of the right one as beta_{2-k};
 //   * squares of second differences and half first differences are computed
