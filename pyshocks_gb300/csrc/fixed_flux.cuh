@@ -26,8 +26,10 @@
 // instructions (add/mul/fma.f32x2).
 // Measured on the batched step (4096 instances, 25.9 M cells, us per step): 8010
 // with the FP64 formula (156 FP64 instructions per cell-step, that pipe 86 %
-// busy), 1199 with this. Error of the states against 64-bit-exact solutions:
-// unchanged (1.4e-16 relative at that batch, 2.9e-16 on 300 ragged instances).
+// busy), 1199 with this. Error of the states against runs in 113-bit arithmetic
+// (Fourier modes and a jump; relative L2, FP64 formula / this): 40 instances of 100
+// to 1000 cells, 50 steps 2.9865e-15 / 2.9869e-15; 40 of 500 to 9000, 10 steps
+// 6.242e-16 / 6.217e-16; 16 of 1024 to 8192, 4 steps 2.674e-16 / 2.674e-16.
 #pragma once
 
 #include <cstdint>
