@@ -34,8 +34,14 @@ __host__ __device__ constexpr int mixed_d_len(int W) { return W > kLearnedScratc
 // The FLUX code of kernels whose Rusanov flux runs on fixed_flux.cuh: double
 // states, Burgers, WENO-JS5, nu = 1 (fixed_flux_scheme). nu enters that flux as
 // 24 a with an integer a; other nu and the other equations keep the FP64
-// formula.
+// formula. So do smoothness parameters outside [kFxEpsMin, kFxEpsMax]: the smoothness
+// sums are pairs of floats of at least 4 eps, and their lower halves (2^-48 of
+// them) must stay above float's smallest number, 2^-149. Against 113-bit
+// arithmetic no accepted face is off by more than 4 units of 2^-53 of the largest
+// value squared for eps >= 1e-30; at eps = 1e-36 it was 1e4 units, at 1e-40 3e7 (the
+// FP64 formula: 4 to 6).
 constexpr int kFluxRusanovFx = 100;
+constexpr double kFxEpsMin = 1.0e-24, kFxEpsMax = 1.0e24;
 // 4-warp CTAs: a stage's warps wait for each other at two barriers, so many small
 // CTAs keep the SM busy where few large ones stall (256 threads, 3 CTAs per SM:
 // issue 43 %). Us per step at 25.9 M cells by CTAs per SM (tile): 6 (1186) 1247,
@@ -44,7 +50,8 @@ constexpr int kFxThreads = 128;
 template <int FLUX>
 __host__ __device__ constexpr int flux_threads() { return FLUX == kFluxRusanovFx ? kFxThreads : kThreads; }
 inline bool fixed_flux_scheme(const shk_scheme* s, int flux = SHK_FLUX_RUSANOV) {
-    return s->flux == flux && s->rec == SHK_REC_WENOJS53 && s->equation == SHK_EQ_BURGERS && s->nu == 1.0;
+    return s->flux == flux && s->rec == SHK_REC_WENOJS53 && s->equation == SHK_EQ_BURGERS && s->nu == 1.0 &&
+           s->eps >= kFxEpsMin && s->eps <= kFxEpsMax;
 }
 
 // halo of a window: 9 cells are needed for three fused stages, rounded up so
