@@ -211,19 +211,20 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         const double2 va = ld2(v, ca), vb = ld2(v, cb), gr = ld2(a.GR, ca);
         const double gl0 = a.GL[ca - 1], gl1 = a.GL[ca];
         // the seeds relative to a power of two of the warp's largest (exact: the
-        // backward is linear in them)
+        // backward is linear in them). Every cell whose seeds are used counts, by
+        // itself: [lo - 2, hi + 2) may begin or end inside a lane's pair, and beyond it
+        // the seeds are not written
         unsigned em = 0;
         {
-            auto top = [&](double q) {
-                const unsigned e = (static_cast<unsigned>(__double2hiint(q)) & 0x7fffffffu) >> 20;
-                em = e > em ? e : em;
+            auto top = [&](int c, double r, double l) {
+                if (c < lo - 2 || c >= hi + 2) return;
+                const unsigned er = (static_cast<unsigned>(__double2hiint(r)) & 0x7fffffffu) >> 20;
+                const unsigned el = (static_cast<unsigned>(__double2hiint(l)) & 0x7fffffffu) >> 20;
+                em = er > em ? er : em;
+                em = el > em ? el : em;
             };
-            if (c0 >= lo - 2 && c0 + 1 < hi + 2) {
-                top(gr.x);
-                top(gr.y);
-                top(gl0);
-                top(gl1);
-            }
+            top(c0, gr.x, gl0);
+            top(c0 + 1, gr.y, gl1);
             em = __reduce_max_sync(kFull, em);
         }
         const bool out_of_range = em > 1846u;

@@ -1,5 +1,6 @@
 """Inputs at the edges of what the float pairs of ``csrc/fixed_flux.cuh`` hold:
-smoothness parameters whose products leave float's range."""
+smoothness parameters whose products leave float's range, and cotangents of
+compact support."""
 
 from __future__ import annotations
 
@@ -8,6 +9,7 @@ import pytest
 import torch
 
 from oracle import numpy_ref as R
+from oracle import torch_ref as T
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +53,58 @@ def test_steps_for_any_smoothness_parameter(eps, amp, flux):
         for b, n in enumerate(sizes):
             err = np.max(np.abs(solver.instance(b).cpu().numpy() - refs[b])) / np.max(np.abs(u0[b]))
             assert err < 1.0e-13, (n, tile, err)
+
+
+def _vjp(u, p, dt, dx):
+    from pyshocks_gb300 import _lib as L
+
+    n = u.numel()
+    ud = torch.cat([u[-3:], u, u[:3]]).cuda()
+    pd = torch.cat([p[-3:], p, p[:3]]).cuda()
+    out = torch.empty_like(ud)
+    st = L.lib().shk_ssprk33_vjp_f64(_scheme("rusanov", 1e-6).c_scheme(dx), ud.data_ptr(), pd.data_ptr(),
+                                     out.data_ptr(), n, 3, dx, dt, L.stream_handle())
+    assert st == 0, L.errstr(st)
+    return out.cpu()[3:-3]
+
+
+def _local_error(got, ref, floor):
+    """Largest error against the largest of an entry and its neighbours, over the
+    entries whose surroundings are at least *floor* of the largest."""
+    a = ref.abs()
+    size = torch.stack([a.roll(-1), a, a.roll(1)]).amax(0)
+    m = size > floor * a.max()
+    return float(((got - ref).abs()[m] / size[m]).max())
+
+
+# Entry by entry: the reverse step and autograd differ by the operator's second
+# derivative (at most about 1e3 per unit) times a step's roundings of 1e-16, and
+# an entry's terms exceed it and its neighbours by at most some 1e3 (the
+# farthest taps, 2 / 60 of a face value, thrice): 1e-7 leaves three digits.
+LOCAL_BAR = 1.0e-7
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("n", [1025, 1100])
+def test_transposed_step_of_compact_cotangents(n, flat):
+    """Cotangents that end (or begin) at every cell around the edge of a 512-cell
+    tile and of a warp's 58 cells, on a smooth state or one whose left part is
+    constant."""
+    x = (torch.arange(n, dtype=torch.float64) + 0.5) / n
+    u = 0.8 + 0.3 * torch.sin(40 * np.pi * x) + 0.1 * torch.cos(22 * np.pi * x)
+    if flat:
+        u[200:480] = 0.7
+    dx = 2.0 / n
+    dt = 0.4 * dx / float(u.abs().max())
+    rng = np.random.default_rng(3)
+    p0 = torch.tensor(rng.uniform(0.5, 1.0, n))
+    for edge in list(range(484, 540)) + list(range(40, 76)):
+        for side in (0, 1):
+            p = p0.clone()
+            if side:
+                p[:edge] = 0.0
+            else:
+                p[edge:] = 0.0
+            ref = T.step_vjp(u[None], p[None], dt, dx)[0]
+            err = _local_error(_vjp(u, p, dt, dx), ref, 1.0e-30)
+            assert err < LOCAL_BAR, (edge, side, err)
