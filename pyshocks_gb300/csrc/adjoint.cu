@@ -183,15 +183,21 @@ __device__ void vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<T>& a,
 // are listed and take the FP64 backward, less the linear part. In units of
 // g / 60: GR, GL, GA hold the flux seeds of the faces; a.H takes the pair part of
 // z, a.D the list, a.Q the flags of the listed cells, T0..T4 their taps.
+// The pairs hold the seeds relative to the warp's largest. Where a warp's cells span
+// more than kPairRange powers of two (then the lower halves of the smallest near
+// float's smallest number, 2^-149) or leave 2^+-823, every cell of the window is listed:
+// warps share cells, so one warp alone cannot list its own.
 constexpr float kSmoothWeights = 0.125f;
+constexpr unsigned kPairRange = 80u;
 template <class PV, class PW, class PZ, class PC>
 __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<double>& a, const OpParams<double>& p,
                              double dtdx, PC UL, PC UR) {
     constexpr unsigned kFull = 0xffffffffu;
     const int tid = threadIdx.x, nt = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-    const Win<int> list = win_cast<int>(a.D), flag = win_cast<int>(a.Q);  // list[0]: count, from list[4]
-    if (tid == 0) list[0] = 0;
+    // list[0]: count, list[1]: list every cell, from list[4]: the cells
+    const Win<int> list = win_cast<int>(a.D), flag = win_cast<int>(a.Q);
+    if (tid == 0) list[0] = list[1] = 0;
     const double cf = dtdx * (1.0 / 120.0);
     for (int j = lo - 3 + tid; j < hi + 2; j += nt) {
         const double fb = (w[j + 1] - w[j]) * cf;
@@ -214,21 +220,21 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         // backward is linear in them). Every cell whose seeds are used counts, by
         // itself: [lo - 2, hi + 2) may begin or end inside a lane's pair, and beyond it
         // the seeds are not written
-        unsigned em = 0;
+        unsigned em, least;
         {
-            auto top = [&](int c, double r, double l) {
-                if (c < lo - 2 || c >= hi + 2) return;
-                const unsigned er = (static_cast<unsigned>(__double2hiint(r)) & 0x7fffffffu) >> 20;
-                const unsigned el = (static_cast<unsigned>(__double2hiint(l)) & 0x7fffffffu) >> 20;
-                em = er > em ? er : em;
-                em = el > em ? el : em;
+            auto top = [&](int c, double r, double l) -> unsigned {
+                const unsigned hr = static_cast<unsigned>(__double2hiint(r)) & 0x7fffffffu;
+                const unsigned hl = static_cast<unsigned>(__double2hiint(l)) & 0x7fffffffu;
+                const bool used = static_cast<unsigned>(c - (lo - 2)) < static_cast<unsigned>(hi - lo + 4);
+                return used ? (hr > hl ? hr : hl) : 0u;
             };
-            top(c0, gr.x, gl0);
-            top(c0 + 1, gr.y, gl1);
-            em = __reduce_max_sync(kFull, em);
+            const unsigned h0 = top(c0, gr.x, gl0), h1 = top(c0 + 1, gr.y, gl1);
+            em = __reduce_max_sync(kFull, h0 > h1 ? h0 : h1) >> 20;
+            // (zeros do not count)
+            least = __reduce_min_sync(kFull, h0 - 1u < h1 - 1u ? h0 - 1u : h1 - 1u) >> 20;
         }
-        const bool out_of_range = em > 1846u;
-        em = em < 200u ? 200u : (out_of_range ? 1846u : em);
+        if (lane == 0 && (em > 1846u || least < 200u || least + kPairRange < em)) list[1] = 1;
+        em = em < 200u ? 200u : em;
         fx::CellGrad g;
         {
             fx::Cell x, y;
@@ -255,8 +261,8 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
                               gL);
         }
         // listed cells: nothing here
-        const bool b0 = !(fx::p2x(g.x) <= kSmoothWeights) || out_of_range;
-        const bool b1 = !(fx::p2y(g.x) <= kSmoothWeights) || out_of_range;
+        const bool b0 = !(fx::p2x(g.x) <= kSmoothWeights);
+        const bool b1 = !(fx::p2y(g.x) <= kSmoothWeights);
         auto keep = [&](fx::P2 q) { return fx::p2(b0 ? 0.0f : fx::p2x(q), b1 ? 0.0f : fx::p2y(q)); };
         auto keep2 = [&](fx::FF q) { return fx::FF{keep(q.h), keep(q.l)}; };
         const fx::FF tm = keep2(g.tm), t0 = keep2(g.t0), sg = keep2(g.sg), et = keep2(g.et);
@@ -288,7 +294,16 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         }
     }
     __syncthreads();
-    const int cnt = list[0];
+    int cnt = list[0];
+    if (list[1] != 0) {
+        cnt = hi - lo + 4;
+        for (int c = lo - 2 + tid; c < hi + 2; c += nt) {
+            list[4 + c - (lo - 2)] = c;
+            flag[c] = 1;
+            if (c >= lo && c < hi) a.H[c] = 0.0;
+        }
+        __syncthreads();
+    }
     for (int q = tid; q < cnt; q += nt) {
         const int c = list[4 + q];
         const double Hm2 = 0.5 * (v[c - 1] - v[c - 2]), Hm1 = 0.5 * (v[c] - v[c - 1]);

@@ -1,6 +1,6 @@
 """Inputs at the edges of what the float pairs of ``csrc/fixed_flux.cuh`` hold:
-smoothness parameters whose products leave float's range, and cotangents of
-compact support."""
+smoothness parameters whose products leave float's range, cotangents of compact
+support, and cotangents whose magnitudes cross the range of a warp's scale."""
 
 from __future__ import annotations
 
@@ -108,3 +108,22 @@ def test_transposed_step_of_compact_cotangents(n, flat):
             ref = T.step_vjp(u[None], p[None], dt, dx)[0]
             err = _local_error(_vjp(u, p, dt, dx), ref, 1.0e-30)
             assert err < LOCAL_BAR, (edge, side, err)
+
+
+@pytest.mark.parametrize(("lo", "hi"), [(-290, -285), (-292, -276), (240, 255), (246, 250), (-260, 260)])
+def test_transposed_step_of_cotangents_across_the_scales(lo, hi):
+    """Cotangents rising from 10^lo to 10^hi over the cells: inside a few warps
+    they pass the magnitudes that the pairs of floats are scaled for."""
+    n = 400
+    x = (torch.arange(n, dtype=torch.float64) + 0.5) / n
+    u = 0.8 + 0.3 * torch.sin(16 * np.pi * x) + 0.1 * torch.cos(10 * np.pi * x)
+    dx = 2.0 / n
+    dt = 0.4 * dx / float(u.abs().max())
+    rng = np.random.default_rng(4)
+    p = torch.tensor(rng.uniform(0.5, 1.0, n) * 10.0 ** np.linspace(lo, hi, n))
+    ref = T.step_vjp(u[None], p[None], dt, dx)[0]
+    inner = slice(20, n - 20)  # (away from the jump of the periodic continuation)
+    got = _vjp(u, p, dt, dx)
+    a = ref.abs()
+    size = torch.stack([a.roll(-1), a, a.roll(1)]).amax(0)
+    assert float(((got - ref).abs() / size)[inner].max()) < LOCAL_BAR
