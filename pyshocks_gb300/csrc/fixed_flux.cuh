@@ -492,12 +492,13 @@ SHK_FX double face_flux_lf(const Cell& c, int64_t Z, int64_t D, const Speed& sp)
     return to_double(((square_hi(Z) + square_hi(D)) >> sh) + product_hi(D, sp.M), c.k + static_cast<int>(d));
 }
 
-// 288 F from face values R, L formed in double (v0, v1: the face's cells, a: the
-// speed if it is the larger), with the integer arithmetic of the other faces:
-// next to a constant state, where R = L = v, the flux equals theirs and the
-// difference vanishes exactly. False where the integers do not hold it.
-SHK_FX bool listed_flux(double R, double L, double v0, double v1, double aglob, double& G) {
-    const Mag r = mag(R), l = mag(L), a = mag(v0), b = mag(v1), g = mag(aglob);
+// 288 F from six times the corrections tR = 6 (R - v0), tL = 6 (L - v1) of the face values
+// formed in double (v0, v1: the face's cells, a: the speed if it is the larger), with
+// the integer arithmetic of the other faces: next to a constant state, where R = L =
+// v, the flux equals theirs and the difference vanishes exactly. False where the
+// integers do not hold it.
+SHK_FX bool listed_flux(double tR, double tL, double v0, double v1, double aglob, double& G) {
+    const Mag r = mag(tR), l = mag(tL), a = mag(v0), b = mag(v1), g = mag(aglob);
     uint32_t exm = r.e > l.e ? r.e : l.e;
     exm = exm > a.e ? exm : a.e;
     exm = exm > b.e ? exm : b.e;
@@ -508,9 +509,10 @@ SHK_FX bool listed_flux(double R, double L, double v0, double v1, double aglob, 
     const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm), A2 = fix_abs(g, exm);
     uint64_t A = A0 > A1 ? A0 : A1;
     A = A > A2 ? A : A2;
-    const int64_t D = 6 * (x - y), Q = D + static_cast<int64_t>(24u * A);
+    const int64_t V0 = with_sign(A0, a), V1 = with_sign(A1, b);
+    const int64_t D = 6 * (V0 - V1) + (x - y), Q = D + static_cast<int64_t>(24u * A);
     if (Q < 0) return false;
-    G = face_flux(2 * static_cast<int>(exm) - 2094, 6 * (x + y), D, Q);
+    G = face_flux(2 * static_cast<int>(exm) - 2094, 6 * (V0 + V1) + (x + y), D, Q);
     return true;
 }
 

@@ -766,24 +766,58 @@ __device__ unsigned int step_tile_f32_weno(const Smem<float>& sm, Win<float> gou
 // double state, Burgers + Rusanov (nu = 1) + WENO-JS5: the stages on the fluxes
 // of fixed_flux.cuh
 // ---------------------------------------------------------------------------
-// face value at the right of the middle cell of v (WENO-JS5 in product form, the
-// middle sub-stencil's value plus weighted third differences)
-__device__ __forceinline__ double weno53_side_d(double vm2, double vm1, double v, double vp1, double vp2,
-                                                double eps4) {
-    const double dm2 = vm1 - vm2, dm1 = v - vm1, d0 = vp1 - v, dp1 = vp2 - vp1;
-    const double Em = dm1 - dm2, E0 = d0 - dm1, Ep = dp1 - d0;
-    const double h0 = fma(2.0, dm1, Em), h1 = d0 + dm1, h2 = fma(-2.0, d0, Ep);
-    double s0 = fma(h0, h0, fma((13.0 / 3.0) * Em, Em, eps4)); s0 = s0 * s0;
-    double s1 = fma(h1, h1, fma((13.0 / 3.0) * E0, E0, eps4)); s1 = s1 * s1;
-    double s2 = fma(h2, h2, fma((13.0 / 3.0) * Ep, Ep, eps4)); s2 = s2 * s2;
-    const double P0 = s1 * s2, P1 = s0 * s2, P2 = s0 * s1;
-    const double cr0 = fma(2.0, h0, -dm1), cr1 = fma(12.0, d0, 6.0 * dm1), cr2 = 3.0 * (d0 - h2);
-    const double nr = fma(P0, cr0, fma(P1, cr1, P2 * cr2));
-    const double dr = fma(6.0, P0, fma(18.0, P2, 36.0 * P1));
-    return fma(nr, rcp_nr(dr), v);
+// The faces that fixed_flux.cuh leaves, in FP64: six times the corrections that
+// WENO-JS5 adds to the middle cell for its two face values, tR = 6 (ur - v) and
+// tL = 6 (ul - v), as the middle sub-stencil's plus weighted third differences (product
+// form, P_k = 1 / (4 (eps + beta_k))^2 up to a common factor). From the differences a, b
+// on the left and right, E and G = 13/3 E^2 + 4 eps of the cell and of those beside.
+// The mirrored input gives the mirrored values bit for bit.
+struct WenoTerms {
+    double P0, P1, P2, A, B, S;
+};
+__device__ __forceinline__ WenoTerms weno53_terms(double a, double b, double Em, double E, double Ep, double Gm,
+                                                  double G, double Gp) {
+    const double h0 = fma(2.0, a, Em), h1 = b + a, h2 = fma(-2.0, b, Ep);
+    const double e0 = fma(h0, h0, Gm), e1 = fma(h1, h1, G), e2 = fma(h2, h2, Gp);
+    const double p0 = e1 * e2, p1 = e0 * e2, p2 = e0 * e1;
+    WenoTerms w;
+    w.P0 = p0 * p0;
+    w.P1 = p1 * p1;
+    w.P2 = p2 * p2;
+    w.A = w.P0 * (E - Em);
+    w.B = w.P2 * (Ep - E);
+    w.S = __dadd_rn(w.A, w.B);  // (not contracted: that would not mirror)
+    return w;
+}
+__device__ __forceinline__ double weno53_right(const WenoTerms& w, double a, double b) {
+    return fma(-fma(2.0, w.S, w.B), rcp_nr(fma(6.0, w.P1, fma(3.0, w.P2, w.P0))), fma(2.0, b, a));
+}
+__device__ __forceinline__ double weno53_left(const WenoTerms& w, double a, double b) {
+    return fma(fma(2.0, w.S, w.A), rcp_nr(fma(6.0, w.P1, fma(3.0, w.P0, w.P2))), -fma(2.0, a, b));
+}
+__device__ __forceinline__ double weno53_g(double E, double eps4) { return fma((13.0 / 3.0) * E, E, eps4); }
+
+// the flux of such a face from its two corrections
+template <class PV, class FaceOut>
+__device__ __forceinline__ void fx_listed_flux(PV v, Win<double> G, int j, double tR, double tL, double aglob,
+                                               const FaceOut& out) {
+    const double v0 = v[j], v1 = v[j + 1];
+    double g;
+    const bool ok = fx::listed_flux(tR, tL, v0, v1, aglob, g);
+    if (!ok || out.ul) {
+        const double R = fma(tR, 1.0 / 6.0, v0), L = fma(tL, 1.0 / 6.0, v1);
+        if (!ok) {
+            auto ab = abs_bits(v0) > abs_bits(v1) ? abs_bits(v0) : abs_bits(v1);
+            ab = ab > abs_bits(aglob) ? ab : abs_bits(aglob);
+            g = 72.0 * fma(L, L, fma(R, R, twice_abs_bits(ab) * (R - L)));
+        }
+        if (out.ul) out(j, R, L);
+    }
+    G[j] = g;
 }
 
-// what the listed faces need; two lanes per face, one for each side's value
+// few among a warp's faces: shared out over the CTA after a barrier, two lanes per
+// face, one for each side (38 FP64 instructions for 16 faces)
 template <class PV, class FaceOut>
 __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list, int cnt, double eps,
                                              double aglob, FaceOut out) {
@@ -793,20 +827,52 @@ __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list,
         const int q = q0 + (lane >> 1);
         const int j = list[q < cnt ? q : q0];
         const int c = j + (lane & 1), o = (lane & 1) ? -1 : 1;  // cell and direction of this side
-        const double w = weno53_side_d(v[c - 2 * o], v[c - o], v[c], v[c + o], v[c + 2 * o], eps4);
-        const double w1 = __shfl_xor_sync(0xffffffffu, w, 1);
-        const double R = (lane & 1) ? w1 : w, L = (lane & 1) ? w : w1;
-        if (q < cnt && (lane & 1) == 0) {
-            double g;
-            if (!fx::listed_flux(R, L, v[j], v[j + 1], aglob, g)) {
-                auto ab = abs_bits(v[j]) > abs_bits(v[j + 1]) ? abs_bits(v[j]) : abs_bits(v[j + 1]);
-                ab = ab > abs_bits(aglob) ? ab : abs_bits(aglob);
-                g = 72.0 * fma(L, L, fma(R, R, twice_abs_bits(ab) * (R - L)));
-            }
-            G[j] = g;
-            if (out.ul) out(j, R, L);
-        }
+        const double x = v[c], vm = v[c - o], vp = v[c + o];
+        const double dm2 = vm - v[c - 2 * o], dm1 = x - vm, d0 = vp - x, dp1 = v[c + 2 * o] - vp;
+        const double Em = dm1 - dm2, E0 = d0 - dm1, Ep = dp1 - d0;
+        const WenoTerms w = weno53_terms(dm1, d0, Em, E0, Ep, weno53_g(Em, eps4), weno53_g(E0, eps4),
+                                         weno53_g(Ep, eps4));
+        const double t = weno53_right(w, dm1, d0), t1 = __shfl_xor_sync(0xffffffffu, t, 1);
+        if (q < cnt && (lane & 1) == 0) fx_listed_flux(v, G, j, t, t1, aglob, out);
     }
+}
+
+// many: at once by that warp, both sides of every cell, two cells per lane (74 FP64
+// instructions for 60 faces), the neighbours' differences by shuffle. The same operations
+// on the same values give a side's correction, so it does not depend on how many
+// others are left. l0, l1: this lane's faces c0 = r0 + 2 lane and c0 + 1
+template <class PV, class FaceOut>
+__device__ __noinline__ void fx_listed_chunk(PV v, Win<double> G, int r0, int W, bool l0, bool l1, double eps,
+                                             double aglob, FaceOut out) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int c0 = r0 + 2 * (threadIdx.x & 31);
+    const double eps4 = 4.0 * eps;
+    // (cells outside the window only feed faces that are not stored)
+    const int ca = c0 < 0 ? 0 : (c0 < W - 2 ? c0 : W - 2);
+    const double vm = v[ca > 0 ? ca - 1 : 0], v0 = v[ca], v1 = v[ca + 1], v2 = v[ca < W - 2 ? ca + 2 : ca + 1];
+    const double dm = v0 - vm, d0 = v1 - v0, d1 = v2 - v1;
+    const double E0 = d0 - dm, E1 = d1 - d0;
+    const double G0 = weno53_g(E0, eps4), G1 = weno53_g(E1, eps4);
+    const double Em = __shfl_up_sync(kFull, E1, 1), Gm = __shfl_up_sync(kFull, G1, 1);
+    const double Ep = __shfl_down_sync(kFull, E0, 1), Gp = __shfl_down_sync(kFull, G0, 1);
+    const WenoTerms a = weno53_terms(dm, d0, Em, E0, E1, Gm, G0, G1);
+    const WenoTerms b = weno53_terms(d0, d1, E0, E1, Ep, G0, G1, Gp);
+    const double L2 = __shfl_down_sync(kFull, weno53_left(a, dm, d0), 1);
+    const double R0 = weno53_right(a, dm, d0), L1 = weno53_left(b, d0, d1), R1 = weno53_right(b, d0, d1);
+    if (l0) fx_listed_flux(v, G, c0, R0, L1, aglob, out);
+    if (l1) fx_listed_flux(v, G, c0 + 1, R1, L2, aglob, out);
+}
+// Whether a warp's faces that are left make a chunk. An FP64 instruction holds a quarter
+// of an SM for 64 clocks: short windows, whose chunks would leave quarters idle, spread
+// their faces by the list (up to 90 faces always, up to 180 unless nearly all of a chunk
+// are left). Measured (us per step: FP64 formula for every face / all left faces in the
+// list with two one-sided evaluations each / this), 1024 instances, 6.4 M cells: 0.5 %
+// noise 1948 / 2794 / 1597, random cells 1948 / 3016 / 1598, smooth 1948 / 285 / 286; 24
+// instances of 100 to 1000 cells: noise 57 / 40 / 34, random 57 / 78 / 48; 1000 random
+// instances of 128 cells: 71 / 81 / 50, of 64 cells: 57 / 47 / 47.
+__device__ __forceinline__ bool fx_many(int faces, bool l0, bool l1) {
+    const int left = __popc(__ballot_sync(0xffffffffu, l0)) + __popc(__ballot_sync(0xffffffffu, l1));
+    return left > 32 && (faces > 180 || (faces > 90 && left > 50));
 }
 
 // face values of the cells [lo, hi) of a window to ul, ur (indexed from the
@@ -858,26 +924,33 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
                                           fx::p2(s.x.iu, s.y.iu));
         const bool inner = lane >= 1 && lane <= 30;
         const bool m0 = inner && c0 >= jlo && c0 < jhi, m1 = inner && c0 + 1 >= jlo && c0 + 1 < jhi;
-        // (the flux of a face left to the list is overwritten after the barrier)
+        // (the flux of a face that is left is overwritten)
         auto face = [&](int j, const fx::Cell& c, bool mine, float xR, float xL, float tR, float tL, float rs,
-                        float rd) -> double {
+                        float rd, bool& left) -> double {
             int64_t Z, D, Q;
             const bool ok = fx::face_sums(c, xR, xL, tR, tL, rs, rd, Z, D, Q) && speed.in;
-            if (mine) {
-                if (!ok) list[atomicAdd(&sm.fx[slot], 1)] = j;
-                else if (out.ul)
-                    out(j, fx::to_double(Z + D, c.kz) * (1.0 / 12.0), fx::to_double(Z - D, c.kz) * (1.0 / 12.0));
-            }
+            left = mine && !ok;
+            if (out.ul && mine && ok)
+                out(j, fx::to_double(Z + D, c.kz) * (1.0 / 12.0), fx::to_double(Z - D, c.kz) * (1.0 / 12.0));
             if constexpr (LF) return fx::face_flux_lf(c, Z, D, speed);
             else return fx::face_flux(c.k, Z, D, Q);
         };
+        bool l0, l1;
         const double f0 = face(c0, s.x, m0, fx::p2x(u.xR), fx::p2x(u.xL), fx::p2x(u.tR), fx::p2x(u.tL),
-                               fx::p2x(u.rs), fx::p2x(u.rd));
+                               fx::p2x(u.rs), fx::p2x(u.rd), l0);
         const double f1 = face(c0 + 1, s.y, m1, fx::p2y(u.xR), fx::p2y(u.xL), fx::p2y(u.tR), fx::p2y(u.tL),
-                               fx::p2y(u.rs), fx::p2y(u.rd));
+                               fx::p2y(u.rs), fx::p2y(u.rd), l1);
         if (m0 && m1) *reinterpret_cast<double2*>(win_span(sm.D, c0, 2)) = make_double2(f0, f1);
         else if (m0) sm.D[c0] = f0;
         else if (m1) sm.D[c0 + 1] = f1;
+        if (__any_sync(kFull, l0 || l1)) {
+            if (fx_many(jhi - jlo, l0, l1)) {
+                fx_listed_chunk(v, sm.D, r0, sm.W, l0, l1, p.eps, aglob, out);
+            } else {
+                if (l0) list[atomicAdd(&sm.fx[slot], 1)] = c0;
+                if (l1) list[atomicAdd(&sm.fx[slot], 1)] = c0 + 1;
+            }
+        }
     }
     __syncthreads();
     const int cnt = sm.fx[slot];

@@ -1,0 +1,71 @@
+"""Faces that the integer / float-pair forms leave to FP64 (``csrc/stencil.cuh``
+``fx_listed_faces``, ``fx_listed_chunk``): states of noise, of runs of it, and random
+ones, at the window lengths where the list, the chunks of 60 faces and their
+threshold change."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import numpy_ref as R
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [5, 31, 46, 47, 75, 76, 77, 78, 106, 107, 165, 166, 167, 168, 226, 400, 1000]
+KINDS = ["noise", "runs", "random", "zeros"]
+
+
+def _state(kind, n, rng):
+    x = (np.arange(n) + 0.5) / n
+    u = 0.3 + np.sin(2 * np.pi * x) + 0.1 * np.cos(6 * np.pi * x)
+    if kind == "noise":
+        return u + 0.005 * rng.standard_normal(n)
+    if kind == "random":
+        return rng.uniform(-1.0, 1.0, n)
+    if kind == "zeros":  # random stretches between exact zeros
+        return np.where((np.arange(n) // 29) % 2 == 0, rng.uniform(-1.0, 1.0, n), 0.0)
+    mask = np.zeros(n, dtype=bool)  # runs of 1 to 70 noisy cells
+    i = 0
+    while i < n:
+        run = int(rng.integers(1, 71))
+        mask[i : i + run] = True
+        i += run + int(rng.integers(1, 60))
+    return u + np.where(mask, 0.05 * rng.standard_normal(n), 0.0)
+
+
+def _scheme(flux):
+    import pyshocks_gb300 as gb
+    from pyshocks_gb300 import burgers
+
+    return burgers.make_scheme_from_name(flux, rec=gb.reconstruction.make_reconstruction_from_name("wenojs53", eps=1.0e-6))
+
+
+@pytest.mark.parametrize("flux", ["rusanov", "lf"])
+@pytest.mark.parametrize("kind", KINDS)
+def test_steps_match_oracle_and_do_not_depend_on_the_tile(kind, flux):
+    """Three steps: 1e-13 of the largest value (about 900 roundings) from the
+    oracle; bit for bit the same in every tile, resident or launched, however the
+    faces were shared out."""
+    from pyshocks_gb300.batched import BatchedSolver
+
+    nsteps = 3
+    rng = np.random.default_rng(17)
+    u0 = [_state(kind, n, rng) for n in SIZES]
+    out = []
+    for tile in (0, 16, 60, 90, 180, 226, 466, 1024):
+        s = BatchedSolver(_scheme(flux), SIZES, [2.0 / n for n in SIZES], theta=0.9, tile=tile)
+        s.reset(torch.tensor(np.concatenate(u0)))
+        s.step(nsteps)
+        assert s.status() == 0
+        out.append((s.u.clone(), s))
+    for u, _ in out[1:]:
+        assert torch.equal(u, out[0][0])
+    for b, n in enumerate(SIZES):
+        og = R.make_uniform_cell_grid(-1.0, 1.0, n, 3)
+        ug = np.zeros(n + 6)
+        ug[3:-3] = u0[b]
+        ref, _ = R.evolve(R.SchemeSpec(flux_kind=flux), og, ug, theta=0.9, maxit=nsteps)
+        err = np.max(np.abs(out[0][1].instance(b).cpu().numpy() - ref[3:-3])) / np.max(np.abs(u0[b]))
+        assert err < 1.0e-13, (n, err)
