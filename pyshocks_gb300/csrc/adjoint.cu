@@ -174,19 +174,67 @@ __device__ void vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<T>& a,
     __syncthreads();
 }
 
+// The FP64 backward of a cell's two face values for the listed cells of fx_vjp_stage
+// (113 operations; weno53_cell_vjp with its inputs 147): the taps t_o of v_{c+o},
+// o = -2..2, for gR, gL = 1/6 of the cotangents of the right and left face value. On
+// c_k = 6 (sub-stencil value - v), their weights rho_k, lam_k times the seed and the
+// sums e_k = 4 (eps + beta_k), e = h^2 + 13/3 E^2 + 4 eps: a weight's part is
+// -2 rho_k (c_k - mean) / e_k in e_k. The taps sum to 6 (gR + gL).
+template <class PV>
+__device__ __forceinline__ void weno53_listed_vjp(PV v, int c, double eps4, double gR, double gL, double& t0,
+                                                  double& t1, double& t2, double& t3, double& t4) {
+    const double vm = v[c - 1], x = v[c], vp = v[c + 1];
+    const double dm = vm - v[c - 2], a = x - vm, b = vp - x, dp = v[c + 2] - vp;
+    const double Em = a - dm, E = b - a, Ep = dp - b;
+    const double h0 = fma(2.0, a, Em), h1 = b + a, h2 = fma(-2.0, b, Ep);
+    const double f0 = (13.0 / 3.0) * Em, f1 = (13.0 / 3.0) * E, f2 = (13.0 / 3.0) * Ep;
+    const double e0 = fma(h0, h0, fma(f0, Em, eps4));
+    const double e1 = fma(h1, h1, fma(f1, E, eps4));
+    const double e2 = fma(h2, h2, fma(f2, Ep, eps4));
+    const double e12 = e1 * e2, e02 = e0 * e2, e01 = e0 * e1;
+    const double P0 = e12 * e12, P1 = 6.0 * (e02 * e02), P2 = e01 * e01, Q0 = 3.0 * P0, Q2 = 3.0 * P2;
+    const double c0 = fma(2.0, h0, -a), c1 = fma(2.0, b, a), c2 = b - h2;
+    const double l0 = fma(2.0, h2, b), l1 = -fma(2.0, a, b), l2 = -(h0 + a);
+    const double iR = rcp_nr(P0 + P1 + Q2), iL = rcp_nr(P2 + P1 + Q0);
+    const double cR = fma(P0, c0, fma(P1, c1, Q2 * c2)) * iR, cL = fma(P2, l0, fma(P1, l1, Q0 * l2)) * iL;
+    const double gsum = gR + gL;
+    gR *= iR;
+    gL *= iL;
+    const double rho0 = gR * P0, rho1 = gR * P1, rho2 = gR * Q2;
+    const double lam0 = gL * P2, lam1 = gL * P1, lam2 = gL * Q0;
+    const double q = rcp_nr(e01 * e2);
+    const double k0 = fma(rho0, c0 - cR, lam2 * (l2 - cL)) * (e12 * q);
+    const double k1 = fma(rho1, c1 - cR, lam1 * (l1 - cL)) * (e02 * q);
+    const double k2 = fma(rho2, c2 - cR, lam0 * (l0 - cL)) * (e01 * q);
+    const double kh0 = k0 * h0, kh1 = k1 * h1, kh2 = k2 * h2, kE0 = k0 * f0, kE1 = k1 * f1, kE2 = k2 * f2;
+    // h_0 (1, -4, 3, 0, 0), h_1 (0, -1, 0, 1, 0), h_2 (0, 0, 3, -4, 1), E_k (1, -2, 1);
+    // c_0 (2, -7, 5, 0, 0), c_1 (0, -1, -1, 2, 0), c_2 (0, 0, -4, 5, -1), l_k mirrored
+    t0 = fma(-4.0, kh0 + kE0, fma(2.0, rho0, -lam2));
+    t1 = fma(-4.0, fma(-4.0, kh0, fma(-2.0, kE0, kE1 - kh1)),
+             fma(5.0, lam2, fma(2.0, lam1, fma(-7.0, rho0, -rho1))));
+    t3 = fma(-4.0, fma(-4.0, kh2, fma(-2.0, kE2, kE1 + kh1)),
+             fma(5.0, rho2, fma(2.0, rho1, fma(-7.0, lam0, -lam1))));
+    t4 = fma(-4.0, kh2 + kE2, fma(2.0, lam0, -rho2));
+    t2 = fma(6.0, gsum, -((t0 + t1) + (t3 + t4)));
+}
+
 // vjp_stage for the schemes of fixed_flux_scheme. The FP64 pipe bounded the
 // reverse step at 159 operations per cell and stage, most of them in the
 // reconstruction's backward. Its linear (ideal-weight) part, the flux seeds and
 // the sums stay in FP64 (25 operations); the rest, small where the state is
 // smooth, is formed in pairs of floats two cells per lane (lane_grad). Cells
 // with a weight change |x0| + |x2| above 1/8 or a third difference out of range
-// are listed and take the FP64 backward, less the linear part. In units of
+// are listed and take the FP64 backward, without the linear part. In units of
 // g / 60: GR, GL, GA hold the flux seeds of the faces; a.H takes the pair part of
 // z, a.D the list, a.Q the flags of the listed cells, T0..T4 their taps.
 // The pairs hold the seeds relative to the warp's largest. Where a warp's cells span
 // more than kPairRange powers of two (then the lower halves of the smallest near
 // float's smallest number, 2^-149) or leave 2^+-823, every cell of the window is listed:
 // warps share cells, so one warp alone cannot list its own.
+// A warp whose cells are all listed skips its pairs. Reverse sweep of ten steps, 96
+// instances (0.4 M cells), us (FP64 backward everywhere / the pairs in vain and the linear
+// part twice / this): 0.5 % noise 5327 / 6680 / 4725, random 5326 / 7032 / 4741, smooth 5324 /
+// 1444 / 1456.
 constexpr float kSmoothWeights = 0.125f;
 constexpr unsigned kPairRange = 80u;
 template <class PV, class PW, class PZ, class PC>
@@ -236,6 +284,7 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         if (lane == 0 && (em > 1846u || least < 200u || least + kPairRange < em)) list[1] = 1;
         em = em < 200u ? 200u : em;
         fx::CellGrad g;
+        bool b0, b1;
         {
             fx::Cell x, y;
             {
@@ -250,6 +299,29 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
             T0.h = fx::p2(x.ok ? fx::p2x(T0.h) : nan, y.ok ? fx::p2y(T0.h) : nan);
             const float Tmh = __shfl_up_sync(kFull, fx::p2y(T0.h), 1), Tml = __shfl_up_sync(kFull, fx::p2y(T0.l), 1);
             const fx::FF Tm{fx::p2(Tmh, fx::p2x(T0.h)), fx::p2(Tml, fx::p2x(T0.l))};
+            const fx::FF S = fx::to_ff(x.S, y.S, u36, u12, u0), E = fx::to_ff(x.E, y.E, u36, u12, u0);
+            const fx::CellWeights cw = fx::lane_weights(S, E, Tm, T0, eps4);
+            // listed cells: nothing here
+            b0 = !(fx::p2x(cw.x) <= kSmoothWeights);
+            b1 = !(fx::p2y(cw.x) <= kSmoothWeights);
+            auto mark = [&](int q, int c, bool bad) {
+                const bool mine = (q >= 4 && q < 62) || (r0 == first && q >= 2 && q < 4) || (r0 + 62 >= hi && q >= 62);
+                if (mine && c >= lo - 2 && c < hi + 2) {
+                    flag[c] = bad ? 1 : 0;
+                    if (bad) list[4 + atomicAdd(&list[0], 1)] = c;
+                }
+            };
+            mark(2 * lane, c0, b0);
+            mark(2 * lane + 1, c0 + 1, b1);
+            // (noise: all of them)
+            const bool out0 = c0 < lo - 2 || c0 >= hi + 2, out1 = c0 + 1 < lo - 2 || c0 + 1 >= hi + 2;
+            if (__all_sync(kFull, lane == 0 || ((b0 || out0) && (b1 || out1)))) {
+                if (lane >= 2 && lane <= 30) {
+                    if (c0 >= lo && c0 < hi) a.H[c0] = 0.0;
+                    if (c0 + 1 >= lo && c0 + 1 < hi) a.H[c0 + 1] = 0.0;
+                }
+                continue;
+            }
             float h0, l0, h1, l1;
             fx::split_double(gr.x, em, h0, l0);
             fx::split_double(gr.y, em, h1, l1);
@@ -257,24 +329,11 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
             fx::split_double(gl0, em, h0, l0);
             fx::split_double(gl1, em, h1, l1);
             const fx::FF gL{fx::p2(h0, h1), fx::p2(l0, l1)};
-            g = fx::lane_grad(fx::to_ff(x.S, y.S, u36, u12, u0), fx::to_ff(x.E, y.E, u36, u12, u0), Tm, T0, eps4, gR,
-                              gL);
+            g = fx::lane_grad(cw, S, E, Tm, T0, gR, gL);
         }
-        // listed cells: nothing here
-        const bool b0 = !(fx::p2x(g.x) <= kSmoothWeights);
-        const bool b1 = !(fx::p2y(g.x) <= kSmoothWeights);
         auto keep = [&](fx::P2 q) { return fx::p2(b0 ? 0.0f : fx::p2x(q), b1 ? 0.0f : fx::p2y(q)); };
         auto keep2 = [&](fx::FF q) { return fx::FF{keep(q.h), keep(q.l)}; };
         const fx::FF tm = keep2(g.tm), t0 = keep2(g.t0), sg = keep2(g.sg), et = keep2(g.et);
-        auto mark = [&](int q, int c, bool bad) {
-            const bool mine = (q >= 4 && q < 62) || (r0 == first && q >= 2 && q < 4) || (r0 + 62 >= hi && q >= 62);
-            if (mine && c >= lo - 2 && c < hi + 2) {
-                flag[c] = bad ? 1 : 0;
-                if (bad) list[4 + atomicAdd(&list[0], 1)] = c;
-            }
-        };
-        mark(2 * lane, c0, b0);
-        mark(2 * lane + 1, c0 + 1, b1);
         // transposes of T, E and S: the cotangent of T_c, of E_c, then z (neighbours'
         // values from the lanes beside)
         auto dn = [&](float q) { return __shfl_down_sync(kFull, q, 1); };
@@ -304,20 +363,18 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         }
         __syncthreads();
     }
+    // (the seeds of a listed cell are its own: they are taken out of the linear part below)
     for (int q = tid; q < cnt; q += nt) {
         const int c = list[4 + q];
-        const double Hm2 = 0.5 * (v[c - 1] - v[c - 2]), Hm1 = 0.5 * (v[c] - v[c - 1]);
-        const double H0 = 0.5 * (v[c + 1] - v[c]), Hp1 = 0.5 * (v[c + 2] - v[c + 1]);
-        const double Dm1 = Hm1 - Hm2, D0 = H0 - Hm1, Dp1 = Hp1 - H0;
-        const double R = a.GR[c], L = a.GL[c - 1];
         double t0, t1, t2, t3, t4;
-        weno53_cell_vjp<double>(Hm2, Hm1, H0, Hp1, Dm1, D0, Dp1, (13.0 / 3.0 * Dm1) * Dm1, (13.0 / 3.0 * D0) * D0,
-                                (13.0 / 3.0 * Dp1) * Dp1, p.eps, 60.0 * R, 60.0 * L, t0, t1, t2, t3, t4);
-        a.T0[c] = t0 - fma(2.0, R, -3.0 * L);
-        a.T1[c] = t1 - fma(-13.0, R, 27.0 * L);
-        a.T2[c] = t2 - 47.0 * (R + L);
-        a.T3[c] = t3 - fma(27.0, R, -13.0 * L);
-        a.T4[c] = t4 - fma(-3.0, R, 2.0 * L);
+        weno53_listed_vjp(v, c, 4.0 * p.eps, a.GR[c], a.GL[c - 1], t0, t1, t2, t3, t4);
+        a.T0[c] = t0;
+        a.T1[c] = t1;
+        a.T2[c] = t2;
+        a.T3[c] = t3;
+        a.T4[c] = t4;
+        a.GR[c] = 0.0;
+        a.GL[c - 1] = 0.0;
     }
     if (cnt > 0) __syncthreads();
     // the cotangent of max(x, y) that x takes, by the magnitudes' bits: all, half at
@@ -328,13 +385,28 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         return __hiloint2double(x > y ? h : (x == y ? half : 0), x >= y ? __double2loint(g) : 0);
     };
     for (int i = lo + tid; i < hi; i += nt) {
-        // ideal weights: taps (2, -13, 47, 27, -3) of the right face values, mirrored
-        // of the left ones
-        double s = fma(2.0, a.GR[i + 2] + a.GL[i - 3], 47.0 * (a.GR[i] + a.GL[i - 1]));
-        s = fma(-13.0, a.GR[i + 1] + a.GL[i - 2], s);
-        s = fma(27.0, a.GR[i - 1] + a.GL[i], s);
-        s = fma(-3.0, a.GR[i - 2] + a.GL[i + 1], s);
-        s = fma(10.0, a.H[i], s);
+        double s = 0.0;
+        bool all = cnt > 0;
+        if (cnt > 0) {
+            const bool f0 = flag[i - 2], f1 = flag[i - 1], f2 = flag[i], f3 = flag[i + 1], f4 = flag[i + 2];
+            all = f0 && f1 && f2 && f3 && f4;
+            double t = f4 ? a.T0[i + 2] : 0.0;
+            if (f3) t += a.T1[i + 1];
+            if (f2) t += a.T2[i];
+            if (f1) t += a.T3[i - 1];
+            if (f0) t += a.T4[i - 2];
+            s = 10.0 * t;
+        }
+        if (!all) {
+            // ideal weights: taps (2, -13, 47, 27, -3) of the right face values, mirrored
+            // of the left ones
+            s = fma(2.0, a.GR[i + 2] + a.GL[i - 3], s);
+            s = fma(47.0, a.GR[i] + a.GL[i - 1], s);
+            s = fma(-13.0, a.GR[i + 1] + a.GL[i - 2], s);
+            s = fma(27.0, a.GR[i - 1] + a.GL[i], s);
+            s = fma(-3.0, a.GR[i - 2] + a.GL[i + 1], s);
+            s = fma(10.0, a.H[i], s);
+        }
         // wave speed terms of the two faces, 60 GA d max(|v_i|, |v_i+-1|) / dv_i
         // (compared, halved and signed on the integer pipe)
         const double vi = v[i];
@@ -342,13 +414,6 @@ __device__ void fx_vjp_stage(PV v, PW w, PZ z, int lo, int hi, const AdjSmem<dou
         const double q = share(a.GA[i - 1], bi, bm) + share(a.GA[i], bi, bp);
         const int sgn60 = bi == 0 ? 0 : 0x404e0000 | (__double2hiint(vi) & static_cast<int>(0x80000000u));
         s = fma(__hiloint2double(sgn60, 0), q, s);
-        if (cnt > 0) {
-            if (flag[i + 2]) s += a.T0[i + 2];
-            if (flag[i + 1]) s += a.T1[i + 1];
-            if (flag[i]) s += a.T2[i];
-            if (flag[i - 1]) s += a.T3[i - 1];
-            if (flag[i - 2]) s += a.T4[i - 2];
-        }
         z[i] = s;
     }
     __syncthreads();

@@ -319,11 +319,15 @@ SHK_FX void lane_cells(const Lane& s, float amh, float aml, float gph, float gpl
 // e_1 - e_2 = T_c (2S - T_c - 13/3 (2E + T_c)), the remaining weights
 //   r0/D_R - 1/10 = 3 (3 x0 - x2) / 10 D_R,  r2/D_R - 1/10 = (7 x2 - x0) / 10 D_R
 // (and mirrored on the left) are small where the state is smooth, and every term
-// below carries one of them or a third difference. gR, gL: 1/6 of the cotangents
-// of the face values; `x`: |x0| + |x2|, the caller's measure of smooth.
+// below carries one of them or a third difference. lane_weights: the weights and `x` =
+// |x0| + |x2|, the caller's measure of smooth; lane_grad: the rest, gR, gL 1/6 of the
+// cotangents of the face values.
+struct CellWeights {
+    FF h0, h2, E0, E2, e0, e1, e2, x0, x2;
+    P2 x;
+};
 struct CellGrad {
     FF tm, t0, sg, et;
-    P2 x;
 };
 // a times a constant of few bits
 SHK_FX FF mul_const(FF a, float c) {
@@ -332,21 +336,29 @@ SHK_FX FF mul_const(FF a, float c) {
     return FF{p, fma2(a.l, C, fma2(a.h, C, neg(p)))};
 }
 SHK_FX P2 abs2(P2 a) { return p2(bitsf(fbits(p2x(a)) & 0x7fffffffu), bitsf(fbits(p2y(a)) & 0x7fffffffu)); }
-SHK_FX CellGrad lane_grad(FF S, FF E, FF Tm, FF T0, FF eps4, FF gR, FF gL) {
+SHK_FX CellWeights lane_weights(FF S, FF E, FF Tm, FF T0, FF eps4) {
     const FF c133{dup(4.33333349f), dup(-1.58945718e-07f)};  // 13/3
+    CellWeights w;
+    w.h0 = sub(S, Tm);
+    w.h2 = sub(S, T0);
+    w.E0 = sub(E, Tm);
+    w.E2 = add(E, T0);
+    w.e1 = add(add(sqr(S), mul(sqr(E), c133)), eps4);
+    w.e0 = add(add(sqr(w.h0), mul(sqr(w.E0), c133)), eps4);
+    w.e2 = add(add(sqr(w.h2), mul(sqr(w.E2), c133)), eps4);
+    const FF b0 = mul(Tm, add(add(S, w.h0), mul(add(E, w.E0), c133)));
+    const FF b2 = mul(T0, sub(add(S, w.h2), mul(add(E, w.E2), c133)));
+    w.x0 = mul(quot(b0, w.e0, 1.0f), quot(add(w.e1, w.e0), w.e0, 1.0f));
+    w.x2 = mul(quot(b2, w.e2, 1.0f), quot(add(w.e1, w.e2), w.e2, 1.0f));
+    w.x = abs2(w.x0.h) + abs2(w.x2.h);
+    return w;
+}
+SHK_FX CellGrad lane_grad(const CellWeights& w, FF S, FF E, FF Tm, FF T0, FF gR, FF gL) {
     const FF c263{dup(8.66666698f), dup(-3.17891436e-07f)};  // 26/3
     const FF c03{dup(0.300000012f), dup(-1.19209291e-08f)};  // 3/10
     const FF one{dup(1.0f), dup(0.0f)}, ten{dup(10.0f), dup(0.0f)};
+    const FF h0 = w.h0, h2 = w.h2, E0 = w.E0, E2 = w.E2, e0 = w.e0, e1 = w.e1, e2 = w.e2, x0 = w.x0, x2 = w.x2;
     CellGrad g;
-    const FF h0 = sub(S, Tm), h2 = sub(S, T0), E0 = sub(E, Tm), E2 = add(E, T0);
-    const FF e1 = add(add(sqr(S), mul(sqr(E), c133)), eps4);
-    const FF e0 = add(add(sqr(h0), mul(sqr(E0), c133)), eps4);
-    const FF e2 = add(add(sqr(h2), mul(sqr(E2), c133)), eps4);
-    const FF b0 = mul(Tm, add(add(S, h0), mul(add(E, E0), c133)));
-    const FF b2 = mul(T0, sub(add(S, h2), mul(add(E, E2), c133)));
-    const FF x0 = mul(quot(b0, e0, 1.0f), quot(add(e1, e0), e0, 1.0f));
-    const FF x2 = mul(quot(b2, e2, 1.0f), quot(add(e1, e2), e2, 1.0f));
-    g.x = abs2(x0.h) + abs2(x2.h);
     const FF X = add(ten, add(x0, x2));
     const FF DR = add(X, twice(x2)), DL = add(X, twice(x0));
     const FF r0 = add(one, x0), r2 = add(one, x2);

@@ -1,7 +1,7 @@
-"""Faces that the integer / float-pair forms leave to FP64 (``csrc/stencil.cuh``
-``fx_listed_faces``, ``fx_listed_chunk``): states of noise, of runs of it, and random
-ones, at the window lengths where the list, the chunks of 60 faces and their
-threshold change."""
+"""Faces and cells that the integer / float-pair forms leave to FP64 (``csrc/stencil.cuh``
+``fx_listed_faces``, ``fx_listed_chunk``, ``csrc/adjoint.cu`` ``weno53_listed_vjp``): states of noise, of runs of
+it, and random ones, at the window lengths where the list, the chunks of 60 faces and
+their threshold change."""
 
 from __future__ import annotations
 
@@ -10,6 +10,7 @@ import pytest
 import torch
 
 from oracle import numpy_ref as R
+from oracle import torch_ref as T
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +70,38 @@ def test_steps_match_oracle_and_do_not_depend_on_the_tile(kind, flux):
         ref, _ = R.evolve(R.SchemeSpec(flux_kind=flux), og, ug, theta=0.9, maxit=nsteps)
         err = np.max(np.abs(out[0][1].instance(b).cpu().numpy() - ref[3:-3])) / np.max(np.abs(u0[b]))
         assert err < 1.0e-13, (n, err)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_gradient_does_not_depend_on_the_tile(kind):
+    """Checkpointed gradients through stored stages, bit for bit, and against
+    autograd: 1e-11 of the largest entry per step (as the transposed step), four
+    steps."""
+    from pyshocks_gb300.adjoint import CheckpointedSolve
+    from pyshocks_gb300.batched import BatchedSolver
+
+    nsteps = 4
+    sizes = [31, 77, 166, 400, 1000]
+    rng = np.random.default_rng(23)
+    u0 = torch.tensor(np.concatenate([_state(kind, n, rng) for n in sizes]))
+    p = torch.tensor(rng.standard_normal(sum(sizes))).cuda()
+    out = []
+    for tile in (0, 64, 216, 448):
+        s = BatchedSolver(_scheme("rusanov"), sizes, [2.0 / n for n in sizes], theta=0.5, tile=tile, max_steps=nsteps)
+        c = CheckpointedSolve(s, nsteps)
+        c.forward(u0.cuda())
+        out.append(c.backward(p).clone())
+        dts = s.dt_history()
+    for g in out[1:]:
+        assert torch.equal(g, out[0])
+    o = 0
+    for b, n in enumerate(sizes):
+        states = [u0[o : o + n]]
+        for k in range(nsteps - 1):
+            states.append(T.ssprk33(states[-1][None], float(dts[k][b]), 2.0 / n)[0])
+        q = p[o : o + n].cpu()
+        for k in reversed(range(nsteps)):
+            q = T.step_vjp(states[k][None], q[None], float(dts[k][b]), 2.0 / n)[0]
+        err = float((out[0][o : o + n].cpu() - q).abs().max() / q.abs().max())
+        assert err < nsteps * 1.0e-11, (n, err)
+        o += n
