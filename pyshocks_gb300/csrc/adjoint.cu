@@ -1117,6 +1117,11 @@ struct SingleVjpLaunch {
 
 extern "C" {
 
+// longest array that the single transposed step leaves to the FP64 backward, as the single
+// step does (us, FP64 / float pairs, smooth and random states: 64 cells 31 / 47, 41; 96
+// 34 / 47, 45; 128 42 / 47, 52; 192 50 / 46, 56; 256 80 / 47, 72)
+static constexpr int64_t kFxVjpCells = 128;
+
 int shk_ssprk33_vjp_bc_f64(const shk_scheme* scheme, const shk_boundary* bc, const double* u,
                            const double* p_next, double* p_out, int64_t n, int32_t nghosts,
                            double dx, double dt, void* stream) {
@@ -1135,7 +1140,7 @@ int shk_ssprk33_vjp_bc_f64(const shk_scheme* scheme, const shk_boundary* bc, con
     const size_t smem = AdjSmem<double>::host_bytes(W);
     const int blocks = static_cast<int>((n + tile - 1) / tile);
     SingleVjpLaunch f{u, p_next, p_out, n, nghosts, tile, dt / dx, adj_params<double>(scheme),
-                      smem, blocks, st, b, dx, fixed_flux_scheme(scheme)};
+                      smem, blocks, st, b, dx, fixed_flux_scheme(scheme) && n > kFxVjpCells};
     return by_equation<double>(scheme->equation, f);
 }
 

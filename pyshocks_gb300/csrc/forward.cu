@@ -873,11 +873,14 @@ struct ApplyOpLaunch {
 struct SingleStepLaunch {
     const double* u; double* uo; int64_t n; int g; int tile; double dtdx;
     OpParams<double> p; size_t smem; int blocks; cudaStream_t st; shk_boundary bc; double dx;
+    bool fixed;  // (of a scheme with a kFluxRusanovFx form)
     template <class T, int EQ, int REC, int FLUX> int operator()() {
         if constexpr (FLUX == SHK_FLUX_LF) {
             return SHK_EUNSUPPORTED;
         } else {
             auto k = single_step_kernel<T, EQ, REC, FLUX>;
+            if constexpr (FLUX == kFluxRusanovFx)
+                if (!fixed) k = single_step_kernel<T, EQ, REC, SHK_FLUX_RUSANOV>;
             SHK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             k<<<blocks, kThreads, smem, st>>>(u, uo, n, g, tile, dtdx, p, nullptr, bc, dx);
             return cuda_check(cudaGetLastError());
@@ -1184,6 +1187,12 @@ int shk_predict_timestep_f64(const shk_scheme* scheme, const double* u, int64_t 
     return cuda_check(cudaGetLastError());
 }
 
+// longest array that the single step leaves to the FP64 formula: on the coarsest grids
+// most faces are left to FP64 anyhow (us, FP64 formula / fixed fluxes, smooth and random
+// states: 64 cells 12.4 / 14.3, 20.8; 96 12.6 / 14.5, 20.8; 128 14.6 / 13.5, 20.8; 192
+// 16.6 / 8.4, 20.8; 256 26.9 / 8.5, 22.7)
+static constexpr int64_t kFxStepCells = 96;
+
 int shk_ssprk33_step_bc_f64(const shk_scheme* scheme, const shk_boundary* bc, const double* u,
                             double* u_out, int64_t n, int32_t nghosts, double dx, double dt,
                             void* stream) {
@@ -1195,13 +1204,14 @@ int shk_ssprk33_step_bc_f64(const shk_scheme* scheme, const shk_boundary* bc, co
     if (!valid_boundary(b)) return SHK_EINVAL;
     cudaStream_t st = as_stream(stream);
     // fixed fluxes: 8 warps x 60 faces cover a tile and its first stage's halo
-    const int tile = fixed_flux_scheme(scheme) ? 466 : 512;
+    const bool fixed = fixed_flux_scheme(scheme) && n > kFxStepCells;
+    const int tile = fixed ? 466 : 512;
     const int W = tile + 2 * step_halo<double>();
-    const size_t smem = Smem<double>::step_bytes(W, scheme->rec, fixed_flux_scheme(scheme));
+    const size_t smem = Smem<double>::step_bytes(W, scheme->rec, fixed);
     const int blocks = static_cast<int>((n + tile - 1) / tile);
     OpParams<double> p = make_params<double>(scheme);
     p.dx = dx;
-    SingleStepLaunch f{u, u_out, n, nghosts, tile, dt / dx, p, smem, blocks, st, b, dx};
+    SingleStepLaunch f{u, u_out, n, nghosts, tile, dt / dx, p, smem, blocks, st, b, dx, fixed};
     const int r = dispatch_scheme<double>(scheme, f);
     if (r != SHK_OK || (b.left == SHK_BC_PERIODIC && b.right == SHK_BC_PERIODIC)) return r;
     bc_ghost_kernel<double><<<1, 64, 0, st>>>(u_out, n, nghosts, b, dx, 1, 0);
@@ -1354,7 +1364,9 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
     // waits for another's steps) and is short enough for one: up to 1536 cells a
     // CTA of its share of an SM's 32 warps needs at most two rounds of 60 faces a
     // warp; longer instances are faster spread over several SMs. A caller that
-    // names a launch shape gets that shape.
+    // names a launch shape gets that shape. Four warps at least: each quarter of an SM
+    // has its own FP64 pipe (24 instances of 32 cells, where nearly all faces are left
+    // to FP64: 20.0 us a step with one warp, 12.2 with four; FP64 formula, launched: 16.6).
     if (!(opts && (opts->tile > 0 || opts->ctas_per_sm > 0)) && resident_scheme(scheme, dtype)) {
         int64_t nmax = 0;
         for (int b = 0; b < batch; ++b) nmax = std::max(nmax, h_offsets[b + 1] - h_offsets[b]);
@@ -1364,7 +1376,7 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
                           2 * (dtype == SHK_F64 ? step_halo<double>() : step_halo<float>());
             const size_t smem = dtype == SHK_F64 ? Smem<double>::step_bytes(W, scheme->rec, true)
                                                  : Smem<float>::step_bytes(W, scheme->rec);
-            const int warps = std::min<int>(static_cast<int>((nmax + 14 + 59) / 60), 32 / share);
+            const int warps = std::min<int>(std::max<int>(4, static_cast<int>((nmax + 14 + 59) / 60)), 32 / share);
             if (share * (smem + 2048) <= size_t(227) * 1024) {
                 P->resident = 32 * std::max(1, warps);
                 P->resident_W = W;

@@ -105,3 +105,27 @@ def test_gradient_does_not_depend_on_the_tile(kind):
         err = float((out[0][o : o + n].cpu() - q).abs().max() / q.abs().max())
         assert err < nsteps * 1.0e-11, (n, err)
         o += n
+
+
+@pytest.mark.parametrize("n", [31, 95, 96, 97, 127, 128, 129, 130, 470])
+@pytest.mark.parametrize("kind", ["noise", "random"])
+def test_single_step_and_transpose_on_coarse_grids(kind, n):
+    """The single-instance step and its transpose at the lengths where the FP64
+    formula hands over (96, 128 cells): 1e-13 and 1e-11 of the largest value."""
+    from pyshocks_gb300 import _lib as L
+
+    rng = np.random.default_rng(n)
+    u = torch.tensor(_state(kind, n, rng))
+    p = torch.tensor(rng.standard_normal(n))
+    dx = 2.0 / n
+    dt = 0.4 * dx / float(u.abs().max())
+    cs = _scheme("rusanov").c_scheme(dx)
+    ud, pd = torch.cat([u[-3:], u, u[:3]]).cuda(), torch.cat([p[-3:], p, p[:3]]).cuda()
+    out = torch.empty_like(ud)
+    lib = L.lib()
+    assert lib.shk_ssprk33_step_f64(cs, ud.data_ptr(), out.data_ptr(), n, 3, dx, dt, L.stream_handle()) == 0
+    ref = T.ssprk33(u[None], dt, dx)[0]
+    assert float((out.cpu()[3:-3] - ref).abs().max()) <= 1.0e-13 * float(u.abs().max())
+    assert lib.shk_ssprk33_vjp_f64(cs, ud.data_ptr(), pd.data_ptr(), out.data_ptr(), n, 3, dx, dt, L.stream_handle()) == 0
+    ref = T.step_vjp(u[None], p[None], dt, dx)[0]
+    assert float((out.cpu()[3:-3] - ref).abs().max()) <= 1.0e-11 * float(ref.abs().max())
