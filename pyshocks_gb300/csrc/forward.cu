@@ -610,8 +610,10 @@ __global__ void finalize_dt_kernel(double* dt, double cfl, double theta) {
     *dt = theta * (cfl / smax);
 }
 
-// both in one CTA: a short state's CFL step in one launch instead of three
-constexpr int64_t kBlockDtCells = 32768;
+// both in one CTA: a short state's CFL step in one launch instead of three (us, three
+// launches / one: 256 cells 7.2 / 3.2, 8192 7.3 / 4.9, 12000 7.3 / 6.2, 24000 7.3 / 8.3, 32768
+// 7.3 / 8.5; with the read of dt by the host 8192 21.8 / 19.5, 12000 21.8 / 23.1)
+constexpr int64_t kBlockDtCells = 8192;
 template <int EQ>
 __global__ void __launch_bounds__(1024) block_dt_kernel(const double* __restrict__ u, int n, double c, double cfl,
                                                         double theta, double* dt) {

@@ -1,0 +1,25 @@
+"""Short single-instance calls at the lengths where one CTA hands over to a launch
+per piece (``kBlockDtCells`` in ``csrc/forward.cu``)."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 20000])
+def test_predicted_timestep(n):
+    """theta (cfl / max|u|) with the maximum at either end: exact."""
+    from pyshocks_gb300 import _lib as L
+
+    s = L.ShkScheme(flux=L.SHK_FLUX_RUSANOV, rec=L.SHK_REC_WENOJS53, eps=1.0e-6, nu=1.0, speed=1.0)
+    dt = torch.empty((), dtype=torch.float64, device="cuda")
+    for at in (0, n - 1):
+        u = torch.full((n + 6,), 0.25, dtype=torch.float64, device="cuda")
+        u[3 + at] = -1.7
+        u[:3] = 9.0
+        u[n + 3 :] = -9.0
+        assert L.lib().shk_predict_timestep_f64(s, u.data_ptr(), n, 3, 0.125, 0.5, dt.data_ptr(), L.stream_handle()) == 0
+        assert float(dt) == 0.5 * (0.125 / 1.7)
