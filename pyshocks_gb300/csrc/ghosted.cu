@@ -47,13 +47,19 @@ namespace {
 constexpr int kGhThreads = 256;
 constexpr int kPad = 3;          // zero cells beyond each end of the array
 constexpr int kGhMaxBlocks = 1024;
-// Longest array (cells with ghosts) that one CTA handles. Measured in one CTA
-// against a launch per piece (us, step / transpose): constant reconstruction, LF:
-// 256 cells 14 / 29, 2048 cells 49 / 94 against 75 / 130; WENO-JS5, whose FP64
-// operations one SM carries alone: 256 cells 25 / 72, 1024 cells 78 / 250 against
-// 60 / 125.
-template <int REC>
-constexpr int64_t kGhBlockCells = REC == SHK_REC_CONSTANT ? 3072 : 512;
+// Longest array (cells with ghosts) that one CTA handles, for the step and for its
+// transpose. Measured in one CTA against a launch per piece (us), on either side of the
+// line:
+//   constant, LF step: 2560 cells 58 / 73, 3072 68 / 73; transpose: 2048 90 / 126, 2560
+//     110 / 126, 3072 129 / 127
+//   constant, Rusanov step: 1024 27 / 49, 2048 46 / 48, 3072 65 / 49; transpose: 1024 52 / 78,
+//     2048 95 / 76
+//   WENO-JS5, whose FP64 operations one SM carries alone, LF: 512 cells 42 / 78 and 122 /
+//     156; Rusanov: 448 35 / 57 and 104 / 120, 512 40 / 55 and 118 / 117; 1024 78 / 60 and 250 / 125
+template <int REC, int FLUX, bool VJP>
+constexpr int64_t kGhBlockCells = REC != SHK_REC_CONSTANT ? 512
+                                  : FLUX == SHK_FLUX_LF   ? (VJP ? 2560 : 3072)
+                                                          : (VJP ? 1536 : 2048);
 
 struct GhArgs {
     int64_t n;   // interior cells
@@ -644,7 +650,7 @@ struct GhStep {
     double dt;
     template <int EQ, int REC, int FLUX>
     int run() {
-        if (L.A.M <= kGhBlockCells<REC>) {
+        if (L.A.M <= kGhBlockCells<REC, FLUX, false>) {
             gh_step_block_kernel<EQ, REC, FLUX><<<1, kGhBlockThreads, 0, L.st>>>(L.A, L.W, u, out, dt);
             return gh_cuda(cudaGetLastError());
         }
@@ -701,7 +707,7 @@ struct GhVjp {
     }
     template <int EQ, int REC, int FLUX>
     int run() {
-        if (L.A.M <= kGhBlockCells<REC>) {
+        if (L.A.M <= kGhBlockCells<REC, FLUX, true>) {
             gh_vjp_block_kernel<EQ, REC, FLUX><<<1, kGhBlockThreads, 0, L.st>>>(L.A, L.W, u, p, out, dt);
             return gh_cuda(cudaGetLastError());
         }

@@ -1,5 +1,5 @@
 """Short single-instance calls at the lengths where one CTA hands over to a launch
-per piece (``kBlockDtCells`` in ``csrc/forward.cu``)."""
+per piece (``kBlockDtCells`` in ``csrc/forward.cu``, ``kGhBlockCells`` in ``csrc/ghosted.cu``)."""
 
 from __future__ import annotations
 
@@ -23,3 +23,13 @@ def test_predicted_timestep(n):
         u[n + 3 :] = -9.0
         assert L.lib().shk_predict_timestep_f64(s, u.data_ptr(), n, 3, 0.125, 0.5, dt.data_ptr(), L.stream_handle()) == 0
         assert float(dt) == 0.5 * (0.125 / 1.7)
+
+
+@pytest.mark.parametrize("extra", [0, 1])
+@pytest.mark.parametrize(("fk", "limit"), [("lf", 2560), ("rusanov", 1536), ("rusanov", 2048)])
+def test_ghosted_step_and_transpose(fk, limit, extra):
+    """The constant reconstruction's lines (step and transpose), at the bars of the
+    other ghosted tests."""
+    from test_gpu_block_paths import test_ghosted_step_and_transpose as check
+
+    check("constant", fk, 1, limit, extra)
