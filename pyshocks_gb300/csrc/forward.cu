@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_steps_kernel(
     const double inv_dx = P.inv_dx[b];
     unsigned long long amax = P.amax[size_t(k0 & 1) * P.B + b];  // thread 0 keeps it up to date
     bool ok = load_window<T>(sm.U, uin + off, n, -HL, n + 2 * HL, &bar, phase);
-    if (!ok && threadIdx.x == 0) atomicOr(P.status, ERR_TIMEOUT);
+    if (!ok && threadIdx.x == 0) atomicOr(P.status, ERR_TIMEOUT);  // (and no state is written)
     const Win<T> ug = make_win(u_cur, P.offsets[P.B]) + off;
     const Win<T> pg = make_win(u_prev, P.offsets[P.B]) + off;
     OpParams<T> pb = p;
@@ -273,7 +273,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_steps_kernel(
         }
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ug[i] = sm.U[HL + i];
+    if (ok)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) ug[i] = sm.U[HL + i];
     if (threadIdx.x == 0) {
         P.amax[size_t((k0 + nsteps) & 1) * P.B + b] = amax;
         P.amax[size_t((k0 + nsteps + 1) & 1) * P.B + b] = 0ull;
