@@ -1366,13 +1366,31 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
     // Resident steps where every instance can have a CTA at once (so no instance
     // waits for another's steps) and is short enough for one: up to 1536 cells a
     // CTA of its share of an SM's 32 warps needs at most two rounds of 60 faces a
-    // warp; longer instances are faster spread over several SMs. A caller that
-    // names a launch shape gets that shape. Four warps at least: each quarter of an SM
-    // has its own FP64 pipe (24 instances of 32 cells, where nearly all faces are left
-    // to FP64: 20.0 us a step with one warp, 12.2 with four; FP64 formula, launched: 16.6).
+    // warp where an SM has one or two; longer instances are faster spread over several
+    // SMs. A caller that names a launch shape gets that shape. Four warps at least: each
+    // quarter of an SM has its own FP64 pipe (24 instances of 32 cells, where nearly all
+    // faces are left to FP64: 20.0 us a step with one warp, 12.0 with four; FP64 formula,
+    // launched: 16.6). Double states, whose steps are long, stay launched where most of
+    // the cells (`bulk`, the mean length of a cell's instance) lie in instances that take
+    // several rounds while the others' CTAs idle. Us per step of a call of ten, resident /
+    // launched, by instances per SM:
+    //   all 1000 cells (bulk / mean length 1.0): 1 15 / 21, 2 23 / 29, 3 29 / 40, 5 43 / 59
+    //   uniform 100 to 1536 (1.25): 2 29 / 32, 3 37 / 36, 4 42 / 44, 5 50 / 54
+    //   logarithmic 300 to 1536 (1.21): 2 29 / 29, 3 39 / 35, 4 43 / 40, 5 54 / 49
+    //   logarithmic 100 to 600 (1.26): 1 15 / 25, 3 20 / 30, 5 27 / 34, 8 35 / 49
+    //   logarithmic 100 to 1536 (1.57): 1 20 / 27, 2 28 / 29, 3 38 / 33, 4 40 / 36, 5 48 / 42
+    //   half 200, half 1500 (1.58): 1 20 / 23, 2 31 / 28, 3 42 / 36, 5 61 / 52
+    //   a tenth 1500, the others 200 (2.4): 1 20 / 21, 2 22 / 23, 3 36 / 25, 5 43 / 31
+    //   one 1536, the others 100 (1.3 to 2.1): 1 22 / 28, 3 27 / 31, 5 33 / 41
     if (!(opts && (opts->tile > 0 || opts->ctas_per_sm > 0)) && resident_scheme(scheme, dtype)) {
         int64_t nmax = 0;
-        for (int b = 0; b < batch; ++b) nmax = std::max(nmax, h_offsets[b + 1] - h_offsets[b]);
+        double cells = 0.0, squares = 0.0;
+        for (int b = 0; b < batch; ++b) {
+            const int64_t n = h_offsets[b + 1] - h_offsets[b];
+            nmax = std::max(nmax, n);
+            cells += double(n);
+            squares += double(n) * double(n);
+        }
         const int share = (batch + sm_count() - 1) / sm_count();
         if (nmax <= 1536 && share <= 8) {
             const int W = static_cast<int>((nmax + 3) / 4 * 4) +
@@ -1380,7 +1398,9 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
             const size_t smem = dtype == SHK_F64 ? Smem<double>::step_bytes(W, scheme->rec, true)
                                                  : Smem<float>::step_bytes(W, scheme->rec);
             const int warps = std::min<int>(std::max<int>(4, static_cast<int>((nmax + 14 + 59) / 60)), 32 / share);
-            if (share * (smem + 2048) <= size_t(227) * 1024) {
+            const double bulk = squares / cells, mean = cells / batch;
+            const bool idle = dtype == SHK_F64 && bulk + 14 > 60 * warps && bulk > 1.3 * mean;
+            if (share * (smem + 2048) <= size_t(227) * 1024 && !idle) {
                 P->resident = 32 * std::max(1, warps);
                 P->resident_W = W;
             }

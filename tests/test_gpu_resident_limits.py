@@ -1,8 +1,9 @@
 """Resident plans (all steps of a call in one launch) at their limits: a wait that
-runs out."""
+runs out, and batches of mixed lengths on either side of the rule that chooses them."""
 
 from __future__ import annotations
 
+import numpy as np
 import pytest
 import torch
 
@@ -44,3 +45,28 @@ def test_a_timed_out_window_writes_no_state():
                 assert checked.shk_check_force_timeout(0, 0) == 0
             assert torch.equal(s.buf_a.cpu(), u0)
             assert torch.all(s.buf_b == 7.0)
+
+
+@pytest.mark.parametrize("long_share", [2, 10, 400])
+@pytest.mark.parametrize("batch", [300, 456, 760])
+def test_mixed_lengths_equal_launched_steps(batch, long_share):
+    """Every second, every tenth instance, or one, has 1500 cells and the others 200
+    (two, three and five instances an SM): bit for bit the launched steps."""
+    from pyshocks_gb300.batched import BatchedSolver
+
+    sizes = np.where(np.arange(batch) % long_share, 200, 1500)
+    if long_share == 400:
+        sizes[1:] = 200
+    rng = np.random.default_rng(9)
+    x = np.concatenate([(np.arange(n) + 0.5) / n for n in sizes])
+    u0 = torch.tensor(0.4 + np.sin(2 * np.pi * x) * np.repeat(rng.uniform(0.2, 1.0, batch), sizes))
+    out = []
+    for tile in (0, 466):
+        s = BatchedSolver(_scheme(), sizes, 2.0 / sizes, theta=0.9, tile=tile)
+        s.reset(u0)
+        s.step(3)
+        s.step(2)
+        assert s.status() == 0
+        out.append((s.u.clone(), s.time()))
+    assert torch.equal(out[0][0], out[1][0])
+    assert torch.equal(out[0][1], out[1][1])
