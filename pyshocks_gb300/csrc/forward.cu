@@ -1077,6 +1077,8 @@ int launch_step(shk_plan* P, const void* uin, void* uout, cudaStream_t st) {
 }  // namespace
 
 namespace {
+// most steps of one resident launch (some 10 ms): nothing can stop a kernel
+constexpr int kResidentSteps = 512;
 // steps of a resident plan (see shk_plan_create)
 template <class T>
 int launch_resident(shk_plan* P, void* u_a, void* u_b, int nsteps, cudaStream_t st) {
@@ -1465,11 +1467,16 @@ int shk_plan_reset(shk_plan* plan, const void* u, const double* t0, const double
 int shk_plan_step(shk_plan* plan, void* u_a, void* u_b, int32_t nsteps, void* stream) {
     if (!plan || !u_a || !u_b || u_a == u_b || nsteps < 0) return SHK_EINVAL;
     cudaStream_t st = as_stream(stream);
-    if (plan->resident && nsteps > 0) {
-        const int r = plan->dtype == SHK_F64 ? launch_resident<double>(plan, u_a, u_b, nsteps, st)
-                                             : launch_resident<float>(plan, u_a, u_b, nsteps, st);
-        if (r == SHK_OK) plan->host_steps += nsteps;
-        return r;
+    if (plan->resident) {
+        while (nsteps > 0) {
+            const int k = std::min(nsteps, kResidentSteps);
+            const int r = plan->dtype == SHK_F64 ? launch_resident<double>(plan, u_a, u_b, k, st)
+                                                 : launch_resident<float>(plan, u_a, u_b, k, st);
+            if (r != SHK_OK) return r;
+            plan->host_steps += k;
+            nsteps -= k;
+        }
+        return SHK_OK;
     }
     for (int i = 0; i < nsteps; ++i) {
         const bool even = (plan->host_steps % 2) == 0;

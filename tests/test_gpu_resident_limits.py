@@ -1,5 +1,6 @@
 """Resident plans (all steps of a call in one launch) at their limits: a wait that
-runs out, and batches of mixed lengths on either side of the rule that chooses them."""
+runs out, batches of mixed lengths on either side of the rule that chooses them, and
+calls longer than one launch."""
 
 from __future__ import annotations
 
@@ -70,3 +71,24 @@ def test_mixed_lengths_equal_launched_steps(batch, long_share):
         out.append((s.u.clone(), s.time()))
     assert torch.equal(out[0][0], out[1][0])
     assert torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("nsteps", [511, 512, 513, 1025])
+def test_long_calls_equal_launched_steps(nsteps, dtype):
+    """A call of more than 512 steps takes several launches: both buffers and the
+    times of the launched steps, bit for bit, and of the call after it."""
+    from pyshocks_gb300.batched import BatchedSolver
+
+    sizes = np.array([40, 77, 128])
+    x = np.concatenate([(np.arange(n) + 0.5) / n for n in sizes])
+    out = []
+    for tile in (0, 64):
+        s = BatchedSolver(_scheme(), sizes, 2.0 / sizes, theta=0.9, tile=tile, dtype=dtype)
+        s.reset(torch.tensor(0.4 + np.sin(2 * np.pi * x)))
+        s.step(nsteps)
+        s.step(2)
+        assert s.status() == 0
+        out.append((s.buf_a.clone(), s.buf_b.clone(), s.time()))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
