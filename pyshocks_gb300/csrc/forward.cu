@@ -1018,6 +1018,7 @@ struct shk_plan {
     // all steps of a call in one launch, one CTA per instance: its threads (0: no)
     // and window length
     int resident = 0, resident_W = 0;
+    bool too_long = false;  // tile beyond the FP64 formula's layout (see shk_plan_create)
     // captured two-step graph
     cudaGraphExec_t graph = nullptr;
     void* graph_a = nullptr;
@@ -1051,8 +1052,11 @@ int launch_max(shk_plan* P, const void* u, int slot, cudaStream_t st) {
     return cuda_check(cudaGetLastError());
 }
 
+constexpr size_t kStepStatic = 312;  // static shared memory of the FP64 formula's step
+
 template <class T>
 int launch_step(shk_plan* P, const void* uin, void* uout, cudaStream_t st) {
+    if (P->too_long) return SHK_ECUDA;
     const PlanDev D = P->dev();
     if (P->scheme.flux == SHK_FLUX_LF) {
         if constexpr (sizeof(T) != 8) {
@@ -1348,10 +1352,25 @@ int shk_plan_create(const shk_scheme* scheme, int32_t batch, const int64_t* h_of
         shk_plan_destroy(P);
         return SHK_ECUDA;
     }
-    // persistent grid: resident CTAs per SM x SMs
+    // The integer-flux layouts are shorter than the FP64 formula's, but which tiles a
+    // plan takes does not depend on eps or nu: a tile beyond that formula's layout is
+    // refused (here, or by the step where the caller names the CTAs)
+    const bool fixed_lf = fixed_flux_scheme(scheme, SHK_FLUX_LF);
     int per_sm = opts && opts->ctas_per_sm > 0 ? opts->ctas_per_sm : 0;
+    if (dtype == SHK_F64 && (fixed_lf || fixed_flux_scheme(scheme))) {
+        const size_t bytes = lf ? Smem<double>::lf_stage_bytes(tile + 2 * op_halo<double>(), false)
+                                : Smem<double>::step_bytes(tile + 2 * step_halo<double>(), scheme->rec);
+        int dev = 0, optin = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        P->too_long = bytes + kStepStatic > static_cast<size_t>(optin);
+        if (P->too_long && per_sm == 0) {
+            shk_plan_destroy(P);
+            return SHK_EINVAL;
+        }
+    }
+    // persistent grid: resident CTAs per SM x SMs
     if (per_sm == 0) {
-        const bool fixed_lf = fixed_flux_scheme(scheme, SHK_FLUX_LF);
         const size_t smem = lf ? Smem<double>::lf_stage_bytes(tile + 2 * op_halo<double>(), fixed_lf)
                                : (dtype == SHK_F64 ? Smem<double>::step_bytes(tile + 2 * step_halo<double>(), scheme->rec, fixed_flux_scheme(scheme))
                                                    : Smem<float>::step_bytes(tile + 2 * step_halo<float>(), scheme->rec));
