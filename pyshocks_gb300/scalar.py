@@ -135,11 +135,20 @@ def _fill_neumann(bc, grid, t, u) -> None:
     boundary mirrored, plus distance x gradient (none for a zero gradient)."""
     g = grid.nghosts
     n = u.shape[0]
+    x = grid.x
+    if u.ndim != 1 or n != x.numel() or u.dtype != x.dtype or u.device != x.device:
+        # not a state of this grid: by cell numbers, with what indexing and
+        # broadcasting make of it or refuse
+        ifrom = torch.arange(*grid.gi_[bc.side].indices(n), device=u.device)
+        first = g - 1 if bc.side == -1 else n - 1
+        ito = torch.arange(first, first - g, -1, device=u.device)
+        u[ito] = u[ifrom] + bc.side * (x[ifrom] - x[ito]) * float(bc.g(t))
+        return
     inner, ghost = (slice(g, 2 * g), slice(0, g)) if bc.side == -1 else (slice(n - 2 * g, n - g), slice(n - g, n))
     gn = float(bc.g(t))
     v = u[inner]
     if gn != 0.0:
-        v = v + (grid.x[inner] - grid.x[ghost].flip(0)) * (bc.side * gn)
+        v = v + (x[inner] - x[ghost].flip(0)) * (bc.side * gn)
     u[ghost] = v.flip(0)
 
 
