@@ -65,20 +65,31 @@ class Grid:
     def ghost_centres(self, side: int) -> torch.Tensor:
         """Centres (float64, a tensor of the caller's own) of the three ghost
         cells of *side* (0: left, 1: right), the one next to the interior first;
-        beyond a grid's own ghosts they continue outward. Laid out once per grid,
-        from host values."""
-        rows = self.__dict__.get("_ghost_centres")
-        if rows is None:
-            g, n, h = self.nghosts, self.ncells, float(self.dx_min)
-            x, f = self.x.detach().cpu().double(), self.f.detach().cpu().double()
-            out = []
-            for s, first, x0, sgn in ((0, g - 1, float(f[g]), -1), (1, g + n, float(f[g + n]), 1)):
-                out.append([float(x[first + sgn * k]) if k < g else x0 + sgn * (k + 0.5) * h for k in range(3)])
-            rows = torch.tensor(out, dtype=torch.float64, device=self.x.device)
-            if rows.is_cuda:  # complete before any other stream reads it
-                torch.cuda.current_stream(rows.device).synchronize()
-            object.__setattr__(self, "_ghost_centres", rows)
+        beyond a grid's own ghosts they continue outward. Laid out once per grid
+        (and again after its coordinates were changed in place), from host
+        values."""
+        versions = _versions(self.x, self.f)
+        kept = self.__dict__.get("_ghost_centres")
+        if kept is not None and versions is not None and kept[0] == versions:
+            return kept[1][side].clone()
+        g, n, h = self.nghosts, self.ncells, float(self.dx_min)
+        x, f = self.x.detach().cpu().double(), self.f.detach().cpu().double()
+        out = []
+        for s, first, x0, sgn in ((0, g - 1, float(f[g]), -1), (1, g + n, float(f[g + n]), 1)):
+            out.append([float(x[first + sgn * k]) if k < g else x0 + sgn * (k + 0.5) * h for k in range(3)])
+        rows = torch.tensor(out, dtype=torch.float64, device=self.x.device)
+        if rows.is_cuda:  # complete before any other stream reads it
+            torch.cuda.current_stream(rows.device).synchronize()
+        if versions is not None and not rows.is_inference():
+            object.__setattr__(self, "_ghost_centres", (versions, rows))
         return rows[side].clone()
+
+
+def _versions(*tensors: torch.Tensor) -> tuple | None:
+    """Counters of the tensors' in-place changes (None where there are none)."""
+    if any(t.is_inference() for t in tensors):
+        return None
+    return tuple(t._version for t in tensors)
 
 
 @dataclass(frozen=True)
