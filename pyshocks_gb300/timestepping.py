@@ -92,8 +92,9 @@ class TimestepPredictor:
         from pyshocks_gb300 import burgers
         from pyshocks_gb300.schemes import predict_timestep
 
-        if predict_timestep.dispatch(type(self.scheme)) is burgers._predict_timestep_gpu:
-            # the product is formed by the kernel that forms the estimate
+        if (isinstance(self.theta, (int, float))
+                and predict_timestep.dispatch(type(self.scheme)) is burgers._predict_timestep_gpu):
+            # a number's product is formed by the kernel that forms the estimate
             return burgers.scaled_timestep(self.scheme, self.grid, self.theta, u)
         return self.theta * predict_timestep(self.scheme, self.grid, self.bc, t, u)
 

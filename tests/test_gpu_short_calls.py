@@ -33,3 +33,24 @@ def test_ghosted_step_and_transpose(fk, limit, extra):
     from test_gpu_block_paths import test_ghosted_step_and_transpose as check
 
     check("constant", fk, 1, limit, extra)
+
+
+@pytest.mark.parametrize("theta", [0.5, 1, torch.tensor([0.25, 0.5], dtype=torch.float64), torch.tensor(0.5)])
+def test_time_step_factor_of_any_kind(theta):
+    """The driver's ``theta * predict_timestep``: a number, or a tensor that
+    broadcasts and keeps its gradient."""
+    import pyshocks_gb300 as gb
+    from pyshocks_gb300 import burgers, scalar, timestepping
+    from pyshocks_gb300.schemes import predict_timestep
+
+    rec = gb.reconstruction.make_reconstruction_from_name("wenojs53", eps=1.0e-6)
+    grid = gb.make_uniform_cell_grid(a=-1.0, b=1.0, n=64, nghosts=3)
+    bc = scalar.PeriodicBoundary()
+    scheme = gb.bind(burgers.Rusanov(rec=rec), grid, bc)
+    u = torch.sin(grid.x)
+    if torch.is_tensor(theta):
+        theta = theta.cuda().requires_grad_()
+    dt = timestepping.TimestepPredictor(scheme, grid, bc, theta)(0.0, u)
+    ref = theta * predict_timestep(scheme, grid, bc, 0.0, u)
+    assert dt.shape == ref.shape and torch.equal(dt.detach(), ref.detach())
+    assert dt.requires_grad == ref.requires_grad
