@@ -24,15 +24,19 @@ from typing import Sequence
 import numpy as np
 import torch
 
-#: candidate tile lengths (multiples of 16 cells keep every window 16-byte aligned)
+#: candidate tile lengths (even numbers of 16 bytes: every window starts 16-byte
+#: aligned)
 TILES = (512, 1024, 2048, 4096)
-#: float64 WENO-JS5 plans add the tiles that fill whole rounds of the integer-flux
-#: kernels' warps (60 faces each; 58 outputs each in the reverse step): 4096
+#: integer-flux plans add the tiles that fill whole rounds of those kernels' warps (60 faces each; 58 outputs each in the reverse step): 4096
 #: instances, 25.9 M cells, per step: tile 946 1129 us, 706 1164, 466 1246
 TILES_F64 = (226, 466, 706, 946)
 TILES_F64_ADJOINT = (216, 448)
-#: candidate resident CTAs per SM (0: the plan's own choice from shared memory)
+#: candidate resident CTAs per SM (0: the plan's own choice from shared memory); the
+#: integer-flux kernels are built for up to eight
 CTAS_PER_SM = (0, 1, 2, 3, 4)
+CTAS_PER_SM_FIXED = CTAS_PER_SM + (6, 8)
+#: longest instance of plans that may take all steps of a call in one launch
+SHORT_CELLS = 1536
 #: the shared memory one SM offers to resident CTAs (bytes)
 SMEM_PER_SM = 227 * 1024
 
@@ -72,8 +76,20 @@ LEARNED_STATIC = 3584
 LEARNED_STATIC_ADJOINT = 6400
 
 
-def _smem_bytes(tile: int, dtype: torch.dtype, learned: bool = False, weno5: bool = False) -> int:
-    # the step tile's shared memory: 7 double arrays of the window (halo 10),
+def integer_flux(scheme, dx: float) -> bool:
+    """Whether the library steps *scheme* on the integer fluxes (``fixed_flux_scheme``
+    in ``csrc/stencil.cuh``, for float64 states)."""
+    from pyshocks_gb300 import _lib as L
+
+    cs = scheme.c_scheme(float(dx))
+    return (cs.rec == L.SHK_REC_WENOJS53 and cs.equation == L.SHK_EQ_BURGERS and cs.nu == 1.0
+            and cs.flux in (L.SHK_FLUX_RUSANOV, L.SHK_FLUX_LF) and 1.0e-24 <= cs.eps <= 1.0e24)
+
+
+def _smem_bytes(tile: int, dtype: torch.dtype, learned: bool = False, weno5: bool = False,
+                fixed: bool = False) -> int:
+    # the step tile's shared memory: 7 double arrays of the window (halo 10), 3 and
+    # a list of ints for the integer fluxes,
     # or for the learned reconstruction the double window plus 6 float arrays
     # (the face-flux array at least 1028 floats); for float32 states (halo 12)
     # 6 float arrays with WENO-JS5, else 8
@@ -81,7 +97,7 @@ def _smem_bytes(tile: int, dtype: torch.dtype, learned: bool = False, weno5: boo
         w = tile + 20
         if learned:
             return w * 8 + (5 * w + max(w, 1028)) * 4 + LEARNED_STATIC
-        return w * 7 * 8
+        return w * 3 * 8 + (w + 4) * 4 if fixed else w * 7 * 8
     return (6 if weno5 else 8) * (tile + 24) * 4 + (LEARNED_STATIC if learned else 0)
 
 
@@ -96,23 +112,25 @@ def _adjoint_smem_bytes(tile: int, dtype: torch.dtype, learned: bool = False) ->
 
 
 def candidates(dtype: torch.dtype, max_cells: int, learned: bool = False,
-               adjoint: bool = False, weno5: bool = False) -> list[tuple[int, int]]:
+               adjoint: bool = False, weno5: bool = False, fixed: bool = False) -> list[tuple[int, int]]:
     """(tile, ctas_per_sm) pairs whose shared memory fits one SM; tiles longer
     than twice the largest instance are skipped (they only add idle lanes);
-    with ``adjoint`` only tiles whose reverse step fits too."""
-    out = []
+    with ``adjoint`` only tiles whose reverse step fits too. ``fixed``: the integer
+    fluxes. The first pair, (0, 0), is the plan's own choice: the only one by
+    which short instances take all steps of a call in one launch."""
+    out = [(0, 0)]
     tiles = TILES
-    if dtype == torch.float64 and weno5:
+    if dtype == torch.float64 and fixed:
         tiles = (TILES_F64_ADJOINT if adjoint else TILES_F64) + TILES
     for tile in tiles:
         if tile > max(2 * max_cells, TILES[0]):
             continue
         if adjoint and _adjoint_smem_bytes(tile, dtype, learned) > SMEM_PER_SM:
             continue
-        per = _smem_bytes(tile, dtype, learned, weno5)
+        per = _smem_bytes(tile, dtype, learned, weno5, fixed)
         if per > SMEM_PER_SM:
             continue
-        for c in CTAS_PER_SM:
+        for c in CTAS_PER_SM_FIXED if fixed else CTAS_PER_SM:
             if c and c * per > SMEM_PER_SM:
                 continue
             out.append((tile, c))
@@ -151,13 +169,17 @@ def tune(scheme, sizes: Sequence[int], dx, *, dtype: torch.dtype = torch.float64
         step dominates and prefers other shapes than the forward).
 
     :arg u0: packed state to step from (default: a smooth state of O(1)
-        values); the step cost does not depend on the data except through the
-        learned reconstruction's fallback branches.
+        values). The cost of a step depends on the data where rough faces leave
+        the integer fluxes for FP64 (with noise, several times the smooth cost)
+        or the network falls back: give a typical state for such batches.
     """
     from pyshocks_gb300.batched import BatchedSolver, pack_offsets
 
-    # (v2: shapes timed on kernels with other CTA sizes are not taken from the file)
-    key = shape_key(scheme, sizes, dtype, device) + (":adjoint" if adjoint else "") + ":v2"
+    fixed = dtype == torch.float64 and integer_flux(scheme, np.ravel(dx)[0])
+    # (v3: shapes timed on kernels with other CTA sizes, or without the plan's own
+    # choice among them, are not taken from the file)
+    key = (shape_key(scheme, sizes, dtype, device) + (":integer" if fixed else "") + (":adjoint" if adjoint else "")
+           + ":v3")
     if use_cache:
         if key in _MEMO:
             return _MEMO[key]
@@ -174,10 +196,12 @@ def tune(scheme, sizes: Sequence[int], dx, *, dtype: torch.dtype = torch.float64
     stream = torch.cuda.Stream(device=device)
     table = []
     k = 2 * max(1, steps // 2)
+    if not adjoint and sizes.max() <= SHORT_CELLS:
+        k = max(k, 32)  # (a call's launch would hide what its steps cost)
     learned = type(getattr(scheme, "rec", None)).__name__ == "LearnedWENO"
     weno5 = type(getattr(scheme, "rec", None)).__name__ == "WENOJS53"
-    for tile, cps in candidates(dtype, int(sizes.max()), learned, adjoint, weno5):
-        if learned and tile < 512:
+    for tile, cps in candidates(dtype, int(sizes.max()), learned, adjoint, weno5, fixed):
+        if learned and 0 < tile < 512:
             continue  # the learned phase's warp scratch needs 512-cell tiles
         solver = BatchedSolver(scheme, sizes, dx, theta=theta, dtype=dtype, tile=tile,
                                ctas_per_sm=cps, device=device, max_steps=k if adjoint else 0)

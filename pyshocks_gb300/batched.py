@@ -156,8 +156,10 @@ class BatchedSolver:
     :arg dtype: ``torch.float64`` or ``torch.float32`` state.
     :arg max_steps: capacity of the per-step dt history (for the adjoint).
     :arg tile: cells per work item (0: the library default, which depends on
-        the scheme, precision and whether the plan keeps a dt history; ``"auto"``:
-        chosen with ``ctas_per_sm`` by :func:`pyshocks_gb300.autotune.tune`).
+        the scheme, precision, the plan's cells and whether it keeps a dt history;
+        short instances may then take all steps of a call in one launch, with no
+        tiles; ``"auto"``: chosen with ``ctas_per_sm`` by
+        :func:`pyshocks_gb300.autotune.tune`).
     :arg ctas_per_sm: resident CTAs per SM of the persistent grid (0: as many
         as the shared memory allows, at most 8).
     """
