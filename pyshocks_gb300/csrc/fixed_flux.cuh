@@ -386,8 +386,8 @@ SHK_FX CellGrad lane_grad(const CellWeights& w, FF S, FF E, FF Tm, FF T0, FF gR,
     return g;
 }
 
-// v 2^(1023 - em) as two floats (truncated upper part, exact rest), on the integer
-// pipe; em the biased exponent of the largest value of the warp, 200 .. 1846. 2^-120
+// v 2^(1023 - em) as two floats (truncated upper part, the rest rounded to 24 bits: 48
+// bits in all), on the integer pipe; em the biased exponent of the largest value of the warp, 200 .. 1846. 2^-120
 // below it and less: zero.
 SHK_FX void split_double(double v, uint32_t em, float& h, float& l) {
     const uint32_t hi = static_cast<uint32_t>(dhi(v)), lo = dlo(v);
@@ -399,11 +399,13 @@ SHK_FX void split_double(double v, uint32_t em, float& h, float& l) {
     // power of two
     l = (static_cast<float>(lo & 0x1fffffffu) * 0x1p-52f) * bitsf(b & 0xff800000u);
 }
-// (h + l) 2^(em - 1023) as a double, |l| at most a unit of h, on the integer pipe
+// (h + l) 2^(em - 1023) as a double, |l| at most a unit of h, on the integer pipe; down to
+// |h| = 2^-97, where l's units reach float's smallest number
 SHK_FX double join_double(float h, float l, uint32_t em) {
     const uint32_t b = fbits(h), e = (b >> 23) & 0xffu;
-    const uint32_t es = 306u - (e > 60u ? e : 60u);
-    const int32_t li = f2i(l * bitsf(es << 23));
+    // l in units of 2^-52 of h's power of two, in two factors where one would overflow
+    const uint32_t ec = e > 52u ? e : 52u;
+    const int32_t li = f2i((l * bitsf((306u - ec) << 23)) * bitsf((127u + ec - e) << 23));
     const int64_t u = (static_cast<int32_t>(b) < 0) ? -int64_t(li) : int64_t(li);
     const uint64_t d = (uint64_t(((b & 0x7fffffffu) >> 3) + ((em - 127u) << 20)) << 32 | uint64_t(b << 29)) +
                        static_cast<uint64_t>(u);
