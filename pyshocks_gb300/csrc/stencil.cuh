@@ -816,8 +816,7 @@ __device__ __forceinline__ void fx_listed_flux(PV v, Win<double> G, int j, doubl
     G[j] = g;
 }
 
-// few among a warp's faces: shared out over the CTA after a barrier, two lanes per
-// face, one for each side (38 FP64 instructions for 16 faces)
+// few: two lanes per face, one for each side (38 FP64 instructions for 16 faces)
 template <class PV, class FaceOut>
 __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list, int cnt, double eps,
                                              double aglob, FaceOut out) {
@@ -837,42 +836,50 @@ __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list,
     }
 }
 
-// many: at once by that warp, both sides of every cell, two cells per lane (74 FP64
-// instructions for 60 faces), the neighbours' differences by shuffle. The same operations
-// on the same values give a side's correction, so it does not depend on how many
-// others are left. l0, l1: this lane's faces c0 = r0 + 2 lane and c0 + 1
+// many: both sides of every cell, two cells per lane (74 FP64 instructions for 60
+// faces), the neighbours' differences by shuffle; chunks without a listed face are
+// skipped. The same operations on the same values give a side's correction, so it does
+// not depend on how many others are listed.
+// Taken for more than half of a window's faces where it has more than one
+// chunk and a half: an FP64 instruction holds a quarter of an SM for 64 clocks, and the
+// list spreads the faces of a short window further. Measured (us per step: FP64 formula
+// for every face / all listed faces by two one-sided product-form evaluations / this),
+// 1024 instances, 6.4 M cells: 0.5 % noise 1948 / 2794 / 1606, random cells 1948 / 3016 /
+// 1611, smooth 1948 / 285 / 284; 24 instances of 100 to 1000 cells: noise 57 / 40 / 36,
+// random 57 / 78 / 49; 1000 random instances of 128 cells: 71 / 81 / 55, of 64 cells:
+// 57 / 47 / 47. (Each warp taking its own chunk at once, before the barrier: noise 5 %
+// faster on 300 ragged instances, smooth states 1 % slower.)
+__device__ __forceinline__ bool fx_many(int cnt, int faces) { return 2 * cnt > faces && faces > 90; }
 template <class PV, class FaceOut>
-__device__ __noinline__ void fx_listed_chunk(PV v, Win<double> G, int r0, int W, bool l0, bool l1, double eps,
-                                             double aglob, FaceOut out) {
+__device__ __noinline__ void fx_listed_tile(PV v, Win<double> G, Win<int> list, int cnt, int jlo, int jhi, int W,
+                                            double eps, double aglob, FaceOut out) {
     constexpr unsigned kFull = 0xffffffffu;
-    const int c0 = r0 + 2 * (threadIdx.x & 31);
+    constexpr int kMark = 0x7ff80001;  // upper word of a listed face's place in G
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const double eps4 = 4.0 * eps;
-    // (cells outside the window only feed faces that are not stored)
-    const int ca = c0 < 0 ? 0 : (c0 < W - 2 ? c0 : W - 2);
-    const double vm = v[ca > 0 ? ca - 1 : 0], v0 = v[ca], v1 = v[ca + 1], v2 = v[ca < W - 2 ? ca + 2 : ca + 1];
-    const double dm = v0 - vm, d0 = v1 - v0, d1 = v2 - v1;
-    const double E0 = d0 - dm, E1 = d1 - d0;
-    const double G0 = weno53_g(E0, eps4), G1 = weno53_g(E1, eps4);
-    const double Em = __shfl_up_sync(kFull, E1, 1), Gm = __shfl_up_sync(kFull, G1, 1);
-    const double Ep = __shfl_down_sync(kFull, E0, 1), Gp = __shfl_down_sync(kFull, G0, 1);
-    const WenoTerms a = weno53_terms(dm, d0, Em, E0, E1, Gm, G0, G1);
-    const WenoTerms b = weno53_terms(d0, d1, E0, E1, Ep, G0, G1, Gp);
-    const double L2 = __shfl_down_sync(kFull, weno53_left(a, dm, d0), 1);
-    const double R0 = weno53_right(a, dm, d0), L1 = weno53_left(b, d0, d1), R1 = weno53_right(b, d0, d1);
-    if (l0) fx_listed_flux(v, G, c0, R0, L1, aglob, out);
-    if (l1) fx_listed_flux(v, G, c0 + 1, R1, L2, aglob, out);
-}
-// Whether a warp's faces that are left make a chunk. An FP64 instruction holds a quarter
-// of an SM for 64 clocks: short windows, whose chunks would leave quarters idle, spread
-// their faces by the list (up to 90 faces always, up to 180 unless nearly all of a chunk
-// are left). Measured (us per step: FP64 formula for every face / all left faces in the
-// list with two one-sided evaluations each / this), 1024 instances, 6.4 M cells: 0.5 %
-// noise 1948 / 2794 / 1597, random cells 1948 / 3016 / 1598, smooth 1948 / 285 / 286; 24
-// instances of 100 to 1000 cells: noise 57 / 40 / 34, random 57 / 78 / 48; 1000 random
-// instances of 128 cells: 71 / 81 / 50, of 64 cells: 57 / 47 / 47.
-__device__ __forceinline__ bool fx_many(int faces, bool l0, bool l1) {
-    const int left = __popc(__ballot_sync(0xffffffffu, l0)) + __popc(__ballot_sync(0xffffffffu, l1));
-    return left > 32 && (faces > 180 || (faces > 90 && left > 50));
+    for (int q = threadIdx.x; q < cnt; q += blockDim.x) G[list[q]] = __hiloint2double(kMark, 0);
+    __syncthreads();
+    for (int r0 = (jlo & ~1) - 2 + 60 * warp; r0 + 2 < jhi; r0 += 60 * nw) {
+        const int c0 = r0 + 2 * lane;
+        const bool inner = lane >= 1 && lane <= 30;
+        const bool l0 = inner && c0 >= jlo && c0 < jhi && __double2hiint(G[c0]) == kMark;
+        const bool l1 = inner && c0 + 1 >= jlo && c0 + 1 < jhi && __double2hiint(G[c0 + 1]) == kMark;
+        if (!__any_sync(kFull, l0 || l1)) continue;
+        // (cells outside the window only feed faces that are not stored)
+        const int ca = c0 < 0 ? 0 : (c0 < W - 2 ? c0 : W - 2);
+        const double vm = v[ca > 0 ? ca - 1 : 0], v0 = v[ca], v1 = v[ca + 1], v2 = v[ca < W - 2 ? ca + 2 : ca + 1];
+        const double dm = v0 - vm, d0 = v1 - v0, d1 = v2 - v1;
+        const double E0 = d0 - dm, E1 = d1 - d0;
+        const double G0 = weno53_g(E0, eps4), G1 = weno53_g(E1, eps4);
+        const double Em = __shfl_up_sync(kFull, E1, 1), Gm = __shfl_up_sync(kFull, G1, 1);
+        const double Ep = __shfl_down_sync(kFull, E0, 1), Gp = __shfl_down_sync(kFull, G0, 1);
+        const WenoTerms a = weno53_terms(dm, d0, Em, E0, E1, Gm, G0, G1);
+        const WenoTerms b = weno53_terms(d0, d1, E0, E1, Ep, G0, G1, Gp);
+        const double L2 = __shfl_down_sync(kFull, weno53_left(a, dm, d0), 1);
+        const double R0 = weno53_right(a, dm, d0), L1 = weno53_left(b, d0, d1), R1 = weno53_right(b, d0, d1);
+        if (l0) fx_listed_flux(v, G, c0, R0, L1, aglob, out);
+        if (l1) fx_listed_flux(v, G, c0 + 1, R1, L2, aglob, out);
+    }
 }
 
 // face values of the cells [lo, hi) of a window to ul, ur (indexed from the
@@ -924,33 +931,26 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
                                           fx::p2(s.x.iu, s.y.iu));
         const bool inner = lane >= 1 && lane <= 30;
         const bool m0 = inner && c0 >= jlo && c0 < jhi, m1 = inner && c0 + 1 >= jlo && c0 + 1 < jhi;
-        // (the flux of a face that is left is overwritten)
+        // (the flux of a face left to the list is overwritten after the barrier)
         auto face = [&](int j, const fx::Cell& c, bool mine, float xR, float xL, float tR, float tL, float rs,
-                        float rd, bool& left) -> double {
+                        float rd) -> double {
             int64_t Z, D, Q;
             const bool ok = fx::face_sums(c, xR, xL, tR, tL, rs, rd, Z, D, Q) && speed.in;
-            left = mine && !ok;
-            if (out.ul && mine && ok)
-                out(j, fx::to_double(Z + D, c.kz) * (1.0 / 12.0), fx::to_double(Z - D, c.kz) * (1.0 / 12.0));
+            if (mine) {
+                if (!ok) list[atomicAdd(&sm.fx[slot], 1)] = j;
+                else if (out.ul)
+                    out(j, fx::to_double(Z + D, c.kz) * (1.0 / 12.0), fx::to_double(Z - D, c.kz) * (1.0 / 12.0));
+            }
             if constexpr (LF) return fx::face_flux_lf(c, Z, D, speed);
             else return fx::face_flux(c.k, Z, D, Q);
         };
-        bool l0, l1;
         const double f0 = face(c0, s.x, m0, fx::p2x(u.xR), fx::p2x(u.xL), fx::p2x(u.tR), fx::p2x(u.tL),
-                               fx::p2x(u.rs), fx::p2x(u.rd), l0);
+                               fx::p2x(u.rs), fx::p2x(u.rd));
         const double f1 = face(c0 + 1, s.y, m1, fx::p2y(u.xR), fx::p2y(u.xL), fx::p2y(u.tR), fx::p2y(u.tL),
-                               fx::p2y(u.rs), fx::p2y(u.rd), l1);
+                               fx::p2y(u.rs), fx::p2y(u.rd));
         if (m0 && m1) *reinterpret_cast<double2*>(win_span(sm.D, c0, 2)) = make_double2(f0, f1);
         else if (m0) sm.D[c0] = f0;
         else if (m1) sm.D[c0 + 1] = f1;
-        if (__any_sync(kFull, l0 || l1)) {
-            if (fx_many(jhi - jlo, l0, l1)) {
-                fx_listed_chunk(v, sm.D, r0, sm.W, l0, l1, p.eps, aglob, out);
-            } else {
-                if (l0) list[atomicAdd(&sm.fx[slot], 1)] = c0;
-                if (l1) list[atomicAdd(&sm.fx[slot], 1)] = c0 + 1;
-            }
-        }
     }
     __syncthreads();
     const int cnt = sm.fx[slot];
@@ -959,7 +959,8 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
         if (slot == 1) sm.fx[0] = 0;  // (a step may end before its third stage)
     }
     if (cnt > 0) {
-        fx_listed_faces(v, sm.D, list, cnt, p.eps, aglob, out);
+        if (fx_many(cnt, jhi - jlo)) fx_listed_tile(v, sm.D, list, cnt, jlo, jhi, sm.W, p.eps, aglob, out);
+        else fx_listed_faces(v, sm.D, list, cnt, p.eps, aglob, out);
         __syncthreads();
     }
 }

@@ -1,5 +1,5 @@
 """Faces and cells that the integer / float-pair forms leave to FP64 (``csrc/stencil.cuh``
-``fx_listed_faces``, ``fx_listed_chunk``, ``csrc/adjoint.cu`` ``weno53_listed_vjp``): states of noise, of runs of
+``fx_listed_faces``, ``fx_listed_tile``, ``csrc/adjoint.cu`` ``weno53_listed_vjp``): states of noise, of runs of
 it, and random ones, at the window lengths where the list, the chunks of 60 faces and
 their threshold change."""
 
