@@ -822,13 +822,15 @@ __global__ void __launch_bounds__(kThreads, REC == SHK_REC_LEARNED || FLUX == kF
 }
 
 // The reverse step of a periodic instance of a fixed_flux_scheme plan from the
-// replay's stored stages, bound by latency (FP64 pipe 51 % busy, 0.34 instructions
-// per clock; barriers and loads are the top stalls): one loop over the reverse stages, each loading its own
+// replay's stored stages, bound by latency (FP64 pipe 52 % busy, 40 % of the issue
+// slots; loads, shared memory and barriers are the top stalls; 240 B of spills at the 80
+// registers of three CTAs): one loop over the reverse stages, each loading its own
 // state and face values, in 13 windows (batched_adjoint_kernel keeps 24, for its
 // recompute) so that three CTAs fit an SM. UL/UR hold T0/T1 once the seeds are
 // formed; the cotangent is updated in place; Z overwrites the pair part. 96
 // instances, 0.4 M cells: 471 us per reverse step with the FP64 backward, 202 with
-// the float pairs in 24 windows (two CTAs), 147 here.
+// the float pairs in 24 windows (two CTAs), 147 here, about 139 since the listed cells
+// have a backward of their own.
 constexpr int kAdjFxArrays = 13;
 constexpr int kAdjFxThreads = 256, kAdjFxCtas = 3;
 __device__ __forceinline__ void carve_adjoint_fx(AdjSmem<double>& a, unsigned char* base, int W) {

@@ -27,9 +27,10 @@
 // Measured on the batched step (4096 instances, 25.9 M cells, us per step): 8010
 // with the FP64 formula (156 FP64 instructions per cell-step, that pipe 86 %
 // busy), 1199 with this. Error of the states against runs in 113-bit arithmetic
-// (Fourier modes and a jump; relative L2, FP64 formula / this): 40 instances of 100
-// to 1000 cells, 50 steps 2.9865e-15 / 2.9869e-15; 40 of 500 to 9000, 10 steps
-// 6.242e-16 / 6.217e-16; 16 of 1024 to 8192, 4 steps 2.674e-16 / 2.674e-16.
+// (relative L2, FP64 formula / this): Fourier modes and a jump, 24 instances of 100 to
+// 1000 cells, 30 steps 1.806e-15 / 1.800e-15; 16 of 500 to 9000, 6 steps 3.941e-16 /
+// 3.957e-16; with 0.5 % noise, 10 steps 6.189e-16 / 6.196e-16; jumps between constants
+// 4.587e-16 / 4.389e-16; random cells, all left to FP64, 6.291e-16 / 6.498e-16.
 #pragma once
 
 #include <cstdint>

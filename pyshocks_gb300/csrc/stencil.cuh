@@ -969,9 +969,9 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
 // one loop over the stages: the flux code is long, and three copies of it
 // missed the instruction cache. The updates stay in these textbook formulas:
 // sums of increments doubled the FP64 work's error (3e-15 against 7e-16 after
-// 50 steps). Bound by issue (0.68 warp instructions per clock and scheduler)
-// with the integer pipe 57 %, FMA 47 % and FP64 46 % busy: the update's FP64
-// operations, the conversions and the listed faces.
+// 50 steps). Bound by issue (65 % of the slots) with the integer pipe 50 %, FMA
+// 47 % and FP64 49 % of its cycles busy: 10 of the 12.8 FP64 instructions per
+// cell-step are the update's, the rest the listed faces'.
 __device__ __forceinline__ unsigned long long step_tile_fx(const Smem<double>& sm, Win<double> gout, int te,
                                                            double dtdx, const OpParams<double>& p,
                                                            const BcView& bc, int64_t g0, int64_t n,
