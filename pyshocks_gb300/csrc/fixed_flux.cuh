@@ -28,9 +28,9 @@
 // with the FP64 formula (156 FP64 instructions per cell-step, that pipe 86 %
 // busy), 1199 with this. Error of the states against runs in 113-bit arithmetic
 // (relative L2, FP64 formula / this): Fourier modes and a jump, 24 instances of 100 to
-// 1000 cells, 30 steps 1.806e-15 / 1.800e-15; 16 of 500 to 9000, 6 steps 3.941e-16 /
+// 1000 cells, 30 steps 1.806e-15 / 1.799e-15; 16 of 500 to 9000, 6 steps 3.941e-16 /
 // 3.957e-16; with 0.5 % noise, 10 steps 6.189e-16 / 6.196e-16; jumps between constants
-// 4.587e-16 / 4.389e-16; random cells, all left to FP64, 6.291e-16 / 6.498e-16.
+// 4.587e-16 / 4.387e-16; random cells, all left to FP64, 6.291e-16 / 6.238e-16.
 #pragma once
 
 #include <cstdint>
@@ -514,13 +514,15 @@ SHK_FX double face_flux_lf(const Cell& c, int64_t Z, int64_t D, const Speed& sp)
 // integers do not hold it.
 SHK_FX bool listed_flux(double tR, double tL, double v0, double v1, double aglob, double& G) {
     const Mag r = mag(tR), l = mag(tL), a = mag(v0), b = mag(v1), g = mag(aglob);
-    uint32_t exm = r.e > l.e ? r.e : l.e;
-    exm = exm > a.e ? exm : a.e;
-    exm = exm > b.e ? exm : b.e;
+    // the scale of the cells and of a quarter of the corrections (|R - v| is a sixth of
+    // them): their integers stay below 2^59, Z and D below 2^62, Q below 2^63
+    uint32_t exm = a.e > b.e ? a.e : b.e;
     exm = exm > g.e ? exm : g.e;
+    exm = exm + 2u > r.e ? exm : r.e - 2u;
+    exm = exm + 2u > l.e ? exm : l.e - 2u;
     if (exm == 0u) exm = 1023u - 60u;
     if (exm - (1023u - 60u) > 120u) return false;
-    const int64_t x = with_sign(fix_abs(r, exm), r), y = with_sign(fix_abs(l, exm), l);
+    const int64_t x = with_sign(shr64(r.m << 2, exm + 3u - r.e), r), y = with_sign(shr64(l.m << 2, exm + 3u - l.e), l);
     const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm), A2 = fix_abs(g, exm);
     uint64_t A = A0 > A1 ? A0 : A1;
     A = A > A2 ? A : A2;

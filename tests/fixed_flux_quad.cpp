@@ -52,18 +52,35 @@ static void cell_double(const double* v, double eps, double& ul, double& ur) {
     ul = std::fma(nl * dr, r, v[2]);
 }
 
+struct Sum;
+static void add_listed(Sum& sum, const double* v, double eps);
 struct Sum {
     double n = 0, s = 0, top = 0;
     void add(double e) { n += 1; s += e * e; top = std::max(top, e); }
     void print(const char* name) const { std::printf("%s.count %.0f\n%s.rms %.6g\n%s.max %.6g\n", name, n, name, std::sqrt(s / std::max(n, 1.0)), name, top); }
 };
 
+// the flux of the face between v[2] and v[3] of six from its rounded corrections, in units
+// of the largest of its four cells and face values
+static void add_listed(Sum& sum, const double* v, double eps) {
+    quad q[6], tR, tL, x;
+    for (int i = 0; i < 6; ++i) q[i] = v[i];
+    corrections(q, eps, tR, x);
+    corrections(q + 1, eps, x, tL);
+    const double tr = double(tR), tl = double(tL);
+    const quad R = q[2] + quad(tr) / 6, L = q[3] + quad(tl) / 6, am = qmax(qabs(q[2]), qabs(q[3]));
+    quad top = qmax(qmax(qabs(R), qabs(L)), am);
+    double g;
+    if (!listed_flux(tr, tl, v[2], v[3], 0.0, g)) return;
+    sum.add(double(qabs(quad(g) - flux288(R, L, am)) / (quad(0x1p-53) * 288 * top * top)));
+}
+
 int main() {
     std::mt19937_64 gen(7);
     std::normal_distribution<double> N(0.0, 1.0);
     std::uniform_real_distribution<double> U(0.0, 1.0);
     const double unit = 0x1p-53;
-    Sum pair, plain, lf, listed, faces, grad;
+    Sum pair, plain, lf, listed, rough, faces, grad;
     double bad_double = 0, bad_split = 0;
     for (double eps : {1e-24, 1e-12, 1e-6, 1.0, 1e24}) {
         const FF eps4{dup(static_cast<float>(4.0 * eps)), dup(static_cast<float>(4.0 * eps - double(static_cast<float>(4.0 * eps))))};
@@ -120,12 +137,7 @@ int main() {
                         faces.add(double(qmax(qabs(quad(to_double(Z + D, c.kz) * (1.0 / 12.0)) - R), qabs(quad(to_double(Z - D, c.kz) * (1.0 / 12.0)) - L)) / (quad(unit) * quad(top))));
                     }
                     // the flux of a left face from its rounded corrections
-                    const double tr = double(tR), tl = double(tL);
-                    double g;
-                    if (listed_flux(tr, tl, v[j], v[j + 1], 0.0, g)) {
-                        const double t2 = std::max(top, std::max(std::fabs(tr), std::fabs(tl)));
-                        listed.add(double(qabs(quad(g) - flux288(w5[2] + quad(tr) / 6, w5[3] + quad(tl) / 6, am)) / (quad(unit) * 288 * quad(t2) * quad(t2))));
-                    }
+                    add_listed(listed, &v[j - 2], eps);
                 }
                 // the backward of the two cells' weights
                 const Cell &cx = s[l].x, &cy = s[l].y;
@@ -165,6 +177,12 @@ int main() {
             }
         }
     }
+    // left faces of random cells, also where one side is much the larger
+    for (int i = 0; i < 100000; ++i) {
+        double v[6];
+        for (double& x : v) x = N(gen) * (i % 2 ? 1.0 : std::pow(10.0, -6.0 * U(gen)));
+        add_listed(rough, v, 1e-6);
+    }
     for (int i = 0; i < 200000; ++i) {
         // integers to doubles: within half a unit in the last place
         const int sh = int(gen() % 63);
@@ -186,6 +204,7 @@ int main() {
     lf.print("lf");
     faces.print("faces");
     listed.print("listed");
+    rough.print("rough");
     grad.print("grad");
     std::printf("to_double.max %.6g\nsplit.max %.6g\n", bad_double, bad_split);
     return 0;
