@@ -502,34 +502,58 @@ SHK_FX Speed speed_begin(double a) {
 // in units 2^(k + sh), sh the distance of the two scales. dt / dx times the
 // speed is at most 1/2, so a resolution of 2^-57 of (speed x local value) in F
 // is one of 2^-57 of the local value in the state.
+SHK_FX double lf_flux(uint32_t exm, int k, int64_t Z, int64_t D, const Speed& sp) {
+    const uint32_t d = sp.e > exm ? sp.e - exm : 0u, sh = d < 63u ? d : 63u;
+    return to_double(((square_hi(Z) + square_hi(D)) >> sh) + product_hi(D, sp.M), k + static_cast<int>(d));
+}
 SHK_FX double face_flux_lf(const Cell& c, int64_t Z, int64_t D, const Speed& sp) {
-    const uint32_t d = sp.e > c.exm ? sp.e - c.exm : 0u, sh = d < 63u ? d : 63u;
-    return to_double(((square_hi(Z) + square_hi(D)) >> sh) + product_hi(D, sp.M), c.k + static_cast<int>(d));
+    return lf_flux(c.exm, c.k, Z, D, sp);
 }
 
-// 288 F from six times the corrections tR = 6 (R - v0), tL = 6 (L - v1) of the face values
-// formed in double (v0, v1: the face's cells, a: the speed if it is the larger), with
-// the integer arithmetic of the other faces: next to a constant state, where R = L =
-// v, the flux equals theirs and the difference vanishes exactly. False where the
-// integers do not hold it.
-SHK_FX bool listed_flux(double tR, double tL, double v0, double v1, double aglob, double& G) {
-    const Mag r = mag(tR), l = mag(tL), a = mag(v0), b = mag(v1), g = mag(aglob);
-    // the scale of the cells and of a quarter of the corrections (|R - v| is a sixth of
-    // them): their integers stay below 2^59, Z and D below 2^62, Q below 2^63
+// Z and D of a face from six times the corrections tR = 6 (R - v0), tL = 6 (L - v1) of its
+// face values formed in double (v0, v1: the face's cells; A: max of their magnitudes), on
+// the scale of the cells and of a quarter of the corrections (|R - v| is a sixth of
+// them): the corrections' integers stay below 2^59, Z and D below 2^62, D + 24 A below
+// 2^63. False where the integers do not hold it.
+struct ListedSums {
+    int64_t Z, D;
+    uint64_t A;
+    uint32_t exm;
+};
+SHK_FX bool listed_sums(double tR, double tL, double v0, double v1, ListedSums& s) {
+    const Mag r = mag(tR), l = mag(tL), a = mag(v0), b = mag(v1);
     uint32_t exm = a.e > b.e ? a.e : b.e;
-    exm = exm > g.e ? exm : g.e;
     exm = exm + 2u > r.e ? exm : r.e - 2u;
     exm = exm + 2u > l.e ? exm : l.e - 2u;
     if (exm == 0u) exm = 1023u - 60u;
+    s.exm = exm;
     if (exm - (1023u - 60u) > 120u) return false;
     const int64_t x = with_sign(shr64(r.m << 2, exm + 3u - r.e), r), y = with_sign(shr64(l.m << 2, exm + 3u - l.e), l);
-    const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm), A2 = fix_abs(g, exm);
-    uint64_t A = A0 > A1 ? A0 : A1;
-    A = A > A2 ? A : A2;
+    const uint64_t A0 = fix_abs(a, exm), A1 = fix_abs(b, exm);
     const int64_t V0 = with_sign(A0, a), V1 = with_sign(A1, b);
-    const int64_t D = 6 * (V0 - V1) + (x - y), Q = D + static_cast<int64_t>(24u * A);
+    s.A = A0 > A1 ? A0 : A1;
+    s.Z = 6 * (V0 + V1) + (x + y);
+    s.D = 6 * (V0 - V1) + (x - y);
+    return true;
+}
+// 288 F with the integer arithmetic of the other faces: next to a constant state, where
+// R = L = v, the flux equals theirs and the difference vanishes exactly
+SHK_FX bool listed_flux(double tR, double tL, double v0, double v1, double& G) {
+    ListedSums s;
+    if (!listed_sums(tR, tL, v0, v1, s)) return false;
+    const int64_t Q = s.D + static_cast<int64_t>(24u * s.A);
     if (Q < 0) return false;
-    G = face_flux(2 * static_cast<int>(exm) - 2094, 6 * (V0 + V1) + (x + y), D, Q);
+    G = face_flux(2 * static_cast<int>(s.exm) - 2094, s.Z, s.D, Q);
+    return true;
+}
+// (with the speed's own scale, as face_flux_lf; a face value may exceed it by a few powers
+// of two)
+SHK_FX bool listed_flux_lf(double tR, double tL, double v0, double v1, const Speed& sp, double& G) {
+    ListedSums s;
+    if (!listed_sums(tR, tL, v0, v1, s) || !sp.in) return false;
+    const uint32_t up = s.exm > sp.e ? s.exm - sp.e : 0u;
+    const Speed scaled{static_cast<int64_t>(shr64(static_cast<uint64_t>(sp.M), up)), sp.e + up, true};
+    G = lf_flux(s.exm, 2 * static_cast<int>(s.exm) - 2094, s.Z, s.D, scaled);
     return true;
 }
 

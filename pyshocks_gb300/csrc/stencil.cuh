@@ -797,18 +797,20 @@ __device__ __forceinline__ double weno53_left(const WenoTerms& w, double a, doub
 }
 __device__ __forceinline__ double weno53_g(double E, double eps4) { return fma((13.0 / 3.0) * E, E, eps4); }
 
-// the flux of such a face from its two corrections
-template <class PV, class FaceOut>
+// the flux of such a face from its two corrections (LF: with the speed aglob)
+template <bool LF, class PV, class FaceOut>
 __device__ __forceinline__ void fx_listed_flux(PV v, Win<double> G, int j, double tR, double tL, double aglob,
                                                const FaceOut& out) {
     const double v0 = v[j], v1 = v[j + 1];
     double g;
-    const bool ok = fx::listed_flux(tR, tL, v0, v1, aglob, g);
+    bool ok;
+    if constexpr (LF) ok = fx::listed_flux_lf(tR, tL, v0, v1, fx::speed_begin(aglob), g);
+    else ok = fx::listed_flux(tR, tL, v0, v1, g);
     if (!ok || out.ul) {
         const double R = fma(tR, 1.0 / 6.0, v0), L = fma(tL, 1.0 / 6.0, v1);
         if (!ok) {
             auto ab = abs_bits(v0) > abs_bits(v1) ? abs_bits(v0) : abs_bits(v1);
-            ab = ab > abs_bits(aglob) ? ab : abs_bits(aglob);
+            if constexpr (LF) ab = ab > abs_bits(aglob) ? ab : abs_bits(aglob);
             g = 72.0 * fma(L, L, fma(R, R, twice_abs_bits(ab) * (R - L)));
         }
         if (out.ul) out(j, R, L);
@@ -817,7 +819,7 @@ __device__ __forceinline__ void fx_listed_flux(PV v, Win<double> G, int j, doubl
 }
 
 // few: two lanes per face, one for each side (38 FP64 instructions for 16 faces)
-template <class PV, class FaceOut>
+template <bool LF, class PV, class FaceOut>
 __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list, int cnt, double eps,
                                              double aglob, FaceOut out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -832,7 +834,7 @@ __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list,
         const WenoTerms w = weno53_terms(dm1, d0, Em, E0, Ep, weno53_g(Em, eps4), weno53_g(E0, eps4),
                                          weno53_g(Ep, eps4));
         const double t = weno53_right(w, dm1, d0), t1 = __shfl_xor_sync(0xffffffffu, t, 1);
-        if (q < cnt && (lane & 1) == 0) fx_listed_flux(v, G, j, t, t1, aglob, out);
+        if (q < cnt && (lane & 1) == 0) fx_listed_flux<LF>(v, G, j, t, t1, aglob, out);
     }
 }
 
@@ -850,7 +852,7 @@ __device__ __noinline__ void fx_listed_faces(PV v, Win<double> G, Win<int> list,
 // 57 / 47 / 47. (Each warp taking its own chunk at once, before the barrier: noise 5 %
 // faster on 300 ragged instances, smooth states 1 % slower.)
 __device__ __forceinline__ bool fx_many(int cnt, int faces) { return 2 * cnt > faces && faces > 90; }
-template <class PV, class FaceOut>
+template <bool LF, class PV, class FaceOut>
 __device__ __noinline__ void fx_listed_tile(PV v, Win<double> G, Win<int> list, int cnt, int jlo, int jhi, int W,
                                             double eps, double aglob, FaceOut out) {
     constexpr unsigned kFull = 0xffffffffu;
@@ -877,8 +879,8 @@ __device__ __noinline__ void fx_listed_tile(PV v, Win<double> G, Win<int> list, 
         const WenoTerms b = weno53_terms(d0, d1, E0, E1, Ep, G0, G1, Gp);
         const double L2 = __shfl_down_sync(kFull, weno53_left(a, dm, d0), 1);
         const double R0 = weno53_right(a, dm, d0), L1 = weno53_left(b, d0, d1), R1 = weno53_right(b, d0, d1);
-        if (l0) fx_listed_flux(v, G, c0, R0, L1, aglob, out);
-        if (l1) fx_listed_flux(v, G, c0 + 1, R1, L2, aglob, out);
+        if (l0) fx_listed_flux<LF>(v, G, c0, R0, L1, aglob, out);
+        if (l1) fx_listed_flux<LF>(v, G, c0 + 1, R1, L2, aglob, out);
     }
 }
 
@@ -959,8 +961,8 @@ __device__ __forceinline__ void fx_fluxes(PV v, int jlo, int jhi, const Smem<dou
         if (slot == 1) sm.fx[0] = 0;  // (a step may end before its third stage)
     }
     if (cnt > 0) {
-        if (fx_many(cnt, jhi - jlo)) fx_listed_tile(v, sm.D, list, cnt, jlo, jhi, sm.W, p.eps, aglob, out);
-        else fx_listed_faces(v, sm.D, list, cnt, p.eps, aglob, out);
+        if (fx_many(cnt, jhi - jlo)) fx_listed_tile<LF>(v, sm.D, list, cnt, jlo, jhi, sm.W, p.eps, aglob, out);
+        else fx_listed_faces<LF>(v, sm.D, list, cnt, p.eps, aglob, out);
         __syncthreads();
     }
 }

@@ -60,6 +60,9 @@ struct Sum {
     void print(const char* name) const { std::printf("%s.count %.0f\n%s.rms %.6g\n%s.max %.6g\n", name, n, name, std::sqrt(s / std::max(n, 1.0)), name, top); }
 };
 
+static Sum lf_rough;
+static int state_shift = 0;
+
 // the flux of the face between v[2] and v[3] of six from its rounded corrections, in units
 // of the largest of its four cells and face values
 static void add_listed(Sum& sum, const double* v, double eps) {
@@ -71,8 +74,12 @@ static void add_listed(Sum& sum, const double* v, double eps) {
     const quad R = q[2] + quad(tr) / 6, L = q[3] + quad(tl) / 6, am = qmax(qabs(q[2]), qabs(q[3]));
     quad top = qmax(qmax(qabs(R), qabs(L)), am);
     double g;
-    if (!listed_flux(tr, tl, v[2], v[3], 0.0, g)) return;
+    if (!listed_flux(tr, tl, v[2], v[3], g)) return;
     sum.add(double(qabs(quad(g) - flux288(R, L, am)) / (quad(0x1p-53) * 288 * top * top)));
+    // Lax-Friedrichs with a speed at least the cells': in units of speed x size
+    const double speed = std::ldexp(double(am), state_shift++ % 40) * 1.25;
+    if (!listed_flux_lf(tr, tl, v[2], v[3], speed_begin(speed), g)) return;
+    lf_rough.add(double(qabs(quad(g) - flux288(R, L, speed)) / (quad(0x1p-53) * 288 * top * qmax(top, speed))));
 }
 
 int main() {
@@ -205,6 +212,7 @@ int main() {
     faces.print("faces");
     listed.print("listed");
     rough.print("rough");
+    lf_rough.print("lf_rough");
     grad.print("grad");
     std::printf("to_double.max %.6g\nsplit.max %.6g\n", bad_double, bad_split);
     return 0;

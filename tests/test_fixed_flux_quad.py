@@ -34,13 +34,13 @@ def values(tmp_path_factory):
 
 
 def test_enough_faces_of_each_kind(values):
-    for kind in ("rusanov", "lf", "listed", "rough", "grad"):
+    for kind in ("rusanov", "lf", "listed", "rough", "lf_rough", "grad"):
         assert values[f"{kind}.count"] > 10000
 
 
 def test_fluxes(values):
     assert values["rusanov.rms"] <= values["formula.rms"]
-    for kind in ("rusanov", "lf", "faces", "listed", "rough"):
+    for kind in ("rusanov", "lf", "faces", "listed", "rough", "lf_rough"):
         assert values[f"{kind}.max"] <= 8.0, kind
 
 

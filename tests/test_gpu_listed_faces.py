@@ -129,3 +129,30 @@ def test_single_step_and_transpose_on_coarse_grids(kind, n):
     assert lib.shk_ssprk33_vjp_f64(cs, ud.data_ptr(), pd.data_ptr(), out.data_ptr(), n, 3, dx, dt, L.stream_handle()) == 0
     ref = T.step_vjp(u[None], p[None], dt, dx)[0]
     assert float((out.cpu()[3:-3] - ref).abs().max()) <= 1.0e-11 * float(ref.abs().max())
+
+
+def test_lax_friedrichs_where_the_state_is_small():
+    """Random cells of size 1e-10 far from cells of size 1: their fluxes carry the
+    instance's speed and are exact to (speed x their own size), so two steps keep
+    1e-13 of 1e-10 (about 900 roundings) away from the large cells' reach."""
+    from pyshocks_gb300.batched import BatchedSolver
+
+    rng = np.random.default_rng(31)
+    sizes, nsteps = [400, 1201], 2
+    u0 = []
+    for n in sizes:
+        x = (np.arange(n) + 0.5) / n
+        u0.append(np.where(x < 0.5, 0.4 + np.sin(2 * np.pi * x), 1.0e-10 * rng.uniform(-1.0, 1.0, n)))
+    for tile in (0, 64):
+        s = BatchedSolver(_scheme("lf"), sizes, [2.0 / n for n in sizes], theta=0.9, tile=tile)
+        s.reset(torch.tensor(np.concatenate(u0)))
+        s.step(nsteps)
+        assert s.status() == 0
+        for b, n in enumerate(sizes):
+            og = R.make_uniform_cell_grid(-1.0, 1.0, n, 3)
+            ug = np.zeros(n + 6)
+            ug[3:-3] = u0[b]
+            ref, _ = R.evolve(R.SchemeSpec(flux_kind="lf"), og, ug, theta=0.9, maxit=nsteps)
+            far = slice(n // 2 + 40, n - 40)
+            err = np.max(np.abs(s.instance(b).cpu().numpy()[far] - ref[3:-3][far]))
+            assert err < 1.0e-23, (n, tile, err)
